@@ -244,7 +244,7 @@ RT_D float clearcoat_shape(const Material& m, float cndv, float cndl, float cndh
     return 0.25f * cD * cG * cF;
 }
 
-// EvaluateDirect (bsdf_eval_direct).
+// EvaluateDirect (bsdf_eval_pdf, direct).
 RT_NI D3 eval_direct_dual(const SceneView& s, const Material& m, const DMat& dm, const Surface& rec, V3 L, V3 V) {
     V3 N = rec.n;
     D3 r = d3(v3(0.0f));
@@ -278,7 +278,7 @@ RT_NI D3 eval_direct_dual(const SceneView& s, const Material& m, const DMat& dm,
     return r + multiscatter_dual(s, dm, ndv, ndl) * (ndl / kPi);
 }
 
-// Evaluate (bsdf_eval), without the cosine.
+// Evaluate (bsdf_eval_pdf), without the cosine.
 RT_NI D3 eval_dual(const SceneView& s, const Material& m, const DMat& dm, const Surface& rec, V3 V, V3 L) {
     V3 N = rec.n;
     D3 r = d3(v3(0.0f));

@@ -66,16 +66,21 @@ RT_D uint32_t lk_permute(uint32_t v, uint32_t seed) {
 }
 RT_D uint32_t owen_scramble(uint32_t v, uint32_t seed) { return __brev(lk_permute(__brev(v), seed)); }
 
+// Dimensions 0 and 1, which only the camera jitter draws: out of line, so that
+// every other draw site carries the padded-dimension code alone.
+__device__ __noinline__ uint32_t sobol_dim01(uint32_t index, uint32_t dim) {
+    if (dim == 0u) return __brev(index);
+    uint32_t v = 0u, i = index;
+#pragma unroll 1
+    for (int k = 0; i != 0u; k++, i >>= 1)
+        if (i & 1u) v ^= c_dim1_dirs[k];
+    return v;
+}
+
 RT_D float sobol_sample(uint32_t index, uint32_t dim, uint32_t pixel_seed) {
     uint32_t v;
-    if (dim == 0u) {
-        v = __brev(index);
-    } else if (dim == 1u) {
-        v = 0u;
-        uint32_t i = index;
-#pragma unroll 1
-        for (int k = 0; i != 0u; k++, i >>= 1)
-            if (i & 1u) v ^= c_dim1_dirs[k];
+    if (dim < 2u) {
+        v = sobol_dim01(index, dim);
     } else {
         uint32_t shuffle = hash_u32(dim * 0x68bc21ebu + 0xc7afe638u);
         v = __brev(owen_scramble(index, shuffle));
@@ -91,15 +96,18 @@ struct Sampler {
     RT_D float next() { return sobol_sample(index, dim++, seed); }
 };
 
-RT_D V3 random_unit_vector(Sampler& s) {   // Core/MathUtils.cs:104-112
-    float u = s.next();
-    float v = s.next();
+RT_D V3 unit_vector(float u, float v) {   // MathUtils.RandomUnitVector (Core/MathUtils.cs:104-112)
     float z = 1.0f - 2.0f * u;
     float r = sqrtf(fmaxf(0.0f, 1.0f - z * z));
     float phi = 2.0f * kPi * v;
     float sn, cs;
     sincosf(phi, &sn, &cs);
     return v3(r * cs, r * sn, z);
+}
+RT_D V3 random_unit_vector(Sampler& s) {
+    float u = s.next();
+    float v = s.next();
+    return unit_vector(u, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -766,7 +774,8 @@ __device__ __forceinline__ bool trace(const SceneView& s, V3 o, V3 d, float tmin
 
 // Surface record of an accepted hit (Core/HitRecord.cs fields on the path).
 struct Surface {
-    V3 p, n, tangent, bitangent;
+    V3 p, n, tangent;
+    int has_bitangent;   // the bitangent has a length (its direction is never read: shading_frame)
     float t;
     int front;
     int material;
@@ -793,10 +802,12 @@ RT_D Surface make_surface(const SceneView& s, const Hit& h, V3 o, V3 d) {
             V3 sn = normalize(w0 * st.n0 + h.u * st.n1 + h.v * st.n2);
             r.n = r.front ? sn : -sn;   // the face normal decides the side
             r.tangent = st.tangent;
-            r.bitangent = st.bitangent;
+            r.has_bitangent = length_sq(st.bitangent) > 1e-10f;
         } else {
             r.tangent = length_sq(e1) > 0.0f ? normalize(e1) : v3(1.0f, 0.0f, 0.0f);
-            r.bitangent = length_sq(e2) > 0.0f ? normalize(e2) : v3(0.0f, 0.0f, 1.0f);
+            // normalize(e2), or (0, 0, 1) when length_sq(e2) is not positive: it has a
+            // length unless length_sq overflows (then e2 / infinity is zero)
+            r.has_bitangent = length_sq(e2) != INFINITY;
         }
         r.entity = s.tri_entity[ti];
         r.prim = s.tri_local[ti];
@@ -806,7 +817,7 @@ RT_D Surface make_surface(const SceneView& s, const Hit& h, V3 o, V3 d) {
         r.front = dot(d, q.normal) < 0.0f;
         r.n = r.front ? q.normal : -q.normal;
         r.tangent = q.tangent;
-        r.bitangent = q.bitangent;
+        r.has_bitangent = length_sq(q.bitangent) > 1e-10f;
         r.entity = h.slot;
         r.prim = 0;
     } else {
@@ -818,7 +829,9 @@ RT_D Surface make_surface(const SceneView& s, const Hit& h, V3 o, V3 d) {
         V3 td = cross(v3(0.0f, 1.0f, 0.0f), outward);
         if (length_sq(td) < 1e-4f) td = v3(1.0f, 0.0f, 0.0f);
         r.tangent = normalize(td);
-        r.bitangent = normalize(cross(outward, r.tangent));
+        // normalize(cross(outward, tangent)) has a length when the cross product has a finite one
+        float bl2 = length_sq(cross(outward, r.tangent));
+        r.has_bitangent = bl2 > 0.0f && bl2 < INFINITY;
         r.entity = h.slot;
         r.prim = 0;
     }
@@ -829,21 +842,15 @@ RT_D Surface make_surface(const SceneView& s, const Hit& h, V3 o, V3 d) {
 // ---------------------------------------------------------------------------
 // Kulla-Conty LUT lookups (Materials/EnergyCompensationLut.cs:140-175)
 // ---------------------------------------------------------------------------
-RT_D float lut_e(const float* e, float mu, float alpha) {
+// E at a material's roughness: the table's alpha interpolation is in
+// Material::lut_mu, the mu interpolation here.
+RT_D float lut_e_mu(const Material& m, float mu) {
     mu = clampf(mu, 0.0f, 1.0f);
-    alpha = clampf(alpha, 0.001f, 1.0f);
     float fmu = mu * 32.0f - 0.5f;
-    float fal = alpha * 32.0f - 0.5f;
     int m0 = min(max((int)floorf(fmu), 0), 31);
-    int a0 = min(max((int)floorf(fal), 0), 31);
     int m1 = min(m0 + 1, 31);
-    int a1 = min(a0 + 1, 31);
     float tu = clampf(fmu - (float)m0, 0.0f, 1.0f);
-    float ta = clampf(fal - (float)a0, 0.0f, 1.0f);
-    float e00 = __ldg(e + m0 * 32 + a0), e01 = __ldg(e + m0 * 32 + a1);
-    float e10 = __ldg(e + m1 * 32 + a0), e11 = __ldg(e + m1 * 32 + a1);
-    float x0 = e00 + (e01 - e00) * ta;
-    float x1 = e10 + (e11 - e10) * ta;
+    float x0 = __ldg(m.lut_mu + m0), x1 = __ldg(m.lut_mu + m1);
     return x0 + (x1 - x0) * tu;
 }
 
@@ -919,7 +926,9 @@ RT_D float sheen_lambda(float c, float alpha) {   // :71-85
     float hi = expf(sheen_lambda_log(c, false));
     return lo + (hi - lo) * t;
 }
-RT_D float sheen_brdf(float ndv, float ndl, float ndh, float alpha) {   // :24-34, :92-121
+// Out of line: few materials have sheen, and its powf and expf expansions are
+// long.
+__device__ __noinline__ float sheen_brdf(float ndv, float ndl, float ndh, float alpha) {   // :24-34, :92-121
     float denom = 4.0f * fmaxf(ndv, 1e-6f) * fmaxf(ndl, 1e-6f);
     float g = 1.0f / ((1.0f + sheen_lambda(ndv, alpha)) * (1.0f + sheen_lambda(ndl, alpha)));
     float al = fmaxf(alpha, 0.04f);
@@ -967,7 +976,7 @@ struct Frame {
 
 RT_D Frame shading_frame(const Surface& rec, const Material& m) {   // :1840-1877
     V3 n = rec.n, t, b;
-    if (length_sq(rec.tangent) > 1e-10f && length_sq(rec.bitangent) > 1e-10f) {
+    if (length_sq(rec.tangent) > 1e-10f && rec.has_bitangent) {
         t = rec.tangent - dot(rec.tangent, n) * n;
         float tl = length_sq(t);
         if (tl > 1e-10f) {
@@ -989,162 +998,111 @@ RT_D Frame shading_frame(const Surface& rec, const Material& m) {   // :1840-187
     return Frame{t, b, n};
 }
 
-RT_D V3 multiscatter_weight(const SceneView& s, const Material& m, float ndv, float ndl) {   // :1906-1926
-    float e_out = lut_e(s.lut_e, ndv, m.alpha_iso);
-    float e_in = lut_e(s.lut_e, ndl, m.alpha_iso);
-    float e_avg = m.e_avg;
-    float one_m = fmaxf(1.0f - e_avg, 1e-6f);
-    V3 f_avg = m.f0 + (v3(1.0f) - m.f0) * (1.0f / 21.0f);
-    V3 den = v3(1.0f) - f_avg * (1.0f - e_avg);
-    den = v3(fmaxf(den.x, 1e-6f), fmaxf(den.y, 1e-6f), fmaxf(den.z, 1e-6f));
-    V3 f_ms = f_avg * f_avg * e_avg / den;
-    return f_ms * ((1.0f - e_out) * (1.0f - e_in) / one_m);
+RT_D V3 multiscatter_weight(const Material& m, float ndv, float ndl) {   // :1906-1926
+    float e_out = lut_e_mu(m, ndv);
+    float e_in = lut_e_mu(m, ndl);
+    return m.f_ms * ((1.0f - e_out) * (1.0f - e_in) / m.ms_one_m);
 }
 
-// EvaluateDirect (:418-535): f(V,L) * max(N.L, 0), the NEE integrand.
-RT_D V3 bsdf_eval_direct(const SceneView& s, const Material& m, const Surface& rec, V3 L, V3 V, V3 N) {
-    float ndl = fmaxf(dot(N, L), 0.0f);
-    if (ndl <= 0.0f) return v3(0.0f);
-    float ndv = fmaxf(dot(N, V), 0.001f);
-    V3 H = normalize(L + V);
-    float ndh = fmaxf(dot(N, H), 0.0f);
-    float vdh = fmaxf(dot(V, H), 0.0f);
-    float ldh = fmaxf(dot(L, H), 0.0f);
-    V3 bc = m.base;
-    V3 diffuse = v3(0.0f);
-    if (m.diffuse_w > 0.0f) {
-        float fd90 = 0.5f + 2.0f * m.roughness * ldh * ldh;
-        float fi = schlick_weight(ndv), fo = schlick_weight(ndl);
-        float fd = (1.0f + (fd90 - 1.0f) * fi) * (1.0f + (fd90 - 1.0f) * fo);
-        diffuse = bc * fd * (m.diffuse_w * ndl / kPi);
-    }
-    V3 specular = v3(0.0f);
-    if (m.alpha > kDeltaAlpha) {
-        Frame fr = shading_frame(rec, m);
-        V3 vl = fr.to_local(V), ll = fr.to_local(L), hl = fr.to_local(H);
-        float D = d_ggx(hl, m.alpha_x, m.alpha_y);
-        float G = g1_ggx(vl, m.alpha_x, m.alpha_y) * g1_ggx(ll, m.alpha_x, m.alpha_y);
-        V3 F = fresnel_schlick(vdh, m.f0);
-        specular = D * G * F / fmaxf(4.0f * ndv, 1e-6f);
-    }
-    V3 clearcoat = v3(0.0f);
-    if (m.clearcoat > 0.0f && m.cc_alpha > kDeltaAlpha) {
-        V3 cn = rec.n;
-        float cndv = fmaxf(dot(cn, V), 0.001f);
-        float cndl = dot(cn, L);
-        if (cndl > 0.0f) {
-            float cndh = fmaxf(dot(cn, H), 0.0f);
-            float cvdh = fmaxf(dot(V, H), 0.0f);
-            float ca2 = m.cc_alpha * m.cc_alpha;
-            float cden = cndh * cndh * (ca2 - 1.0f) + 1.0f;
-            float cD = ca2 / (kPi * cden * cden);
-            float cG = smith_g1(cndv, m.cc_alpha) * smith_g1(cndl, m.cc_alpha);
-            float cF = m.cc_f0 + (1.0f - m.cc_f0) * schlick_weight(cvdh);
-            clearcoat = v3(m.clearcoat * 0.25f * cD * cG * cF / fmaxf(4.0f * cndv, 1e-6f));
-        }
-    }
-    V3 sheen = v3(0.0f);
-    if (m.sheen > 0.0f && m.diffuse_w > 0.0f) {
-        float sb = sheen_brdf(ndv, ndl, ndh, m.sheen_roughness);
-        sheen = m.sheen * sb * m.sheen_col * ndl;
-    }
-    V3 ms = multiscatter_weight(s, m, ndv, ndl) * (1.0f / kPi) * ndl;
-    return diffuse + sheen + specular + ms + clearcoat;
+// What all evaluations at one vertex share: the view direction, in the shading
+// frame, and its masking term.
+struct BsdfView {
+    V3 V, vl;
+    Frame fr;
+    float ndv, g1v;
+};
+RT_D BsdfView bsdf_view(const Material& m, const Surface& rec, V3 V) {
+    BsdfView b;
+    b.V = V;
+    b.fr = shading_frame(rec, m);
+    b.vl = b.fr.to_local(V);
+    b.ndv = dot(rec.n, V);
+    b.g1v = g1_ggx(b.vl, m.alpha_x, m.alpha_y);
+    return b;
 }
 
-// Evaluate (:649-771): f(V, L) without the cosine.
-RT_D V3 bsdf_eval(const SceneView& s, const Material& m, const Surface& rec, V3 V, V3 L) {
-    V3 N = rec.n;
+// One direction L against the view, both values the renderer asks for:
+//   direct : f = EvaluateDirect(L, V, N) (:418-535), f(V,L) max(N.L, 0), the
+//            NEE integrand (when it is zero, pdf is not computed)
+//   !direct: f = Evaluate(V, L) (:649-771), without the cosine
+//   pdf    : Pdf(V, L) (:783-870), the one-sample mixture density of Sample
+// The two integrands and the density share the half vector, the GGX density,
+// the masking terms and the coat's density, and differ in where the cosine and
+// the floors go, so one body serves all three. Shading is bound by instruction
+// supply: a second and third inlined copy of this code cost more than any
+// operation in it.
+RT_D void bsdf_eval_pdf(const Material& m, const Surface& rec, const BsdfView& b, V3 L, bool direct, V3& f,
+                        float& pdf) {
+    const V3 N = rec.n, V = b.V;
+    f = v3(0.0f);
+    pdf = 0.0f;
     float ndl = dot(N, L);
-    float ndv = dot(N, V);
-    if (ndv <= 0.0f) return v3(0.0f);
-    V3 bc = m.base;
-    if (ndl <= 0.0f) {
-        if (m.diff_all <= 0.0f || m.diff_trans <= 0.0f) return v3(0.0f);
-        return bc * (m.diff_all * m.diff_trans / kPi);
-    }
+    if (direct ? fmaxf(ndl, 0.0f) <= 0.0f : b.ndv <= 0.0f) return;
     V3 hraw = V + L;
     float hl2 = length_sq(hraw);
-    if (hl2 < 1e-14f) return v3(0.0f);
     V3 H = hraw / sqrtf(hl2);
-    float ndh = fmaxf(dot(N, H), 0.0f);
+    bool has_h = hl2 >= 1e-14f;   // Evaluate and Pdf need a half vector; EvaluateDirect takes what comes
+    float ndh = dot(N, H);
     float vdh = fmaxf(dot(V, H), 0.0f);
-    float ldh = fmaxf(dot(L, H), 0.0f);
-    V3 diffuse = v3(0.0f);
-    if (m.diffuse_w > 0.0f) {
-        float fd90 = 0.5f + 2.0f * m.roughness * ldh * ldh;
-        float fi = schlick_weight(ndv), fo = schlick_weight(ndl);
-        float fd = (1.0f + (fd90 - 1.0f) * fi) * (1.0f + (fd90 - 1.0f) * fo);
-        diffuse = bc * fd * (m.diffuse_w / kPi);
+    V3 hl = b.fr.to_local(H);
+    float hx = hl.x / m.alpha_x, hy = hl.y / m.alpha_y;   // d_ggx with pi ax ay from the material
+    float hd = hx * hx + hy * hy + hl.z * hl.z;
+    float D = 1.0f / fmaxf(m.pi_axy * hd * hd, 1e-20f);
+    bool spec_ok = m.alpha > kDeltaAlpha;
+    bool coat_ok = m.cc_alpha > kDeltaAlpha;
+    bool coat = m.clearcoat > 0.0f;
+    float cD = 0.0f;
+    if (coat) {   // p_c > 0 needs clearcoat > 0
+        float cndh = fmaxf(ndh, 0.0f);
+        float ca2 = m.cc_alpha * m.cc_alpha;
+        float cden = cndh * cndh * (ca2 - 1.0f) + 1.0f;
+        cD = ca2 / (kPi * cden * cden);
     }
-    V3 sheen = v3(0.0f);
-    if (m.sheen > 0.0f && m.diffuse_w > 0.0f) {
-        float sb = sheen_brdf(ndv, ndl, ndh, m.sheen_roughness);
-        sheen = m.sheen * sb * m.sheen_col;
-    }
-    Frame fr = shading_frame(rec, m);
-    V3 vl = fr.to_local(V), ll = fr.to_local(L), hl = fr.to_local(H);
-    float D = d_ggx(hl, m.alpha_x, m.alpha_y);
-    float G = g1_ggx(vl, m.alpha_x, m.alpha_y) * g1_ggx(ll, m.alpha_x, m.alpha_y);
-    V3 F = fresnel_schlick(vdh, m.f0);
-    V3 specular = D * G / fmaxf(4.0f * ndv * ndl, 1e-7f) * F;
-    V3 clearcoat = v3(0.0f);
-    if (m.clearcoat > 0.0f) {
-        V3 cn = rec.n;
-        float cndv = dot(cn, V), cndl = dot(cn, L);
-        if (cndv > 0.0f && cndl > 0.0f) {
-            float cndh = fmaxf(dot(cn, H), 0.0f);
-            float cvdh = fmaxf(dot(V, H), 0.0f);
-            float ca2 = m.cc_alpha * m.cc_alpha;
-            float cden = cndh * cndh * (ca2 - 1.0f) + 1.0f;
-            float cD = ca2 / (kPi * cden * cden);
-            float cG = smith_g1(cndv, m.cc_alpha) * smith_g1(cndl, m.cc_alpha);
-            float cF = m.cc_f0 + (1.0f - m.cc_f0) * schlick_weight(cvdh);
-            float cc = m.clearcoat * 0.25f * cD * cG * cF / fmaxf(4.0f * cndv * cndl, 1e-7f);
-            clearcoat = v3(cc);
+    if (ndl <= 0.0f) {
+        if (!(m.diff_all <= 0.0f || m.diff_trans <= 0.0f)) f = m.base * (m.diff_all * m.diff_trans / kPi);
+    } else if (direct || has_h) {
+        float ndv = direct ? fmaxf(b.ndv, 0.001f) : b.ndv;
+        float c = direct ? ndl : 1.0f;   // EvaluateDirect's cosine
+        float ldh = fmaxf(dot(L, H), 0.0f);
+        V3 diffuse = v3(0.0f);
+        if (m.diffuse_w > 0.0f) {
+            float fd90 = 0.5f + 2.0f * m.roughness * ldh * ldh;
+            float fi = schlick_weight(ndv), fo = schlick_weight(ndl);
+            float fd = (1.0f + (fd90 - 1.0f) * fi) * (1.0f + (fd90 - 1.0f) * fo);
+            diffuse = m.base * fd * (m.diffuse_w * c / kPi);
         }
+        V3 sheen = v3(0.0f);
+        if (m.sheen > 0.0f && m.diffuse_w > 0.0f) {
+            float sb = sheen_brdf(ndv, ndl, fmaxf(ndh, 0.0f), m.sheen_roughness);
+            sheen = m.sheen * sb * m.sheen_col * c;
+        }
+        V3 specular = v3(0.0f);
+        if (!direct || spec_ok) {
+            float G = b.g1v * g1_ggx(b.fr.to_local(L), m.alpha_x, m.alpha_y);
+            V3 F = fresnel_schlick(vdh, m.f0);
+            if (direct) specular = D * G * F / fmaxf(4.0f * ndv, 1e-6f);
+            else specular = D * G / fmaxf(4.0f * ndv * ndl, 1e-7f) * F;
+        }
+        V3 clearcoat = v3(0.0f);
+        if (coat && (!direct || coat_ok)) {   // ndl > 0, and ndv > 0 past the test above (or the floor)
+            float cG = smith_g1(ndv, m.cc_alpha) * smith_g1(ndl, m.cc_alpha);
+            float cF = m.cc_f0 + (1.0f - m.cc_f0) * schlick_weight(vdh);
+            float den = 4.0f * ndv * (direct ? 1.0f : ndl);
+            clearcoat = v3(m.clearcoat * 0.25f * cD * cG * cF / fmaxf(den, direct ? 1e-6f : 1e-7f));
+        }
+        V3 ms = multiscatter_weight(m, ndv, ndl) * (1.0f / kPi) * c;
+        f = diffuse + sheen + specular + ms + clearcoat;
     }
-    V3 ms = multiscatter_weight(s, m, ndv, ndl) * (1.0f / kPi);
-    return diffuse + sheen + specular + ms + clearcoat;
-}
-
-// Pdf (:783-870): the one-sample mixture density of Sample.
-RT_D float bsdf_pdf(const Material& m, const Surface& rec, V3 V, V3 L) {
-    V3 N = rec.n;
-    float ndl = dot(N, L);
-    float ndv = dot(N, V);
-    if (ndv <= 0.0f) return 0.0f;
+    if (b.ndv <= 0.0f) return;   // Pdf is zero below the horizon
     float cos_pdf = ndl > 0.0f ? ndl / kPi : 0.0f;
     float dt_pdf = ndl < 0.0f ? -ndl / kPi : 0.0f;
     float spec_pdf = 0.0f, cc_pdf = 0.0f;
-    V3 hraw = V + L;
-    float hl2 = length_sq(hraw);
-    if (hl2 >= 1e-14f) {
-        V3 H = hraw / sqrtf(hl2);
-        float ndh = dot(N, H);
-        if (ndh > 0.0f && m.alpha > kDeltaAlpha) {
-            float sndv = fmaxf(ndv, 1e-7f);
-            Frame fr = shading_frame(rec, m);
-            V3 vl = fr.to_local(V), hl = fr.to_local(H);
-            float D = d_ggx(hl, m.alpha_x, m.alpha_y);
-            float g1v = g1_ggx(vl, m.alpha_x, m.alpha_y);
-            spec_pdf = g1v * D / (4.0f * sndv);
-        }
-        if (m.cc_alpha > kDeltaAlpha) {
-            V3 cn = rec.n;
-            float cndv = dot(cn, V), cndh = dot(cn, H);
-            if (cndv > 0.0f && cndh > 0.0f) {
-                float sc = fmaxf(cndv, 1e-7f);
-                float ca2 = m.cc_alpha * m.cc_alpha;
-                float cden = cndh * cndh * (ca2 - 1.0f) + 1.0f;
-                float cD = ca2 / (kPi * cden * cden);
-                float cg1 = smith_g1(cndv, m.cc_alpha);
-                cc_pdf = cg1 * cD / (4.0f * sc);
-            }
-        }
+    if (has_h && ndh > 0.0f) {
+        if (spec_ok) spec_pdf = b.g1v * D / (4.0f * fmaxf(b.ndv, 1e-7f));
+        if (coat && coat_ok) cc_pdf = smith_g1(b.ndv, m.cc_alpha) * cD / (4.0f * fmaxf(b.ndv, 1e-7f));
     }
-    return m.p_d * cos_pdf + m.p_sh * cos_pdf + m.p_ms * cos_pdf + m.p_s * spec_pdf + m.p_c * cc_pdf +
-           m.p_dt * dt_pdf;
+    pdf = m.p_d * cos_pdf + m.p_sh * cos_pdf + m.p_ms * cos_pdf + m.p_s * spec_pdf + m.p_c * cc_pdf +
+          m.p_dt * dt_pdf;
 }
 
 enum : int { LOBE_DIFFUSE = 0, LOBE_SPECULAR, LOBE_TRANSMISSION, LOBE_SHEEN, LOBE_MULTISCATTER, LOBE_DIFFTRANS,
@@ -1152,165 +1110,153 @@ enum : int { LOBE_DIFFUSE = 0, LOBE_SPECULAR, LOBE_TRANSMISSION, LOBE_SHEEN, LOB
 
 RT_D bool any_nonfinite(V3 a) { return !isfinite(a.x) || !isfinite(a.y) || !isfinite(a.z); }
 
-// ScatterInternal (:1176-1248) with the lobe samplers (:1263-1709). ray_dir is
-// the incoming ray direction; V = normalize(-ray_dir). When a reflection lobe
-// fails, *tried (if given) receives the direction it drew.
+// ScatterInternal's lobe choice (:1176-1248).
 // TRANSMIT = false compiles the specular-transmission lobe out, for batches in
 // which no material has specTrans > 0: there p_t is exactly 0, so the lobe is
 // never picked and subtracting p_t leaves the draw unchanged.
 template <bool TRANSMIT = true>
-RT_D bool bsdf_scatter(const SceneView& s, const Material& m, const Surface& rec, V3 ray_dir, float relative_eta,
-                       Sampler& rng, V3& att, V3& dir, int& lobe, V3* tried = nullptr) {
+RT_D int bsdf_pick_lobe(const Material& m, float rnd) {
+    if (rnd < m.p_d) return LOBE_DIFFUSE;
+    rnd -= m.p_d;
+    if (rnd < m.p_s) return LOBE_SPECULAR;
+    rnd -= m.p_s;
+    if (TRANSMIT && rnd < m.p_t) return LOBE_TRANSMISSION;
+    if (TRANSMIT) rnd -= m.p_t;
+    if (rnd < m.p_sh) return LOBE_SHEEN;
+    rnd -= m.p_sh;
+    if (rnd < m.p_ms) return LOBE_MULTISCATTER;
+    rnd -= m.p_ms;
+    if (rnd < m.p_dt) return LOBE_DIFFTRANS;
+    return LOBE_CLEARCOAT;
+}
+
+// Whether the lobe's sampler starts with two draws (all but a smooth
+// transmission and a coat seen from behind). V is ScatterInternal's own view
+// vector, normalize(-ray direction).
+template <bool TRANSMIT = true>
+RT_D bool bsdf_two_draws(const Material& m, const Surface& rec, V3 V, int lobe) {
+    if (TRANSMIT && lobe == LOBE_TRANSMISSION) return m.roughness > 0.01f;
+    return lobe != LOBE_CLEARCOAT || dot(rec.n, V) > 0.0f;
+}
+
+// The lobe samplers (:1263-1709) with the lobe and its two draws u1, u2 given
+// (bsdf_two_draws; a transmission draws once more). V as above; fr is the
+// vertex's shading frame. When the specular lobe fails, tried receives the
+// direction it drew. The four cosine lobes share one direction
+// sampler and the three microfacet lobes one half-vector sampler: lanes of a
+// warp that drew different lobes run the trigonometry together.
+template <bool TRANSMIT = true>
+RT_D bool bsdf_scatter(const Material& m, const Surface& rec, const Frame& sfr, V3 V, V3 ray_dir, float relative_eta,
+                       int lobe, float u1, float u2, Sampler& rng, V3& att, V3& dir, V3& tried) {
     V3 bc = m.base;
     V3 N = rec.n;
-    V3 V = normalize(-ray_dir);
-    float rnd = rng.next();
     bool ok = true;
-    if (rnd < m.p_d) {   // ScatterDiffuse (:1263-1306)
-        lobe = LOBE_DIFFUSE;
-        V3 sd = N + random_unit_vector(rng);
-        if (near_zero(sd)) sd = N;
-        sd = normalize(sd);
-        dir = sd;
-        float ndv = fmaxf(dot(N, V), 0.001f);
-        float ndl = fmaxf(dot(N, sd), 0.001f);
-        V3 hraw = V + sd;
-        float hl2 = length_sq(hraw);
-        V3 H = hl2 > 1e-7f ? hraw / sqrtf(hl2) : N;
-        float ldh = fmaxf(dot(sd, H), 0.0f);
-        float fd90 = 0.5f + 2.0f * m.roughness * ldh * ldh;
-        float fi = schlick_weight(ndv), fo = schlick_weight(ndl);
-        float fd = (1.0f + (fd90 - 1.0f) * fi) * (1.0f + (fd90 - 1.0f) * fo);
-        att = bc * fd;
-        att = att * (1.0f - m.diff_trans);
-        att = att / fmaxf(m.p_d, 0.1f);
-    } else if ((rnd -= m.p_d) < m.p_s) {   // ScatterSpecular (:1399-1444)
-        lobe = LOBE_SPECULAR;
-        Frame fr = shading_frame(rec, m);
-        V3 vl = fr.to_local(V);
-        float u1 = rng.next();
-        float u2 = rng.next();
-        V3 hl = sample_vndf(vl, m.alpha_x, m.alpha_y, u1, u2);
-        V3 H = fr.to_world(hl);
-        V3 L = reflect(-V, H);
-        if (dot(L, N) <= 0.0f) {
-            att = v3(0.0f);
-            dir = N;
-            ok = false;
-            if (tried) *tried = L;
-        } else {
-            dir = L;
-            float vdh = fmaxf(dot(V, H), 1e-4f);
-            V3 fres = fresnel_schlick(vdh, m.f0);
-            float g1l = g1_ggx(fr.to_local(L), m.alpha_x, m.alpha_y);
-            att = fres * g1l;
-            att = att / fmaxf(m.p_s, 0.1f);
+    const bool transmission = TRANSMIT && lobe == LOBE_TRANSMISSION;
+    if (lobe == LOBE_SPECULAR || lobe == LOBE_CLEARCOAT || transmission) {
+        bool coat = lobe == LOBE_CLEARCOAT;
+        Frame fr = sfr;
+        if (coat) {
+            tangent_frame(N, fr.t, fr.b);
+            fr.n = N;
         }
-    } else if ((rnd -= m.p_s), TRANSMIT && rnd < m.p_t) {   // ScatterTransmission (:1473-1608)
-        lobe = LOBE_TRANSMISSION;
-        bool thin = m.thin_walled != 0;
-        float eta = thin ? (1.0f / m.ior) : (relative_eta > 0.0f ? relative_eta : (rec.front ? (1.0f / m.ior) : m.ior));
-        V3 unit = normalize(ray_dir);
-        Frame fr = shading_frame(rec, m);
-        bool rough = m.roughness > 0.01f;
-        V3 Ht;
-        if (rough) {
-            V3 vl = fr.to_local(V);
-            float u1 = rng.next();
-            float u2 = rng.next();
-            Ht = fr.to_world(sample_vndf(vl, m.alpha_x, m.alpha_y, u1, u2));
-        } else {
-            Ht = N;
+        bool half = coat ? dot(N, V) > 0.0f : (!transmission || m.roughness > 0.01f);
+        V3 H = N;
+        if (half) {
+            float ax = coat ? m.cc_alpha : m.alpha_x, ay = coat ? m.cc_alpha : m.alpha_y;
+            H = fr.to_world(sample_vndf(fr.to_local(V), ax, ay, u1, u2));
         }
-        if (dot(Ht, unit) > 0.0f) Ht = -Ht;
-        float ct = fminf(dot(-unit, Ht), 1.0f);
-        float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
-        bool cannot = !thin && eta * st > 1.0f;
-        float frs = cannot ? 1.0f : fresnel_dielectric(ct, eta);
-        V3 d;
-        bool is_refl;
-        if (frs > rng.next()) {
-            d = reflect(unit, Ht);
-            is_refl = true;
-        } else if (thin) {
-            d = unit;
-            is_refl = false;
-        } else {
-            d = refract(unit, Ht, eta);
-            is_refl = false;
-        }
-        if (near_zero(d)) {
-            d = reflect(unit, N);
-            is_refl = true;
-        }
-        dir = normalize(d);
-        att = is_refl ? v3(1.0f) : m.trans_tint;
-        if (rough) {
-            V3 ll = fr.to_local(dir);
-            ll.z = fabsf(ll.z);
-            att = att * g1_ggx(ll, m.alpha_x, m.alpha_y);
-        }
-        att = att / fmaxf(m.p_t, 0.1f);
-    } else if ((rnd -= m.p_t) < m.p_sh) {   // ScatterSheen (:1354-1388)
-        lobe = LOBE_SHEEN;
-        V3 sd = N + random_unit_vector(rng);
-        if (near_zero(sd)) sd = N;
-        sd = normalize(sd);
-        dir = sd;
-        float ndv = fmaxf(dot(N, V), 1e-4f);
-        float ndl = fmaxf(dot(N, sd), 1e-4f);
-        V3 hraw = V + sd;
-        float hl2 = length_sq(hraw);
-        V3 H = hl2 > 1e-7f ? hraw / sqrtf(hl2) : N;
-        float ndh = fmaxf(dot(N, H), 0.0f);
-        float sb = sheen_brdf(ndv, ndl, ndh, m.sheen_roughness);
-        att = m.sheen * kPi * sb * m.sheen_col;
-        att = att / fmaxf(m.p_sh, 0.1f);
-    } else if ((rnd -= m.p_sh) < m.p_ms) {   // ScatterMultiscatter (:1688-1709)
-        lobe = LOBE_MULTISCATTER;
-        V3 sd = N + random_unit_vector(rng);
-        if (near_zero(sd)) sd = N;
-        sd = normalize(sd);
-        dir = sd;
-        float ndv = fmaxf(dot(N, V), 1e-3f);
-        float ndl = fmaxf(dot(N, sd), 1e-3f);
-        att = multiscatter_weight(s, m, ndv, ndl) / fmaxf(m.p_ms, 0.05f);
-    } else if ((rnd -= m.p_ms) < m.p_dt) {   // ScatterDiffTrans (:1321-1338)
-        lobe = LOBE_DIFFTRANS;
-        V3 sd = -N + random_unit_vector(rng);
-        if (near_zero(sd)) sd = -N;
-        sd = normalize(sd);
-        dir = sd;
-        att = bc * m.diff_trans;
-        att = att / fmaxf(m.p_dt, 0.05f);
-    } else {   // ScatterClearcoat (:1623-1678)
-        lobe = LOBE_CLEARCOAT;
-        V3 cn = rec.n;
-        V3 ct_, cb_;
-        tangent_frame(cn, ct_, cb_);
-        Frame fr{ct_, cb_, cn};
-        if (dot(cn, V) <= 0.0f) {
-            att = v3(0.0f);
-            dir = N;
-            ok = false;
-        } else {
-            V3 vl = fr.to_local(V);
-            float u1 = rng.next();
-            float u2 = rng.next();
-            V3 H = fr.to_world(sample_vndf(vl, m.cc_alpha, m.cc_alpha, u1, u2));
+        if (transmission) {   // ScatterTransmission (:1473-1608)
+            bool thin = m.thin_walled != 0;
+            float eta = thin ? (1.0f / m.ior)
+                             : (relative_eta > 0.0f ? relative_eta : (rec.front ? (1.0f / m.ior) : m.ior));
+            V3 unit = normalize(ray_dir);
+            V3 Ht = H;
+            if (dot(Ht, unit) > 0.0f) Ht = -Ht;
+            float ct = fminf(dot(-unit, Ht), 1.0f);
+            float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+            bool cannot = !thin && eta * st > 1.0f;
+            float frs = cannot ? 1.0f : fresnel_dielectric(ct, eta);
+            V3 d;
+            bool is_refl;
+            if (frs > rng.next()) {
+                d = reflect(unit, Ht);
+                is_refl = true;
+            } else if (thin) {
+                d = unit;
+                is_refl = false;
+            } else {
+                d = refract(unit, Ht, eta);
+                is_refl = false;
+            }
+            if (near_zero(d)) {
+                d = reflect(unit, N);
+                is_refl = true;
+            }
+            dir = normalize(d);
+            att = is_refl ? v3(1.0f) : m.trans_tint;
+            if (half) {
+                V3 ll = fr.to_local(dir);
+                ll.z = fabsf(ll.z);
+                att = att * g1_ggx(ll, m.alpha_x, m.alpha_y);
+            }
+            att = att / fmaxf(m.p_t, 0.1f);
+        } else {   // ScatterSpecular (:1399-1444), ScatterClearcoat (:1623-1678)
             V3 L = reflect(-V, H);
-            if (dot(L, N) <= 0.0f || dot(L, cn) <= 0.0f) {
+            if (!half || dot(L, N) <= 0.0f) {
                 att = v3(0.0f);
                 dir = N;
                 ok = false;
+                if (!coat) tried = L;
             } else {
                 dir = L;
-                float cndl = fmaxf(dot(cn, L), 1e-4f);
-                float cvdh = fmaxf(dot(V, H), 1e-4f);
-                float fres = m.cc_f0 + (1.0f - m.cc_f0) * schlick_weight(cvdh);
-                float g1l = smith_g1(cndl, m.cc_alpha);
-                att = v3(fres * g1l);
-                att = att / fmaxf(m.p_c, 0.1f);
+                float vdh = fmaxf(dot(V, H), 1e-4f);
+                if (coat) {
+                    float cndl = fmaxf(dot(N, L), 1e-4f);
+                    float fres = m.cc_f0 + (1.0f - m.cc_f0) * schlick_weight(vdh);
+                    att = v3(fres * smith_g1(cndl, m.cc_alpha));
+                    att = att / fmaxf(m.p_c, 0.1f);
+                } else {
+                    V3 fres = fresnel_schlick(vdh, m.f0);
+                    float g1l = g1_ggx(fr.to_local(L), m.alpha_x, m.alpha_y);
+                    att = fres * g1l;
+                    att = att / fmaxf(m.p_s, 0.1f);
+                }
+            }
+        }
+    } else {
+        V3 base = lobe == LOBE_DIFFTRANS ? -N : N;
+        V3 sd = base + unit_vector(u1, u2);
+        if (near_zero(sd)) sd = base;
+        sd = normalize(sd);
+        dir = sd;
+        if (lobe == LOBE_DIFFTRANS) {   // ScatterDiffTrans (:1321-1338)
+            att = bc * m.diff_trans;
+            att = att / fmaxf(m.p_dt, 0.05f);
+        } else if (lobe == LOBE_MULTISCATTER) {   // ScatterMultiscatter (:1688-1709)
+            float ndv = fmaxf(dot(N, V), 1e-3f);
+            float ndl = fmaxf(dot(N, sd), 1e-3f);
+            att = multiscatter_weight(m, ndv, ndl) / fmaxf(m.p_ms, 0.05f);
+        } else {
+            V3 hraw = V + sd;
+            float hl2 = length_sq(hraw);
+            V3 H = hl2 > 1e-7f ? hraw / sqrtf(hl2) : N;
+            if (lobe == LOBE_SHEEN) {   // ScatterSheen (:1354-1388)
+                float ndv = fmaxf(dot(N, V), 1e-4f);
+                float ndl = fmaxf(dot(N, sd), 1e-4f);
+                float ndh = fmaxf(dot(N, H), 0.0f);
+                float sb = sheen_brdf(ndv, ndl, ndh, m.sheen_roughness);
+                att = m.sheen * kPi * sb * m.sheen_col;
+                att = att / fmaxf(m.p_sh, 0.1f);
+            } else {   // ScatterDiffuse (:1263-1306)
+                float ndv = fmaxf(dot(N, V), 0.001f);
+                float ndl = fmaxf(dot(N, sd), 0.001f);
+                float ldh = fmaxf(dot(sd, H), 0.0f);
+                float fd90 = 0.5f + 2.0f * m.roughness * ldh * ldh;
+                float fi = schlick_weight(ndv), fo = schlick_weight(ndl);
+                float fd = (1.0f + (fd90 - 1.0f) * fi) * (1.0f + (fd90 - 1.0f) * fo);
+                att = bc * fd;
+                att = att * (1.0f - m.diff_trans);
+                att = att / fmaxf(m.p_d, 0.1f);
             }
         }
     }
@@ -1330,106 +1276,76 @@ struct BsdfSample {
 };
 
 // The rest of Sample (:893-997) once ScatterInternal has drawn (att, wo) with
-// `lobe`. Returns false for a null sample.
+// `lobe`: SAMPLE_NULL a null sample, SAMPLE_DELTA a finished one (delta, with
+// the lobe's weight), SAMPLE_EVAL one whose f and pdf are Evaluate's and Pdf's
+// (bsdf_eval_pdf, then bsdf_sample_value).
+enum : int { SAMPLE_NULL = 0, SAMPLE_DELTA, SAMPLE_EVAL };
 template <bool TRANSMIT = true>
-RT_D bool bsdf_sample_finish(const SceneView& s, const Material& m, const Surface& rec, V3 V, V3 att, V3 wo, int lobe,
-                             BsdfSample& out) {
+RT_D int bsdf_sample_kind(const Material& m, const Surface& rec, V3 att, V3 wo, int lobe, BsdfSample& out) {
     float ndwo = dot(rec.n, wo);
     out.wo = wo;
-    // Diffuse transmission and the non-delta reflection lobes both end in
-    // Evaluate + Pdf; one call site serves both (the code is long).
-    bool dt = lobe == LOBE_DIFFTRANS;
-    if (!dt) {
-        if (TRANSMIT && lobe == LOBE_TRANSMISSION) {
-            if (ndwo < 0.0f && !m.thin_walled) {
-                V3 sg = m.trans_sigma;
-                bool has_sigma = sg.x > 0.0f || sg.y > 0.0f || sg.z > 0.0f;
-                if (rec.front && has_sigma) {
-                    out.has_next_absorption = 1;
-                    out.next_absorption = sg;
-                } else if (!rec.front) {
-                    out.has_next_absorption = 1;
-                    out.next_absorption = v3(0.0f);
-                }
-                out.transition = rec.front ? 1 : 2;
+    if (lobe == LOBE_DIFFTRANS) return SAMPLE_EVAL;
+    bool delta = TRANSMIT && lobe == LOBE_TRANSMISSION;
+    if (delta) {
+        if (ndwo < 0.0f && !m.thin_walled) {
+            V3 sg = m.trans_sigma;
+            bool has_sigma = sg.x > 0.0f || sg.y > 0.0f || sg.z > 0.0f;
+            if (rec.front && has_sigma) {
+                out.has_next_absorption = 1;
+                out.next_absorption = sg;
+            } else if (!rec.front) {
+                out.has_next_absorption = 1;
+                out.next_absorption = v3(0.0f);
             }
-            out.f = att;
-            out.pdf = 1.0f;
-            out.is_delta = 1;
-            return true;
+            out.transition = rec.front ? 1 : 2;
         }
+    } else {
         if (ndwo <= 0.0f) {
             out.tried = wo;
-            return false;
+            return SAMPLE_NULL;
         }
-        bool nd_spec = lobe == LOBE_SPECULAR && m.alpha <= kDeltaAlpha;
-        bool nd_coat = lobe == LOBE_CLEARCOAT && m.cc_alpha <= kDeltaAlpha;
-        if (nd_spec || nd_coat) {
-            out.f = att;
-            out.pdf = 1.0f;
-            out.is_delta = 1;
-            return true;
-        }
+        delta = (lobe == LOBE_SPECULAR && m.alpha <= kDeltaAlpha) ||
+                (lobe == LOBE_CLEARCOAT && m.cc_alpha <= kDeltaAlpha);
     }
-    V3 fb = bsdf_eval(s, m, rec, V, wo);
-    float pb = bsdf_pdf(m, rec, V, wo);
-    if (dt && pb <= 0.0f) {   // a diffuse-transmission direction of zero density: a delta with its weight
-        out.f = att;
-        out.pdf = 1.0f;
-        out.is_delta = 1;
-        return true;
-    }
-    out.f = fb;
-    out.pdf = pb;
-    out.is_delta = 0;
-    return true;
+    if (!delta) return SAMPLE_EVAL;
+    out.f = att;
+    out.pdf = 1.0f;
+    out.is_delta = 1;
+    return SAMPLE_DELTA;
+}
+RT_D void bsdf_sample_value(V3 att, V3 f, float pdf, int lobe, BsdfSample& out) {
+    // a diffuse-transmission direction of zero density is a delta with its weight
+    bool delta = lobe == LOBE_DIFFTRANS && pdf <= 0.0f;
+    out.f = delta ? att : f;
+    out.pdf = delta ? 1.0f : pdf;
+    out.is_delta = delta;
 }
 
 // Sample (:893-997). Returns false for a null sample.
 template <bool TRANSMIT = true>
-RT_D bool bsdf_sample(const SceneView& s, const Material& m, const Surface& rec, V3 V, float relative_eta,
-                      Sampler& rng, BsdfSample& out) {
+RT_D bool bsdf_sample(const Material& m, const Surface& rec, const BsdfView& b, float relative_eta, Sampler& rng,
+                      BsdfSample& out) {
     V3 att, wo;
-    int lobe = -1;
     out.transition = 0;
     out.has_next_absorption = 0;
     out.tried = rec.n;
-    bool ok = bsdf_scatter<TRANSMIT>(s, m, rec, -V, relative_eta, rng, att, wo, lobe, &out.tried);
-    out.lobe = lobe;
-    if (!ok) return false;
-    return bsdf_sample_finish<TRANSMIT>(s, m, rec, V, att, wo, lobe, out);
-}
-
-// ShadeSampleBounce's draw: Sample, and when it returns null the legacy
-// Scatter draw the renderer falls back to (Renderer.cs:1127-1225), with fresh
-// random numbers and the ray direction itself. Both draws go through one
-// bsdf_scatter call site, so its long lobe samplers are compiled once.
-// Returns 1 with `out` filled (a sample), 2 with (latt, ldir, llobe) (the
-// legacy draw; out.lobe and out.tried describe the null sample), 0 when both
-// fail.
-template <bool TRANSMIT = true>
-RT_D int bsdf_sample_or_scatter(const SceneView& s, const Material& m, const Surface& rec, V3 V, V3 ray_dir,
-                                float relative_eta, Sampler& rng, BsdfSample& out, V3& latt, V3& ldir, int& llobe) {
-    out.transition = 0;
-    out.has_next_absorption = 0;
-    out.tried = rec.n;
-#pragma unroll 1
-    for (int pass = 0; pass < 2; pass++) {
-        V3 att, wo;
-        int lobe = -1;
-        bool ok = bsdf_scatter<TRANSMIT>(s, m, rec, pass == 0 ? -V : ray_dir, relative_eta, rng, att, wo, lobe,
-                                         pass == 0 ? &out.tried : nullptr);
-        if (pass == 1) {
-            if (!ok) return 0;
-            latt = att;
-            ldir = wo;
-            llobe = lobe;
-            return 2;
-        }
-        out.lobe = lobe;
-        if (ok && bsdf_sample_finish<TRANSMIT>(s, m, rec, V, att, wo, lobe, out)) return 1;
+    V3 vs = normalize(b.V);
+    int lobe = bsdf_pick_lobe<TRANSMIT>(m, rng.next());
+    float u1 = 0.0f, u2 = 0.0f;
+    if (bsdf_two_draws<TRANSMIT>(m, rec, vs, lobe)) {
+        u1 = rng.next();
+        u2 = rng.next();
     }
-    return 0;
+    out.lobe = lobe;
+    if (!bsdf_scatter<TRANSMIT>(m, rec, b.fr, vs, -b.V, relative_eta, lobe, u1, u2, rng, att, wo, out.tried))
+        return false;
+    int kind = bsdf_sample_kind<TRANSMIT>(m, rec, att, wo, lobe, out);
+    if (kind != SAMPLE_EVAL) return kind == SAMPLE_DELTA;
+    V3 f;
+    float pdf;
+    bsdf_eval_pdf(m, rec, b, wo, false, f, pdf);
+    bsdf_sample_value(att, f, pdf, lobe, out);
+    return true;
 }
 
 // ShadowTransmittance (:560-584) and ShadowAbsorption (:609-614).
@@ -1628,7 +1544,14 @@ __device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, 
 // GeometryLight.ComputeAreaSample (GeometryLight.cs:149-190),
 // AreaLight.IlluminateAndTestStratified (AreaLight.cs:129-178),
 // DirectionalLight.IlluminateAndTestStratified (DirectionalLight.cs:102-160).
-RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, int si, Sampler& rng) {
+// u1, u2: the first two draws of a light that light_two_draws() says takes
+// them; the others draw from rng themselves.
+RT_D bool light_two_draws(const Light& l) {
+    return l.type == LIGHT_GEOM_QUAD || l.type == LIGHT_GEOM_MESH || l.type == LIGHT_AREA ||
+           (l.type == LIGHT_DIRECTIONAL && l.angular_radius > 0.0f);
+}
+RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, int si, float u1, float u2,
+                              Sampler& rng) {
     LightSample r;
     r.occluded = 0;
     r.has_ray = 0;
@@ -1641,15 +1564,15 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
             const QuadData& q = s.quads[RT_IX(l.quad, s.n_quads)];
             int su = si % l.sqrt_samples, sv = si / l.sqrt_samples;
             float inv = 1.0f / (float)l.sqrt_samples;
-            float uu = ((float)su + rng.next()) * inv;
-            float vv = ((float)sv + rng.next()) * inv;
+            float uu = ((float)su + u1) * inv;
+            float vv = ((float)sv + u2) * inv;
             sp = q.q + uu * q.u + vv * q.v;
             ln = q.normal;
             area = q.area;
         } else {   // Mesh.SampleStratified (Mesh.cs:151-178) + Triangle.Sample
             int total = max(1, l.sqrt_samples * l.sqrt_samples);
             float stratum = 1.0f / (float)total;
-            float jit = ((float)si + rng.next()) * stratum;
+            float jit = ((float)si + u1) * stratum;
             float target = clampf(jit, 0.0f, 0.9999999f) * l.rep_area;
             int lo = 0, hi = l.mesh_count;   // lower_bound over the cumulative areas
             while (lo < hi) {
@@ -1659,7 +1582,7 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
             }
             int idx = min(max(lo, 0), l.mesh_count - 1);
             const LightTri& t = s.light_tris[RT_IX(l.mesh_first + idx, s.n_light_tris)];
-            float x1 = rng.next();
+            float x1 = u2;
             float x2 = rng.next();
             float r1 = sqrtf(x1);
             float u = 1.0f - r1;
@@ -1703,8 +1626,8 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         return light_sample_sphere_env(s, l, p, sn, si, rng);
     if (l.type == LIGHT_AREA) {
         int su = si % l.sqrt_samples, sv = si / l.sqrt_samples;
-        float ru = ((float)su + rng.next()) * l.inv_sqrt;
-        float rv = ((float)sv + rng.next()) * l.inv_sqrt;
+        float ru = ((float)su + u1) * l.inv_sqrt;
+        float rv = ((float)sv + u2) * l.inv_sqrt;
         V3 sp = l.corner + ru * l.u + rv * l.v;
         V3 tl = sp - p;
         float d2 = length_sq(tl);
@@ -1733,8 +1656,8 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
     V3 tl;
     if (l.angular_radius > 0.0f) {
         int su = si % l.sqrt_samples, sv = si / l.sqrt_samples;
-        float xi1 = ((float)su + rng.next()) * l.inv_sqrt;
-        float xi2 = ((float)sv + rng.next()) * l.inv_sqrt;
+        float xi1 = ((float)su + u1) * l.inv_sqrt;
+        float xi2 = ((float)sv + u2) * l.inv_sqrt;
         float ct = 1.0f - xi1 * (1.0f - l.cos_angular);
         float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
         float phi = 2.0f * kPi * xi2;

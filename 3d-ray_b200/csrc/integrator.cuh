@@ -179,90 +179,6 @@ RT_D V3 path_resolve(const PathState& ps, const RenderConst& rc) {
     return clamp_lum(L, rc.max_rad);
 }
 
-// NEE at a surface vertex: ComputeDirectLighting (Renderer.cs:1894-2036),
-// every light (strategy All) or one picked light (Power, Uniform). The BSDF integrand and the MIS weight are evaluated
-// before the shadow ray and the ray is dropped when they are zero (the
-// reference casts it first; only the cost differs: every draw happens in the
-// light sampler). Each unoccluded sample adds w * colour * brdf * Tr_medium,
-// times the vertex weight, through the sink.
-// MEDIUM = false compiles the participating-medium terms out (a batch none of
-// whose scenes has a medium).
-template <bool MEDIUM = true, class Sink>
-RT_D void nee_surface(const SceneView& s, const RenderConst& rc, PathState& ps, const Surface& rec,
-                      const Material& m, V3 view, Sink& sink) {
-    float view_term = shadow_terminator(rec.n, rec.n, view);
-    int to_la = ps.clamp_mode;
-    int l0 = 0, l1 = s.num_lights;
-    float p_pick = 1.0f, inv_pick = 1.0f;
-    if (rc.light_pick) {   // single-light picking (Renderer.cs:1907-1974): lightAccum / pPick
-        if (s.num_lights == 0) return;
-        l0 = pick_light(s, rc.light_pick, ps.rng.next(), p_pick);
-        l1 = l0 + 1;
-        inv_pick = p_pick > 0.0f ? 1.0f / p_pick : 0.0f;
-    }
-    for (int li = l0; li < l1; li++) {
-        const Light& l = s.lights[RT_IX(li, s.num_lights)];
-        for (int si = 0; si < l.shadow_samples; si++) {
-            LightSample ls = light_sample(s, l, rec.p, rec.n, si, ps.rng);
-            if (ls.occluded || !ls.has_ray) continue;
-            V3 brdf = bsdf_eval_direct(s, m, rec, ls.dir, view, rec.n);
-            float term = view_term * shadow_terminator(rec.n, rec.n, ls.dir);
-            brdf = brdf * term;
-            if (is_zero(brdf)) {
-                sink.skipped(ls.ray_o, ls.dir, ls.ray_tmax);
-                continue;
-            }
-            V3 tr_m = v3(1.0f);
-            if (MEDIUM && s.has_medium) tr_m = medium_tr(s, ls.dist >= kInf ? 1e30f : ls.dist);
-            float wgt = 1.0f;
-            if (!l.is_delta) {
-                float pb = bsdf_pdf(m, rec, view, ls.dir);
-                if (pb > 0.0f) {
-                    float pl = p_pick * light_pdf(s, l, rec.p, ls.dir);   // pNee = pPick * pLightSample
-                    wgt = (pl + pb > 0.0f) ? mis_weight(pl, pb, rc.mis_power) : 1.0f;
-                }
-            }
-            wgt *= inv_pick;
-            V3 c = ps.w * (wgt * ls.color * brdf * tr_m);
-            sink.shadow(ps, ls.ray_o, ls.dir, ls.ray_tmax, c, to_la);
-            sink.nee_surface(ps, li, m, rec, ls.dir, view, term, ps.w * (wgt * ls.color), ls.dist, tr_m, to_la);
-        }
-    }
-}
-
-// NEE at a medium scattering point: ComputeDirectLightingMedium
-// (Renderer.cs:2099-2206), every light or one picked light.
-template <class Sink>
-RT_D void nee_medium(const SceneView& s, const RenderConst& rc, PathState& ps, V3 p, V3 wo, Sink& sink) {
-    int to_la = ps.clamp_mode;
-    int l0 = 0, l1 = s.num_lights;
-    float p_pick = 1.0f, inv_pick = 1.0f;
-    if (rc.light_pick) {   // single-light picking in the volumetric path (Renderer.cs:2110-2160)
-        if (s.num_lights == 0) return;
-        l0 = pick_light(s, rc.light_pick, ps.rng.next(), p_pick);
-        l1 = l0 + 1;
-        inv_pick = p_pick > 0.0f ? 1.0f / p_pick : 0.0f;
-    }
-    for (int li = l0; li < l1; li++) {
-        const Light& l = s.lights[RT_IX(li, s.num_lights)];
-        for (int si = 0; si < l.shadow_samples; si++) {
-            LightSample ls = light_sample(s, l, p, v3(0.0f), si, ps.rng);
-            if (ls.occluded || !ls.has_ray) continue;
-            float ph = hg_eval(s.hg_g, wo, ls.dir);
-            V3 tr_m = medium_tr(s, ls.dist >= kInf ? 1e30f : ls.dist);
-            float wgt = 1.0f;
-            if (!l.is_delta && ph > 0.0f) {
-                float pl = p_pick * light_pdf(s, l, p, ls.dir);
-                if (pl + ph > 0.0f) wgt = mis_weight(pl, ph, rc.mis_power);
-            }
-            wgt *= inv_pick;
-            V3 c = ps.w * (wgt * ls.color * ph * tr_m);
-            sink.shadow(ps, ls.ray_o, ls.dir, ls.ray_tmax, c, to_la);
-            sink.nee_medium(ps, li, ls.dist, to_la);
-        }
-    }
-}
-
 // Russian roulette on the projected throughput (Renderer.cs:1283-1294).
 // q_used: the survival probability a surviving path was drawn against, 0 when
 // the roulette did not run.
@@ -331,85 +247,200 @@ struct NoAdjoint {
 // ps.o/ps.d as the next ray (ps.depth already decremented). MEDIUM = false
 // compiles the volumetric branch out; TRANSMIT = false the specular
 // transmission lobe and the IOR stack (no material has specTrans > 0).
+//
+// The vertex's draws run through one loop: a turn per light sample (NEE:
+// ComputeDirectLighting :1894-2036 and, at a medium scattering point,
+// ComputeDirectLightingMedium :2099-2206, over every light or one picked
+// light), then one for Sample and, when that is null, one for the legacy
+// Scatter draw (:1127-1225). The turns share their two Sobol draws, the light
+// samplers and the BSDF's evaluation, so each long stretch of code is compiled
+// once and the lanes of a warp run it together: shading is bound by
+// instruction supply. The NEE integrand and its MIS weight are evaluated
+// before the shadow ray and the ray is dropped when they are zero (the
+// reference casts it first; only the cost differs: every draw happens in the
+// light sampler).
 template <bool MEDIUM = true, bool TRANSMIT = true, class Sink>
 __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderConst& rc, PathState& ps, const Hit& h,
                                              Sink& sink) {
     bool hit = h.kind != HIT_NONE;
-    V3 beta_s = ps.beta;
+    V3 beta_s = ps.beta;   // the throughput at the vertex
     sink.aov_ray(h, ps.d);
+    bool med = false;      // a medium scattering vertex
+    Surface rec;
     if (MEDIUM && s.has_medium) {
         float tmax = hit ? h.t : 1e30f;
         float tmed;
         V3 mb;
-        bool sc = medium_sample(s, tmax, ps.rng, tmed, mb);
-        if (sc) {
-            V3 p = ps.o + ps.d * tmed;
+        med = medium_sample(s, tmax, ps.rng, tmed, mb);
+        if (med) {
+            rec.p = ps.o + ps.d * tmed;
+            rec.n = v3(0.0f);
             sink.aov_medium(tmed, ps.d);
             sink.segment(ps, tmed, SEG_MEDIUM_SCATTER);
             ps.w = ps.w * bl_factor(ps.cur_abs, tmed) * mb;
-            nee_medium(s, rc, ps, p, ps.d, sink);
-            V3 mthr = ps.beta * mb;
-            int used = rc.max_depth - ps.depth;
-            float scale = 1.0f;
-            if (used >= rc.rr_min_bounces) {
-                float q = fmaxf(mthr.x, fmaxf(mthr.y, mthr.z));
-                q = fmaxf(q, rc.rr_min_survival);
-                q = fminf(q, 0.95f);
-                if (ps.rng.next() > q) return false;
-                scale = 1.0f / q;
-                sink.roulette(ps, mthr, q, 0);
-            }
-            float ppdf;
-            V3 wi = hg_sample(s.hg_g, ps.d, ps.rng, ppdf);
-            float pv = hg_eval(s.hg_g, ps.d, wi);
-            float pw = ppdf > 1e-20f ? pv / ppdf : 0.0f;
-            ps.beta = mthr * (pw * scale);
-            ps.w = ps.w * (pw * scale);
-            ps.o = p;
-            ps.d = wi;
-            ps.prev_pdf = ppdf;
-            ps.prev_delta = 0;
-            ps.first = 0;   // a medium first vertex: no primary clamp
-            ps.depth -= 1;
-            return path_alive(ps);
+        } else {
+            sink.segment(ps, tmax, SEG_MEDIUM_PASS);
+            ps.w = ps.w * mb;
         }
-        sink.segment(ps, tmax, SEG_MEDIUM_PASS);
-        ps.w = ps.w * mb;
         beta_s = ps.beta * mb;
     }
-    if (!hit) {   // SampleSky, then TraceRay's Beer-Lambert over an infinite segment
-        if (s.sky_on) ps.add(ps.w * weight_sky(s, rc, ps.prev_pdf, ps.prev_delta) * bl_factor(ps.cur_abs, INFINITY),
-                             ps.clamp_mode);
-        sink.aov_miss(s.sky);
-        return false;
-    }
-    sink.segment(ps, h.t, SEG_ABSORPTION);
-    ps.w = ps.w * bl_factor(ps.cur_abs, h.t);
-    Surface rec = make_surface(s, h, ps.o, ps.d);
-    const Material& m = s.materials[rec.material];
-    sink.aov_surface(rec.n, m);
-    int to_la = ps.clamp_mode;
-    if (m.type != 0) {   // Emissive: Emit (front face only), no NEE, no scatter
-        if (rec.front && (m.emission.x > 0.0f || m.emission.y > 0.0f || m.emission.z > 0.0f)) {
-            V3 we = weight_emission(s, rc, m.emission, rec.material, ps.o, ps.d, ps.prev_pdf, ps.prev_delta);
-            ps.add(ps.w * we, to_la);
-            sink.emission(ps, rec.material, we, to_la);
-        }
-        return false;
-    }
-    V3 view = normalize(-ps.d);
+    V3 view;
+    const Material* mp = s.materials;
+    BsdfView bv;
     float rel_eta = 0.0f;
-    bool dielectric = TRANSMIT && !m.thin_walled && m.spec_trans_raw > 0.0f;
-    if (dielectric) rel_eta = rec.front ? (ps.iors.top() / m.ior_raw) : (m.ior_raw / ps.iors.enclosing());
-    nee_surface<MEDIUM>(s, rc, ps, rec, m, view, sink);
+    bool dielectric = false;
+    if (!MEDIUM || !med) {
+        if (!hit) {   // SampleSky, then TraceRay's Beer-Lambert over an infinite segment
+            if (s.sky_on) ps.add(ps.w * weight_sky(s, rc, ps.prev_pdf, ps.prev_delta) * bl_factor(ps.cur_abs, INFINITY),
+                                 ps.clamp_mode);
+            sink.aov_miss(s.sky);
+            return false;
+        }
+        sink.segment(ps, h.t, SEG_ABSORPTION);
+        ps.w = ps.w * bl_factor(ps.cur_abs, h.t);
+        rec = make_surface(s, h, ps.o, ps.d);
+        mp += rec.material;
+        sink.aov_surface(rec.n, *mp);
+        if (mp->type != 0) {   // Emissive: Emit (front face only), no NEE, no scatter
+            int to_la = ps.clamp_mode;
+            V3 em = mp->emission;
+            if (rec.front && (em.x > 0.0f || em.y > 0.0f || em.z > 0.0f)) {
+                V3 we = weight_emission(s, rc, em, rec.material, ps.o, ps.d, ps.prev_pdf, ps.prev_delta);
+                ps.add(ps.w * we, to_la);
+                sink.emission(ps, rec.material, we, to_la);
+            }
+            return false;
+        }
+        view = normalize(-ps.d);
+        dielectric = TRANSMIT && !mp->thin_walled && mp->spec_trans_raw > 0.0f;
+        if (dielectric) rel_eta = rec.front ? (ps.iors.top() / mp->ior_raw) : (mp->ior_raw / ps.iors.enclosing());
+        bv = bsdf_view(*mp, rec, view);
+    }
+    const Material& m = *mp;
+    const int to_la = ps.clamp_mode;
+    int li = 0, l1 = s.num_lights, si = 0;
+    float p_pick = 1.0f, inv_pick = 1.0f;
+    if (rc.light_pick && l1 > 0) {   // single-light picking (Renderer.cs:1907-1974, 2110-2160): lightAccum / pPick
+        li = pick_light(s, rc.light_pick, ps.rng.next(), p_pick);
+        l1 = li + 1;
+        inv_pick = p_pick > 0.0f ? 1.0f / p_pick : 0.0f;
+    }
     BsdfSample bs;
-    V3 att, next_o, next_d, next_beta;
-    float next_pdf;
-    int next_delta;
-    V3 latt, ldir;
-    int llobe = -1;
-    int drawn = bsdf_sample_or_scatter<TRANSMIT>(s, m, rec, view, ps.d, rel_eta, ps.rng, bs, latt, ldir, llobe);
-    if (drawn == 1) {   // ShadeSampleBounce
+    bs.transition = 0;
+    bs.has_next_absorption = 0;
+    V3 att, sdir;
+    int lobe = -1, pass = 0;
+#pragma unroll 1
+    for (;;) {
+        while (li < l1 && si >= s.lights[RT_IX(li, s.num_lights)].shadow_samples) {
+            li++;
+            si = 0;
+        }
+        const bool nee = li < l1;
+        if (MEDIUM && !nee && med) break;
+        const Light* l = nullptr;
+        V3 vs;   // ScatterInternal's view vector
+        bool two;
+        if (nee) {
+            l = s.lights + RT_IX(li, s.num_lights);
+            two = light_two_draws(*l);
+        } else {
+            vs = normalize(pass == 0 ? view : -ps.d);
+            lobe = bsdf_pick_lobe<TRANSMIT>(m, ps.rng.next());
+            two = bsdf_two_draws<TRANSMIT>(m, rec, vs, lobe);
+        }
+        float u1 = 0.0f, u2 = 0.0f;
+        if (two) {
+            u1 = ps.rng.next();
+            u2 = ps.rng.next();
+        }
+        LightSample ls;
+        V3 L;
+        if (nee) {
+            ls = light_sample(s, *l, rec.p, rec.n, si, u1, u2, ps.rng);
+            si++;
+            if (ls.occluded || !ls.has_ray) continue;
+            L = ls.dir;
+        } else {
+            V3 tried = rec.n;
+            bool ok = bsdf_scatter<TRANSMIT>(m, rec, bv.fr, vs, pass == 0 ? -view : ps.d, rel_eta, lobe, u1, u2, ps.rng,
+                                             att, sdir, tried);
+            if (pass == 1) {   // the legacy draw ends the vertex either way
+                if (!ok) return false;
+                break;
+            }
+            bs.lobe = lobe;
+            bs.tried = tried;
+            int kind = ok ? bsdf_sample_kind<TRANSMIT>(m, rec, att, sdir, lobe, bs) : SAMPLE_NULL;
+            if (kind == SAMPLE_NULL) {
+                pass = 1;
+                continue;
+            }
+            if (kind == SAMPLE_DELTA) break;
+            L = sdir;
+        }
+        V3 f;
+        float pb;   // the density of L under the vertex's own sampler
+        if (MEDIUM && med) {
+            pb = hg_eval(s.hg_g, ps.d, L);
+        } else {
+            bsdf_eval_pdf(m, rec, bv, L, nee, f, pb);
+            if (!nee) {
+                bsdf_sample_value(att, f, pb, lobe, bs);
+                break;
+            }
+        }
+        float term = 1.0f;
+        if (!MEDIUM || !med) {
+            term = shadow_terminator(rec.n, rec.n, view) * shadow_terminator(rec.n, rec.n, L);
+            f = f * term;
+            if (is_zero(f)) {
+                sink.skipped(ls.ray_o, L, ls.ray_tmax);
+                continue;
+            }
+        }
+        V3 tr_m = v3(1.0f);
+        if (MEDIUM && s.has_medium) tr_m = medium_tr(s, ls.dist >= kInf ? 1e30f : ls.dist);
+        float wgt = 1.0f;
+        if (!l->is_delta && pb > 0.0f) {
+            float pl = p_pick * light_pdf(s, *l, rec.p, L);   // pNee = pPick * pLightSample
+            if (pl + pb > 0.0f) wgt = mis_weight(pl, pb, rc.mis_power);
+        }
+        wgt *= inv_pick;
+        V3 wc = wgt * ls.color;
+        V3 c = (MEDIUM && med) ? wc * pb : wc * f;
+        if (MEDIUM) c = c * tr_m;
+        sink.shadow(ps, ls.ray_o, L, ls.ray_tmax, ps.w * c, to_la);
+        if (MEDIUM && med) sink.nee_medium(ps, li, ls.dist, to_la);
+        else sink.nee_surface(ps, li, m, rec, L, view, term, ps.w * wc, ls.dist, tr_m, to_la);
+    }
+    if (MEDIUM && med) {
+        int used = rc.max_depth - ps.depth;
+        float scale = 1.0f;
+        if (used >= rc.rr_min_bounces) {
+            float q = fmaxf(beta_s.x, fmaxf(beta_s.y, beta_s.z));
+            q = fmaxf(q, rc.rr_min_survival);
+            q = fminf(q, 0.95f);
+            if (ps.rng.next() > q) return false;
+            scale = 1.0f / q;
+            sink.roulette(ps, beta_s, q, 0);
+        }
+        float ppdf;
+        V3 wi = hg_sample(s.hg_g, ps.d, ps.rng, ppdf);
+        float pv = hg_eval(s.hg_g, ps.d, wi);
+        float pw = ppdf > 1e-20f ? pv / ppdf : 0.0f;
+        ps.beta = beta_s * (pw * scale);
+        ps.w = ps.w * (pw * scale);
+        ps.o = rec.p;
+        ps.d = wi;
+        ps.prev_pdf = ppdf;
+        ps.prev_delta = 0;
+        ps.first = 0;   // a medium first vertex: no primary clamp
+        ps.depth -= 1;
+        return path_alive(ps);
+    }
+    const bool sampled = pass == 0;   // ShadeSampleBounce, else the legacy Scatter path
+    if (sampled) {
         if (bs.is_delta) {
             att = bs.f;
         } else {
@@ -418,45 +449,39 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
             att = bs.f * a / bs.pdf;
         }
         sink.aov_bounce(bs.is_delta, bs.f);
-        next_beta = beta_s * att;
-        V3 att_pre = att, thr = next_beta;
-        float q_rr;
-        if (!russian_roulette(rc, ps.depth, att, next_beta, ps.rng, q_rr)) return false;
-        if (q_rr > 0.0f) sink.roulette(ps, thr, q_rr, ps.first);
-        sink.scatter(ps, m, rec, view, bs.wo, bs.lobe, bs.is_delta ? SCATTER_DELTA : SCATTER_SAMPLED, bs.pdf,
-                     att_pre, att, -1, bs.wo);
-        V3 off = dot(bs.wo, rec.n) >= 0.0f ? rec.n : -rec.n;
-        next_o = offset_origin(rec.p, off);
-        next_d = bs.wo;
-        next_pdf = bs.is_delta ? 0.0f : bs.pdf;
-        next_delta = bs.is_delta;
+        sdir = bs.wo;
+    } else {
+        sink.aov_bounce(false, att);   // Disney's IsDeltaScatter is false
+    }
+    V3 next_beta = beta_s * att;
+    V3 att_pre = att, thr = next_beta;
+    float q_rr;
+    if (!russian_roulette(rc, ps.depth, att, next_beta, ps.rng, q_rr)) return false;
+    if (q_rr > 0.0f) sink.roulette(ps, thr, q_rr, ps.first);
+    if (sampled) {
+        sink.scatter(ps, m, rec, view, bs.wo, bs.lobe, bs.is_delta ? SCATTER_DELTA : SCATTER_SAMPLED, bs.pdf, att_pre,
+                     att, -1, bs.wo);
+        V3 off = dot(sdir, rec.n) >= 0.0f ? rec.n : -rec.n;
+        ps.o = offset_origin(rec.p, off);
+        ps.prev_pdf = bs.is_delta ? 0.0f : bs.pdf;
+        ps.prev_delta = bs.is_delta;
         if (bs.has_next_absorption) {
             ps.cur_abs = bs.next_absorption;
             sink.interior(near_zero(bs.next_absorption) ? -1 : rec.material);
         }
         if (TRANSMIT && rc.dielectrics && bs.transition == 1) ps.iors.push(dielectric ? m.ior_raw : ps.iors.top());
         if (TRANSMIT && rc.dielectrics && bs.transition == 2) ps.iors.pop();
-    } else {   // Sample returned null: the legacy Scatter path (:1127-1225)
-        if (drawn == 0) return false;
-        V3 sdir = ldir;
-        int lobe = llobe;
-        att = latt;
-        sink.aov_bounce(false, att);   // Disney's IsDeltaScatter is false
-        next_beta = beta_s * att;
-        V3 att_pre = att, thr = next_beta;
-        float q_rr;
-        if (!russian_roulette(rc, ps.depth, att, next_beta, ps.rng, q_rr)) return false;
-        if (q_rr > 0.0f) sink.roulette(ps, thr, q_rr, ps.first);
+    } else {
         sink.scatter(ps, m, rec, view, sdir, lobe, SCATTER_LEGACY, 1.0f, att_pre, att, bs.lobe, bs.tried);
-        next_o = rec.p;
-        next_d = sdir;
-        next_pdf = 0.0f;
-        next_delta = 0;
-        if (rc.dielectrics && dielectric && dot(sdir, rec.n) < 0.0f) {
+        ps.o = rec.p;
+        ps.prev_pdf = 0.0f;
+        ps.prev_delta = 0;
+        if (TRANSMIT && rc.dielectrics && dielectric && dot(sdir, rec.n) < 0.0f) {
             if (rec.front) ps.iors.push(m.ior_raw);
             else ps.iors.pop();
         }
     }
+    ps.d = sdir;
     if (ps.first) {   // primary surface: deeper terms are clamped as one (:1380-1381)
         ps.first = 0;
         ps.clamp_mode = 1;
@@ -467,10 +492,6 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
         ps.w = ps.w * att;
     }
     ps.beta = next_beta;
-    ps.o = next_o;
-    ps.d = next_d;
-    ps.prev_pdf = next_pdf;
-    ps.prev_delta = next_delta;
     ps.depth -= 1;
     return path_alive(ps);
 }

@@ -481,20 +481,22 @@ __global__ void k_bsdf(rt::SceneView s, const RtBsdfQuery* q, int64_t n, RtBsdfR
     rt::Surface rec;
     rec.n = rt::v3(qq.n[0], qq.n[1], qq.n[2]);
     rec.tangent = rt::v3(qq.tangent[0], qq.tangent[1], qq.tangent[2]);
-    rec.bitangent = rt::v3(qq.bitangent[0], qq.bitangent[1], qq.bitangent[2]);
+    rec.has_bitangent = rt::length_sq(rt::v3(qq.bitangent[0], qq.bitangent[1], qq.bitangent[2])) > 1e-10f;
     rec.p = rt::v3(qq.point[0], qq.point[1], qq.point[2]);
     rec.front = qq.front_face;
     rec.material = qq.material;
     V3 V = rt::v3(qq.v[0], qq.v[1], qq.v[2]);
     V3 L = rt::v3(qq.l[0], qq.l[1], qq.l[2]);
-    V3 f = rt::bsdf_eval(s, m, rec, V, L);
+    rt::BsdfView bv = rt::bsdf_view(m, rec, V);
+    V3 f, fd;
+    float pdf_d;
+    rt::bsdf_eval_pdf(m, rec, bv, L, false, f, r.pdf);
     r.f[0] = f.x; r.f[1] = f.y; r.f[2] = f.z;
-    r.pdf = rt::bsdf_pdf(m, rec, V, L);
-    V3 fd = rt::bsdf_eval_direct(s, m, rec, L, V, rec.n);
+    rt::bsdf_eval_pdf(m, rec, bv, L, true, fd, pdf_d);
     r.fd[0] = fd.x; r.fd[1] = fd.y; r.fd[2] = fd.z;
     rt::Sampler rng{qq.pixel_seed, qq.sample_index, qq.dim};
     rt::BsdfSample bs;
-    bool has = rt::bsdf_sample(s, m, rec, V, 0.0f, rng, bs);
+    bool has = rt::bsdf_sample(m, rec, bv, 0.0f, rng, bs);
     r.dims_used = rng.dim - qq.dim;
     r.lobe = bs.lobe;
     r.has_sample = has ? 1 : 0;

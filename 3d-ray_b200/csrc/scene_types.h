@@ -82,6 +82,10 @@ struct Material {
     float diffuse_w;                   // (1-metallic)(1-specTrans)(1-diffTrans)
     float diff_all;                    // (1-metallic)(1-specTrans)
     float alpha_iso, e_avg;            // sqrt(ax*ay), E_avg(alpha_iso)
+    float pi_axy;                      // pi ax ay, the head of the GGX density's product
+    V3 f_ms;                           // multiscatter lobe: F_avg^2 E_avg / (1 - F_avg (1 - E_avg))
+    float ms_one_m;                    // ... and max(1 - E_avg, 1e-6)
+    float lut_mu[32];                  // E(mu, alpha_iso): the energy table's column at this roughness
 };
 
 enum : int {

@@ -152,6 +152,23 @@ float sample_eavg_host(const float* eavg, float alpha) {   // EnergyCompensation
     return eavg[a0] + (eavg[a1] - eavg[a0]) * ta;
 }
 
+// The material's share of the multiscatter weight (DisneyBsdf.cs:1906-1926)
+// and of the E lookups (EnergyCompensationLut.cs:140-165): what depends on the
+// roughness and F0 alone, with the operations a lookup would do.
+void multiscatter_constants(Material& m, const float* e) {
+    m.ms_one_m = std::fmax(1.0f - m.e_avg, 1e-6f);
+    V3 f_avg = m.f0 + (v3(1.0f) - m.f0) * (1.0f / 21.0f);
+    V3 den = v3(1.0f) - f_avg * (1.0f - m.e_avg);
+    den = v3(std::fmax(den.x, 1e-6f), std::fmax(den.y, 1e-6f), std::fmax(den.z, 1e-6f));
+    m.f_ms = f_avg * f_avg * m.e_avg / den;
+    float alpha = clampf(m.alpha_iso, 0.001f, 1.0f);
+    float fal = alpha * 32.0f - 0.5f;
+    int a0 = std::min(std::max((int)std::floor(fal), 0), 31);
+    int a1 = std::min(a0 + 1, 31);
+    float ta = clampf(fal - (float)a0, 0.0f, 1.0f);
+    for (int k = 0; k < 32; k++) m.lut_mu[k] = e[k * 32 + a0] + (e[k * 32 + a1] - e[k * 32 + a0]) * ta;
+}
+
 }  // namespace
 
 void build_energy_lut(float* e, float* eavg) {   // EnergyCompensationLut.cs:48-134
@@ -209,7 +226,7 @@ Camera make_camera(const RtCameraDesc& c, float aspect) {   // Camera.cs:26-51
     return cam;
 }
 
-Material make_material(const RtMaterialDesc& d, const float* eavg) {
+Material make_material(const RtMaterialDesc& d, const float* lut_e, const float* eavg) {
     Material m{};
     m.type = d.type;
     m.thin_walled = d.thin_walled;
@@ -294,6 +311,8 @@ Material make_material(const RtMaterialDesc& d, const float* eavg) {
     float sheen_w = m.sheen * 0.25f * diffuse_all;
     m.alpha_iso = std::sqrt(m.alpha_x * m.alpha_y);
     m.e_avg = sample_eavg_host(eavg, m.alpha_iso);
+    multiscatter_constants(m, lut_e);
+    m.pi_axy = kPi * m.alpha_x * m.alpha_y;
     float ms_w = spec_w * (1.0f - m.e_avg);
     float sum = diffuse_w + spec_w + trans_w + clear_w + sheen_w + ms_w + dt_w;
     float total = sum < 1e-6f ? 1.0f : sum;
@@ -381,7 +400,7 @@ int build_world(const RtWorldDesc* w, HostScene& sc, std::string& err, const Bui
             err = "material " + std::to_string(i) + ": thin-film iridescence is outside the GPU path";
             return RT_ERR_UNSUPPORTED;
         }
-        sc.materials.push_back(make_material(d, sc.lut_eavg.data()));
+        sc.materials.push_back(make_material(d, sc.lut_e.data(), sc.lut_eavg.data()));
     }
     const int ne = w->num_entities;
     // --- mesh BVHs (independent; built in parallel like BvhNode's Parallel.Invoke)

@@ -91,6 +91,6 @@ void build_energy_lut(float* e1024, float* eavg32);
 Camera make_camera(const RtCameraDesc& c, float aspect);
 
 // Material constants (DisneyBsdf.cs:213-293, 1104-1139, 1943-1959, 1016-1049).
-Material make_material(const RtMaterialDesc& d, const float* lut_eavg);
+Material make_material(const RtMaterialDesc& d, const float* lut_e, const float* lut_eavg);
 
 }  // namespace rt
