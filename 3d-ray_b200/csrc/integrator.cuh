@@ -109,8 +109,9 @@ RT_D V3 weight_sky(const SceneView& s, const RenderConst& rc, float prev_pdf, in
     return s.sky * mis_weight(prev_pdf, pl, rc.mis_power);
 }
 
-// Path state carried from vertex to vertex. The megakernel keeps it in
-// registers; the wavefront stores it in SoA arrays between kernels.
+// Path state carried from vertex to vertex. The megakernel and the adjoint's
+// replay keep it whole; the forward wavefront's shade keeps the part a vertex
+// works on (LeanPath, wavefront.cuh), with the same members shade_vertex uses.
 struct PathState {
     V3 o, d;          // current ray
     V3 beta;          // path throughput used by RR and the dead-path test
@@ -137,6 +138,11 @@ struct PathState {
         if (!isfinite(x.y)) mask.y = 0.0f;
         if (!isfinite(x.z)) mask.z = 0.0f;
         la = la + v3(mask.x != 0.0f ? x.x : 0.0f, mask.y != 0.0f ? x.y : 0.0f, mask.z != 0.0f ? x.z : 0.0f);
+    }
+    // The first surface vertex: its weight and attenuation, for the primary clamp.
+    RT_D void set_primary(V3 att) {
+        pre = w;
+        att0 = att;
     }
 };
 
@@ -169,7 +175,10 @@ RT_D void path_init(PathState& ps, const RenderConst& rc, int px, int py, uint32
 }
 
 // Entry test of TraceRay (Renderer.cs:1589-1603): depth and dead path.
-RT_D bool path_alive(const PathState& ps) { return ps.depth > 0 && max3(ps.beta) >= 1e-4f; }
+template <class PS>
+RT_D bool path_alive(const PS& ps) {
+    return ps.depth > 0 && max3(ps.beta) >= 1e-4f;
+}
 
 // The clamped sample radiance (ClampRadianceIndirect at the primary surface,
 // then ClampRadiance; Renderer.cs:670, 1380-1381).
@@ -209,22 +218,28 @@ enum : int { SCATTER_SAMPLED = 0, SCATTER_DELTA = 1, SCATTER_LEGACY = 2 };
 struct NoAdjoint {
     // ps.w is about to be multiplied by the factors of a segment of length t:
     // interior Beer-Lambert (all modes but SEG_MEDIUM_PASS) and the medium.
-    RT_D void segment(const PathState&, float, int) {}
+    template <class PS>
+    RT_D void segment(const PS&, float, int) {}
     // The interior absorption now belongs to material `mat` (-1: none).
     RT_D void interior(int) {}
     // An emitted-radiance term ps.w * we was just added.
-    RT_D void emission(const PathState&, int, V3, int) {}
+    template <class PS>
+    RT_D void emission(const PS&, int, V3, int) {}
     // A surface NEE sample: the term coef * brdf * term * tr_m * tr went through shadow().
-    RT_D void nee_surface(const PathState&, int, const Material&, const Surface&, V3, V3, float, V3, float, V3,
+    template <class PS>
+    RT_D void nee_surface(const PS&, int, const Material&, const Surface&, V3, V3, float, V3, float, V3,
                           int) {}
-    RT_D void nee_medium(const PathState&, int, float, int) {}
+    template <class PS>
+    RT_D void nee_medium(const PS&, int, float, int) {}
     // A path survived Russian roulette drawn against q = clamp(max(thr)); its
     // throughput now carries 1/q. first: the roulette of the first surface
     // vertex (whose attenuation becomes att0).
-    RT_D void roulette(const PathState&, V3, float, int) {}
+    template <class PS>
+    RT_D void roulette(const PS&, V3, float, int) {}
     // The vertex attenuation: att_pre before Russian roulette, att after. For
     // the legacy path, the lobe and direction of the null sample before it.
-    RT_D void scatter(const PathState&, const Material&, const Surface&, V3, V3, int, int, float, V3, V3, int, V3) {}
+    template <class PS>
+    RT_D void scatter(const PS&, const Material&, const Surface&, V3, V3, int, int, float, V3, V3, int, V3) {}
 
     // Capture hooks (the AOV probe, Renderer.cs:1051-1054, 1139-1145,
     // 1271-1277, 1657-1662, 1716-1724, 1849-1850). None of them draws from
@@ -246,7 +261,8 @@ struct NoAdjoint {
 // ShadeSampleBounce (:1235-1383). Returns true when the path continues with
 // ps.o/ps.d as the next ray (ps.depth already decremented). MEDIUM = false
 // compiles the volumetric branch out; TRANSMIT = false the specular
-// transmission lobe and the IOR stack (no material has specTrans > 0).
+// transmission lobe, the interior absorption it starts and the IOR stack (no
+// material has specTrans > 0).
 //
 // The vertex's draws run through one loop: a turn per light sample (NEE:
 // ComputeDirectLighting :1894-2036 and, at a medium scattering point,
@@ -259,8 +275,8 @@ struct NoAdjoint {
 // before the shadow ray and the ray is dropped when they are zero (the
 // reference casts it first; only the cost differs: every draw happens in the
 // light sampler).
-template <bool MEDIUM = true, bool TRANSMIT = true, class Sink>
-__device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderConst& rc, PathState& ps, const Hit& h,
+template <bool MEDIUM = true, bool TRANSMIT = true, class PS, class Sink>
+__device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderConst& rc, PS& ps, const Hit& h,
                                              Sink& sink) {
     bool hit = h.kind != HIT_NONE;
     V3 beta_s = ps.beta;   // the throughput at the vertex
@@ -277,7 +293,8 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
             rec.n = v3(0.0f);
             sink.aov_medium(tmed, ps.d);
             sink.segment(ps, tmed, SEG_MEDIUM_SCATTER);
-            ps.w = ps.w * bl_factor(ps.cur_abs, tmed) * mb;
+            if constexpr (TRANSMIT) ps.w = ps.w * bl_factor(ps.cur_abs, tmed);
+            ps.w = ps.w * mb;
         } else {
             sink.segment(ps, tmax, SEG_MEDIUM_PASS);
             ps.w = ps.w * mb;
@@ -291,13 +308,16 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
     bool dielectric = false;
     if (!MEDIUM || !med) {
         if (!hit) {   // SampleSky, then TraceRay's Beer-Lambert over an infinite segment
-            if (s.sky_on) ps.add(ps.w * weight_sky(s, rc, ps.prev_pdf, ps.prev_delta) * bl_factor(ps.cur_abs, INFINITY),
-                                 ps.clamp_mode);
+            if (s.sky_on) {
+                V3 x = ps.w * weight_sky(s, rc, ps.prev_pdf, ps.prev_delta);
+                if constexpr (TRANSMIT) x = x * bl_factor(ps.cur_abs, INFINITY);
+                ps.add(x, ps.clamp_mode);
+            }
             sink.aov_miss(s.sky);
             return false;
         }
         sink.segment(ps, h.t, SEG_ABSORPTION);
-        ps.w = ps.w * bl_factor(ps.cur_abs, h.t);
+        if constexpr (TRANSMIT) ps.w = ps.w * bl_factor(ps.cur_abs, h.t);
         rec = make_surface(s, h, ps.o, ps.d);
         mp += rec.material;
         sink.aov_surface(rec.n, *mp);
@@ -312,8 +332,10 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
             return false;
         }
         view = normalize(-ps.d);
-        dielectric = TRANSMIT && !mp->thin_walled && mp->spec_trans_raw > 0.0f;
-        if (dielectric) rel_eta = rec.front ? (ps.iors.top() / mp->ior_raw) : (mp->ior_raw / ps.iors.enclosing());
+        if constexpr (TRANSMIT) {
+            dielectric = !mp->thin_walled && mp->spec_trans_raw > 0.0f;
+            if (dielectric) rel_eta = rec.front ? (ps.iors.top() / mp->ior_raw) : (mp->ior_raw / ps.iors.enclosing());
+        }
         bv = bsdf_view(*mp, rec, view);
     }
     const Material& m = *mp;
@@ -465,28 +487,31 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
         ps.o = offset_origin(rec.p, off);
         ps.prev_pdf = bs.is_delta ? 0.0f : bs.pdf;
         ps.prev_delta = bs.is_delta;
-        if (bs.has_next_absorption) {
-            ps.cur_abs = bs.next_absorption;
-            sink.interior(near_zero(bs.next_absorption) ? -1 : rec.material);
+        if constexpr (TRANSMIT) {
+            if (bs.has_next_absorption) {
+                ps.cur_abs = bs.next_absorption;
+                sink.interior(near_zero(bs.next_absorption) ? -1 : rec.material);
+            }
+            if (rc.dielectrics && bs.transition == 1) ps.iors.push(dielectric ? m.ior_raw : ps.iors.top());
+            if (rc.dielectrics && bs.transition == 2) ps.iors.pop();
         }
-        if (TRANSMIT && rc.dielectrics && bs.transition == 1) ps.iors.push(dielectric ? m.ior_raw : ps.iors.top());
-        if (TRANSMIT && rc.dielectrics && bs.transition == 2) ps.iors.pop();
     } else {
         sink.scatter(ps, m, rec, view, sdir, lobe, SCATTER_LEGACY, 1.0f, att_pre, att, bs.lobe, bs.tried);
         ps.o = rec.p;
         ps.prev_pdf = 0.0f;
         ps.prev_delta = 0;
-        if (TRANSMIT && rc.dielectrics && dielectric && dot(sdir, rec.n) < 0.0f) {
-            if (rec.front) ps.iors.push(m.ior_raw);
-            else ps.iors.pop();
+        if constexpr (TRANSMIT) {
+            if (rc.dielectrics && dielectric && dot(sdir, rec.n) < 0.0f) {
+                if (rec.front) ps.iors.push(m.ior_raw);
+                else ps.iors.pop();
+            }
         }
     }
     ps.d = sdir;
     if (ps.first) {   // primary surface: deeper terms are clamped as one (:1380-1381)
         ps.first = 0;
         ps.clamp_mode = 1;
-        ps.pre = ps.w;
-        ps.att0 = att;
+        ps.set_primary(att);
         ps.w = v3(1.0f);
     } else {
         ps.w = ps.w * att;

@@ -829,7 +829,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     add(wreq.size() * sizeof(rt::WfRequest));
     add(key_base.size() * sizeof(int));
     add(sizeof(rt::WfCtl));
-    for (int k = 0; k < 9; k++) add((size_t)nslots * sizeof(float4));
+    for (int k = 0; k < 10; k++) add((size_t)nslots * sizeof(float4));
     add((size_t)nslots * sizeof(int));
     add((size_t)nslots * sizeof(int));
     add((size_t)nslots * sizeof(int));
@@ -873,6 +873,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     a.P.d = cv.take<float4>(nslots);
     a.P.beta = cv.take<float4>(nslots);
     a.P.w = cv.take<float4>(nslots);
+    a.P.id = cv.take<int4>(nslots);
     a.P.lp = cv.take<float4>(nslots);
     a.P.la = cv.take<float4>(nslots);
     a.P.pre = cv.take<float4>(nslots);
@@ -924,6 +925,11 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     ctl0.total = (unsigned long long)total;
     CUDA_TRY(cudaMemcpyAsync(d_views, views.data(), views.size() * sizeof(rt::SceneView), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_reqs, wreq.data(), wreq.size() * sizeof(rt::WfRequest), cudaMemcpyHostToDevice, stream));
+    const bool one = reqs.size() == 1;
+    if (one) {
+        rt::WfOne c{views[0], wreq[0].rc};
+        CUDA_TRY(cudaMemcpyToSymbolAsync(rt::c_wf_one, &c, sizeof(c), 0, cudaMemcpyHostToDevice, stream));
+    }
     CUDA_TRY(cudaMemcpyAsync(d_kb, key_base.data(), key_base.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_ctl, &ctl0, sizeof(ctl0), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_films, films.data(), films.size() * sizeof(float*), cudaMemcpyHostToDevice, stream));
@@ -991,6 +997,11 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     unsigned gsh = (unsigned)((cap + tblk - 1) / tblk);
     unsigned g256 = (unsigned)((nslots + 255) / 256);
     unsigned gsh256 = (unsigned)((cap + 255) / 256);
+    void (*shade)(const rt::WfArgs) =
+        one ? (medium ? (transmit ? rt::k_wf_shade<true, true, true> : rt::k_wf_shade<true, false, true>)
+                      : (transmit ? rt::k_wf_shade<false, true, true> : rt::k_wf_shade<false, false, true>))
+            : (medium ? (transmit ? rt::k_wf_shade<true, true, false> : rt::k_wf_shade<true, false, false>)
+                      : (transmit ? rt::k_wf_shade<false, true, false> : rt::k_wf_shade<false, false, false>));
     // ev (profiling only): boundaries between the kernel groups of one iteration.
     auto launch_iter = [&](cudaEvent_t* ev) {
         if (ev) cudaEventRecord(ev[0], stream);
@@ -1021,10 +1032,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
             }
             return;
         }
-        if (medium && transmit) rt::k_wf_shade<true, true><<<gs, blk, 0, stream>>>(a);
-        else if (medium) rt::k_wf_shade<true, false><<<gs, blk, 0, stream>>>(a);
-        else if (transmit) rt::k_wf_shade<false, true><<<gs, blk, 0, stream>>>(a);
-        else rt::k_wf_shade<false, false><<<gs, blk, 0, stream>>>(a);
+        shade<<<gs, blk, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[4], stream);   // the ray sorts' scans and scatter count as sorting
         if (a.raysort) rt::k_wf_rscan<<<1, 1024, 0, stream>>>(a.rhist, a.roff, &d_ctl->nbounce);
         if (a.shadowsort) {
@@ -1052,7 +1060,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         // alone (everything else it reads lives in the workspace), so those
         // bytes key the cached one.
         const unsigned shape[] = {(unsigned)blk, (unsigned)tblk, (unsigned)l4, (unsigned)l4_occ, (unsigned)pt,
-                                  (unsigned)medium, (unsigned)transmit, gpt_e, gpt_o, gs, gst, gsh, g256, gsh256,
+                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst, gsh, g256, gsh256,
                                   (unsigned)mode, gadj, (unsigned)adj_shmem};
         std::vector<unsigned char> key(sizeof(a) + sizeof(shape));
         std::memcpy(key.data(), &a, sizeof(a));

@@ -27,6 +27,8 @@
 // with the replay's gradient hooks and its shadow rays inline.
 #pragma once
 
+#include <type_traits>
+
 #include "adjoint.cuh"
 #include "integrator.cuh"
 
@@ -38,6 +40,7 @@ enum : int {
     PF_PREV_DELTA = 4,
     PF_FIRST = 8,
     PF_CLAMP = 16,
+    PF_DEAD = 32,       // 32, 64, 128: channels of la closed by the per-frame sanitize
 };
 
 struct WfRequest {
@@ -52,16 +55,20 @@ struct WfRequest {
                           // value through the rounding of every addition.
 };
 
-// SoA path state (144 B per slot + 16 B hit).
+// SoA path state. A vertex reads and writes o, d, beta, w (64 B) and reads id
+// (16 B) and the hit (16 B); the radiance sums lp and la are touched where a
+// term is added and at resolve, pre and att0 written at the first surface
+// vertex and read at resolve.
 struct WfPaths {
     float4* o;      // o.xyz, prev_pdf
     float4* d;      // d.xyz, flags
     float4* beta;   // beta.xyz, depth
     float4* w;      // w.xyz, rng dim
-    float4* lp;     // lp.xyz, sample index
-    float4* la;     // la.xyz, pixel (lx | ly << 16, window-local)
-    float4* pre;    // pre.xyz, request
-    float4* att0;   // att0.xyz, la mask (3 bits)
+    int4* id;       // sample index, pixel (lx | ly << 16, window-local), request, pixel seed
+    float4* lp;     // lp.xyz, -
+    float4* la;     // la.xyz, -
+    float4* pre;    // pre.xyz, -   (set once PF_CLAMP is)
+    float4* att0;   // att0.xyz, -  (set once PF_CLAMP is)
     float4* ab;     // cur_abs.xyz, ior count   (dielectric scenes)
     float* ior;     // 8 per slot                (dielectric scenes)
     float4* hit;    // t, u, v, kind << 30 | slot
@@ -153,6 +160,17 @@ struct WfArgs {
     WfAdjoint J;
 };
 
+// The scene and constants of a batch of one request, in constant memory: the
+// kernels' ONE variants read them as instruction operands instead of through
+// two dependent loads (request, then scene view) per thread. wf_render, which
+// holds a process-wide lock until its kernels are done, writes them on the
+// stream before the first iteration.
+struct WfOne {
+    SceneView view;
+    RenderConst rc;
+};
+__constant__ WfOne c_wf_one;
+
 RT_D int fbits(float f) { return __float_as_int(f); }
 RT_D float ibits(int i) { return __int_as_float(i); }
 
@@ -178,19 +196,22 @@ RT_D int wagg_next_int(int* ctr) {
     return base + rank;
 }
 
-RT_D void wf_store(const WfArgs& a, int i, const PathState& ps, int flags, int req, int pix) {
+// Stores a whole path state (the adjoint's replay).
+RT_D void wf_store(const WfArgs& a, int i, const PathState& ps, int flags) {
+    int dead = (ps.mask.x == 0.0f ? PF_DEAD : 0) | (ps.mask.y == 0.0f ? 2 * PF_DEAD : 0) |
+               (ps.mask.z == 0.0f ? 4 * PF_DEAD : 0);
     a.P.o[i] = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.prev_pdf);
-    a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(flags));
+    a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(flags | dead));
     a.P.beta[i] = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, ibits(ps.depth));
     a.P.w[i] = make_float4(ps.w.x, ps.w.y, ps.w.z, ibits((int)ps.rng.dim));
-    a.P.lp[i] = make_float4(ps.lp.x, ps.lp.y, ps.lp.z, ibits((int)ps.rng.index));
-    a.P.la[i] = make_float4(ps.la.x, ps.la.y, ps.la.z, ibits(pix));
-    a.P.pre[i] = make_float4(ps.pre.x, ps.pre.y, ps.pre.z, ibits(req));
-    int mask = (ps.mask.x != 0.0f ? 1 : 0) | (ps.mask.y != 0.0f ? 2 : 0) | (ps.mask.z != 0.0f ? 4 : 0);
-    a.P.att0[i] = make_float4(ps.att0.x, ps.att0.y, ps.att0.z, ibits(mask));
+    a.P.lp[i] = make_float4(ps.lp.x, ps.lp.y, ps.lp.z, 0.0f);
+    a.P.la[i] = make_float4(ps.la.x, ps.la.y, ps.la.z, 0.0f);
+    a.P.pre[i] = make_float4(ps.pre.x, ps.pre.y, ps.pre.z, 0.0f);
+    a.P.att0[i] = make_float4(ps.att0.x, ps.att0.y, ps.att0.z, 0.0f);
 }
 
-RT_D int wf_flags(const PathState& ps, int alive) {
+template <class PS>
+RT_D int wf_flags(const PS& ps, int alive) {
     return (alive ? PF_ALIVE : PF_DONE) | (ps.prev_delta ? PF_PREV_DELTA : 0) | (ps.first ? PF_FIRST : 0) |
            (ps.clamp_mode ? PF_CLAMP : 0);
 }
@@ -216,12 +237,12 @@ RT_D int strip_index(int lx, int ly, int ww, int wh) {
 
 RT_D uint32_t pixel_seed(int px, int py) { return ((uint32_t)px * 73856093u) ^ ((uint32_t)py * 19349663u); }
 
-// Rebuilds the register path state of slot i (lp/la read after occlude).
-RT_D void wf_load(const WfArgs& a, int i, const WfRequest& R, PathState& ps, int& flags, int& pix) {
+// Rebuilds the whole path state of slot i (the adjoint's replay).
+RT_D void wf_load(const WfArgs& a, int i, const WfRequest& R, PathState& ps) {
     float4 o = a.P.o[i], d = a.P.d[i], b = a.P.beta[i], w = a.P.w[i], lp = a.P.lp[i], la = a.P.la[i],
            pre = a.P.pre[i], at = a.P.att0[i];
-    flags = fbits(d.w);
-    pix = fbits(la.w);
+    int4 id = a.P.id[i];
+    int flags = fbits(d.w);
     ps.o = v3(o.x, o.y, o.z);
     ps.prev_pdf = o.w;
     ps.d = v3(d.x, d.y, d.z);
@@ -232,13 +253,12 @@ RT_D void wf_load(const WfArgs& a, int i, const WfRequest& R, PathState& ps, int
     ps.la = v3(la.x, la.y, la.z);
     ps.pre = v3(pre.x, pre.y, pre.z);
     ps.att0 = v3(at.x, at.y, at.z);
-    int mask = fbits(at.w);
-    ps.mask = v3((mask & 1) ? 1.0f : 0.0f, (mask & 2) ? 1.0f : 0.0f, (mask & 4) ? 1.0f : 0.0f);
+    ps.mask = v3((flags & PF_DEAD) ? 0.0f : 1.0f, (flags & (2 * PF_DEAD)) ? 0.0f : 1.0f,
+                 (flags & (4 * PF_DEAD)) ? 0.0f : 1.0f);
     ps.prev_delta = (flags & PF_PREV_DELTA) != 0;
     ps.first = (flags & PF_FIRST) != 0;
     ps.clamp_mode = (flags & PF_CLAMP) != 0;
-    int lx = pix & 0xFFFF, ly = pix >> 16;
-    ps.rng = Sampler{pixel_seed(R.x0 + lx, R.y0 + ly), (uint32_t)fbits(lp.w), (uint32_t)fbits(w.w)};
+    ps.rng = Sampler{(uint32_t)id.w, (uint32_t)id.x, (uint32_t)fbits(w.w)};
     ps.cur_abs = v3(0.0f);
     ps.iors.n = 0;
     if (R.rc.dielectrics) {
@@ -249,11 +269,58 @@ RT_D void wf_load(const WfArgs& a, int i, const WfRequest& R, PathState& ps, int
     }
 }
 
-RT_D void wf_store_media(const WfArgs& a, int i, const WfRequest& R, const PathState& ps) {
-    if (!R.rc.dielectrics) return;
+template <class PS>
+RT_D void wf_store_media(const WfArgs& a, int i, const PS& ps) {
     a.P.ab[i] = make_float4(ps.cur_abs.x, ps.cur_abs.y, ps.cur_abs.z, ibits(ps.iors.n));
     for (int k = 0; k < 8; k++) a.P.ior[(size_t)i * 8 + k] = ps.iors.slot[k];
 }
+
+// Adds a term to a slot's radiance sum (its own thread's, between extend and
+// occlude). Out of line: a vertex does so at an emitter, the sky or a
+// non-finite NEE term alone.
+__device__ __noinline__ void wf_add(float4* dst, float x, float y, float z) {
+    float4 v = *dst;
+    v.x += x;
+    v.y += y;
+    v.z += z;
+    *dst = v;
+}
+
+// The part of a path's state that a forward vertex works on. The radiance sums
+// and the primary clamp's terms stay in their slot and are written where they
+// change: a whole PathState held 15 more registers through the vertex and
+// moved 128 B more per slot.
+struct LeanMedia {   // a batch with transmissive materials
+    V3 cur_abs;
+    IorStackD iors;
+};
+struct NoMedia {};
+template <bool TRANSMIT>
+struct LeanPath : std::conditional_t<TRANSMIT, LeanMedia, NoMedia> {
+    V3 o, d, beta, w;
+    float prev_pdf;
+    int prev_delta, first, clamp_mode, depth;
+    int dead;         // PF_DEAD bits
+    Sampler rng;
+    const WfArgs* a;
+    int slot;
+
+    RT_D void add(V3 x, int to_la) {   // PathState::add
+        if (!to_la) {
+            wf_add(a->P.lp + slot, x.x, x.y, x.z);
+            return;
+        }
+        if (!isfinite(x.x)) dead |= PF_DEAD;
+        if (!isfinite(x.y)) dead |= 2 * PF_DEAD;
+        if (!isfinite(x.z)) dead |= 4 * PF_DEAD;
+        wf_add(a->P.la + slot, (dead & PF_DEAD) ? 0.0f : x.x, (dead & (2 * PF_DEAD)) ? 0.0f : x.y,
+               (dead & (4 * PF_DEAD)) ? 0.0f : x.z);
+    }
+    RT_D void set_primary(V3 att) {
+        a->P.pre[slot] = make_float4(w.x, w.y, w.z, 0.0f);
+        a->P.att0[slot] = make_float4(att.x, att.y, att.z, 0.0f);
+    }
+};
 
 RT_D int find_request(const WfRequest* reqs, int n, unsigned long long id) {
     int lo = 0, hi = n - 1;
@@ -266,7 +333,7 @@ RT_D int find_request(const WfRequest* reqs, int n, unsigned long long id) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256) k_wf_regen(WfArgs a) {
+__global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs a) {
     // Work ids come from the global counter with one atomic per block (a
     // ballot prefix over the block's free slots), and the live count with one
     // more: a per-warp atomic on one address serialised in L2.
@@ -280,42 +347,44 @@ __global__ void __launch_bounds__(256) k_wf_regen(WfArgs a) {
     int flags = in ? fbits(a.P.d[i].w) : 0;
     bool alive = in && (flags & PF_ALIVE);
     bool need = in && !alive;
-    if (MODE == WF_RECORD && need && (flags & PF_DONE)) {   // keep the finished sample's end state
-        float4 lp = a.P.lp[i], la = a.P.la[i], pre = a.P.pre[i], at = a.P.att0[i];
-        const WfRequest& R = a.reqs[RT_IX(fbits(pre.w), a.nreq)];
-        int pix = fbits(la.w);
-        int lx = pix & 0xFFFF, ly = pix >> 16;
-        long long id = R.begin + (long long)(fbits(lp.w) - R.spp0) * ((long long)R.ww * R.wh) +
-                       strip_index(lx, ly, R.ww, R.wh);
-        if (id >= 0 && id < a.J.nrec) {
-            float4* r = a.J.rec + 4 * id;
-            r[0] = make_float4(lp.x, lp.y, lp.z, ibits(flags & PF_CLAMP));
-            r[1] = la;
-            r[2] = pre;
-            r[3] = at;
-        } else {
-            atomicExch(a.err, RT_ERR_BOUNDS);
+    if (MODE != WF_REPLAY && need && (flags & PF_DONE)) {
+        // a finished sample: resolve reads lp, la and, past a first surface vertex, pre and att0
+        float4 lp = a.P.lp[i], la = a.P.la[i];
+        float4 pre = make_float4(1.0f, 1.0f, 1.0f, 0.0f), at = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        int4 id = a.P.id[i];
+        if (flags & PF_CLAMP) {
+            pre = a.P.pre[i];
+            at = a.P.att0[i];
         }
-    }
-    if (MODE == WF_RENDER && need && (flags & PF_DONE)) {   // resolve the finished sample into its film
-        // path_resolve reads lp, la, pre, att0 and the clamp flag alone: load
-        // those four records, not the whole path state
-        float4 lp = a.P.lp[i], la = a.P.la[i], pre = a.P.pre[i], at = a.P.att0[i];
-        int req = RT_IX(fbits(pre.w), a.nreq);
-        const WfRequest& R = a.reqs[req];
-        PathState ps;
-        ps.lp = v3(lp.x, lp.y, lp.z);
-        ps.la = v3(la.x, la.y, la.z);
-        ps.pre = v3(pre.x, pre.y, pre.z);
-        ps.att0 = v3(at.x, at.y, at.z);
-        ps.clamp_mode = (flags & PF_CLAMP) != 0;
-        int pix = fbits(la.w);
-        V3 L = path_resolve(ps, R.rc);
-        int lx = pix & 0xFFFF, ly = pix >> 16;
-        size_t plane = (size_t)R.ww * R.wh, k = (size_t)RT_IX(strip_index(lx, ly, R.ww, R.wh), plane);
-        atomicAdd(R.accum + k, (double)L.x);
-        atomicAdd(R.accum + plane + k, (double)L.y);
-        atomicAdd(R.accum + 2 * plane + k, (double)L.z);
+        const WfRequest& R = a.reqs[RT_IX(id.z, a.nreq)];
+        int lx = id.y & 0xFFFF, ly = id.y >> 16;
+        if (MODE == WF_RECORD) {   // keep its end state
+            long long rid = R.begin + (long long)(id.x - R.spp0) * ((long long)R.ww * R.wh) +
+                            strip_index(lx, ly, R.ww, R.wh);
+            if (rid >= 0 && rid < a.J.nrec) {
+                float4* r = a.J.rec + 4 * rid;
+                r[0] = make_float4(lp.x, lp.y, lp.z, ibits(flags & PF_CLAMP));
+                r[1] = la;
+                r[2] = pre;
+                r[3] = at;
+            } else {
+                atomicExch(a.err, RT_ERR_BOUNDS);
+            }
+        } else {   // its clamped radiance into the film
+            PathState ps;
+            ps.lp = v3(lp.x, lp.y, lp.z);
+            ps.la = v3(la.x, la.y, la.z);
+            ps.pre = v3(pre.x, pre.y, pre.z);
+            ps.att0 = v3(at.x, at.y, at.z);
+            ps.clamp_mode = (flags & PF_CLAMP) != 0;
+            V3 L = path_resolve(ps, R.rc);
+            size_t plane = (size_t)R.ww * R.wh, k = (size_t)RT_IX(strip_index(lx, ly, R.ww, R.wh), plane);
+            if (!is_zero(L)) {   // most camera rays of an open scene see nothing
+                atomicAdd(R.accum + k, (double)L.x);
+                atomicAdd(R.accum + plane + k, (double)L.y);
+                atomicAdd(R.accum + 2 * plane + k, (double)L.z);
+            }
+        }
     }
     unsigned m = __ballot_sync(full, need);
     if (lane == 0) s_warp[wid] = __popc(m);
@@ -376,8 +445,18 @@ __global__ void __launch_bounds__(256) k_wf_regen(WfArgs a) {
                 if (J.gmask & 0x3Fu)
                     for (int k = 5; k < kAdjState; k++) q[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            wf_store(a, i, ps, wf_flags(ps, al), req, lx | (ly << 16));
-            wf_store_media(a, i, R, ps);
+            a.P.o[i] = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.prev_pdf);
+            a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(wf_flags(ps, al)));
+            a.P.beta[i] = make_float4(1.0f, 1.0f, 1.0f, ibits(ps.depth));
+            a.P.w[i] = make_float4(1.0f, 1.0f, 1.0f, ibits((int)ps.rng.dim));
+            a.P.id[i] = make_int4((int)ps.rng.index, lx | (ly << 16), req, (int)ps.rng.seed);
+            a.P.lp[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            a.P.la[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (MODE == WF_REPLAY) {
+                a.P.pre[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+                a.P.att0[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            if (R.rc.dielectrics) a.P.ab[i] = make_float4(0.0f, 0.0f, 0.0f, ibits(0));
             live = true;
             if (a.raysort) {   // camera rays after the bounce rays, in work-id (pixel) order
                 long long pos = (long long)a.ctl->nbounce + (long long)(id - a.ctl->iter_first);
@@ -493,7 +572,6 @@ RT_D void extend_store(const WfArgs& a, int i, int req, const SceneView& s, cons
     }
 }
 
-// One thread per slot.
 // One thread per slot. With regroup, the block first reorders its live slots:
 // camera rays, then bounce rays by direction octant. Regen hands a block's free
 // slots consecutive pixels, so its camera rays are coherent, but they sit
@@ -503,7 +581,7 @@ RT_D void extend_store(const WfArgs& a, int i, int req, const SceneView& s, cons
 // autotuned 128 threads share an SM instead of 9: extend -2.5% per 64-spp
 // icosphere frame, for an 8-byte spill.
 template <int STACK, bool L4>
-__global__ void __launch_bounds__(256, 5) k_wf_extend(WfArgs a) {
+__global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ WfArgs a) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.raysort) {
         // order[0 .. nbounce): bounce rays by key; then this iteration's camera rays
@@ -531,7 +609,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend(WfArgs a) {
     float4 d = a.P.d[i];
     if (!(fbits(d.w) & PF_ALIVE)) return;
     float4 o = a.P.o[i];
-    int req = RT_IX(fbits(a.P.pre[i].w), a.nreq);
+    int req = a.nreq == 1 ? 0 : RT_IX(a.P.id[i].z, a.nreq);
     const SceneView& s = a.views[RT_IX(a.reqs[req].scene, a.nviews)];
     Hit h;
     trace<false, STACK, L4>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps, kInf, h, nullptr, a.err);
@@ -547,7 +625,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend(WfArgs a) {
 constexpr int kRefill = 8;
 
 template <int STACK>
-__global__ void __launch_bounds__(256) k_wf_extend_pt(WfArgs a) {
+__global__ void __launch_bounds__(256) k_wf_extend_pt(const __grid_constant__ WfArgs a) {
     const unsigned full = 0xffffffffu;
     int lane = threadIdx.x & 31;
     Walker<false, STACK> w;
@@ -571,7 +649,7 @@ __global__ void __launch_bounds__(256) k_wf_extend_pt(WfArgs a) {
                     float4 d = a.P.d[i];
                     if (fbits(d.w) & PF_ALIVE) {
                         float4 o = a.P.o[i];
-                        req = RT_IX(fbits(a.P.pre[i].w), a.nreq);
+                        req = a.nreq == 1 ? 0 : RT_IX(a.P.id[i].z, a.nreq);
                         slot = (int)i;
                         w.start(a.views[RT_IX(a.reqs[req].scene, a.nviews)], v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps, kInf,
                                 nullptr, false, 0);
@@ -624,12 +702,12 @@ __global__ void k_wf_scatter(WfArgs a) {
 }
 
 // Shadow sink of the wavefront: queue the ray with its contribution.
-// Shadow sink of the wavefront: queue the ray with its contribution.
 struct QueueShadows : NoAdjoint {
     const WfArgs* a;
     int slot;
     int scene;
-    RT_D void shadow(PathState& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
+    template <class PS>
+    RT_D void shadow(PS& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
         if (!isfinite(c.x) || !isfinite(c.y) || !isfinite(c.z)) {
             ps.add(c, to_la);   // records the per-frame sanitize in the mask
             return;
@@ -658,8 +736,8 @@ struct QueueShadows : NoAdjoint {
 
 // Under the ray sort: the continued ray's sort key and its rank in the key's
 // count (one returning atomic per distinct key in the warp).
-RT_D void wf_rank_ray(const WfArgs& a, const SceneView& s, const PathState& ps, int i) {
-    int key = ray_key(s, ps.o, ps.d, a.rkey_bits, a.rdir_bits);
+RT_D void wf_rank_ray(const WfArgs& a, const SceneView& s, V3 o, V3 d, int i) {
+    int key = ray_key(s, o, d, a.rkey_bits, a.rdir_bits);
     unsigned grp = __match_any_sync(__activemask(), key);
     int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
     int base = 0;
@@ -686,8 +764,8 @@ RT_D Hit wf_hit(const WfArgs& a, int i) {
 #ifndef RT_SHADE_MIN_BLOCKS
 #define RT_SHADE_MIN_BLOCKS 2
 #endif
-template <bool MEDIUM, bool TRANSMIT>
-__global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(WfArgs a) {
+template <bool MEDIUM, bool TRANSMIT, bool ONE>
+__global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(const __grid_constant__ WfArgs a) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     int i;
     if (a.sort) {
@@ -698,21 +776,51 @@ __global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(WfArgs a)
         if (t >= a.nslots) return;
         i = t;
     }
-    float4 d4 = a.P.d[i];
-    int flags = fbits(d4.w);
+    float4 d = a.P.d[i];
+    int flags = fbits(d.w);
     if (!(flags & PF_ALIVE)) return;
-    int req = RT_IX(fbits(a.P.pre[i].w), a.nreq);
-    const WfRequest& R = a.reqs[req];
-    const SceneView& s = a.views[RT_IX(R.scene, a.nviews)];
-    PathState ps;
-    int fl, pix;
-    wf_load(a, i, R, ps, fl, pix);
+    float4 o = a.P.o[i], b = a.P.beta[i], w = a.P.w[i];
+    int4 id = a.P.id[i];
     Hit h = wf_hit(a, i);
-    QueueShadows sink{{}, &a, i, R.scene};
-    bool alive = shade_vertex<MEDIUM, TRANSMIT>(s, R.rc, ps, h, sink);
-    wf_store(a, i, ps, wf_flags(ps, alive), req, pix);
-    wf_store_media(a, i, R, ps);
-    if (a.raysort && alive) wf_rank_ray(a, s, ps, i);
+    int req = ONE ? 0 : RT_IX(id.z, a.nreq);
+    const RenderConst& rc = ONE ? c_wf_one.rc : a.reqs[req].rc;
+    int scene = ONE ? 0 : RT_IX(a.reqs[req].scene, a.nviews);
+    const SceneView& s = ONE ? c_wf_one.view : a.views[scene];
+    LeanPath<TRANSMIT> ps;
+    ps.a = &a;
+    ps.slot = i;
+    ps.o = v3(o.x, o.y, o.z);
+    ps.prev_pdf = o.w;
+    ps.d = v3(d.x, d.y, d.z);
+    ps.beta = v3(b.x, b.y, b.z);
+    ps.depth = fbits(b.w);
+    ps.w = v3(w.x, w.y, w.z);
+    ps.rng = Sampler{(uint32_t)id.w, (uint32_t)id.x, (uint32_t)fbits(w.w)};
+    ps.prev_delta = (flags & PF_PREV_DELTA) != 0;
+    ps.first = (flags & PF_FIRST) != 0;
+    ps.clamp_mode = (flags & PF_CLAMP) != 0;
+    ps.dead = flags & (7 * PF_DEAD);
+    if constexpr (TRANSMIT) {
+        ps.cur_abs = v3(0.0f);
+        ps.iors.n = 0;
+        if (rc.dielectrics) {
+            float4 ab = a.P.ab[i];
+            ps.cur_abs = v3(ab.x, ab.y, ab.z);
+            ps.iors.n = fbits(ab.w);
+            for (int k = 0; k < 8; k++) ps.iors.slot[k] = a.P.ior[(size_t)i * 8 + k];
+        }
+    }
+    QueueShadows sink{{}, &a, i, scene};
+    bool alive = shade_vertex<MEDIUM, TRANSMIT>(s, rc, ps, h, sink);
+    a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(wf_flags(ps, alive) | ps.dead));
+    if (!alive) return;   // resolve reads the flags and the radiance sums alone
+    a.P.o[i] = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.prev_pdf);
+    a.P.beta[i] = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, ibits(ps.depth));
+    a.P.w[i] = make_float4(ps.w.x, ps.w.y, ps.w.z, ibits((int)ps.rng.dim));
+    if constexpr (TRANSMIT) {
+        if (rc.dielectrics) wf_store_media(a, i, ps);
+    }
+    if (a.raysort) wf_rank_ray(a, s, ps.o, ps.d, i);
 }
 
 // Exclusive scan of a ray-sort key histogram (kRayKeys counts) into off (one
@@ -777,7 +885,7 @@ __global__ void k_wf_sscatter(WfArgs a) {
 // Persistent any-hit for opaque batches (the walk is one any-hit traversal):
 // the dynamic-fetch scheme of k_wf_extend_pt over the shadow queue.
 template <int STACK>
-__global__ void __launch_bounds__(256) k_wf_occlude_pt(WfArgs a) {
+__global__ void __launch_bounds__(256) k_wf_occlude_pt(const __grid_constant__ WfArgs a) {
     const unsigned full = 0xffffffffu;
     int lane = threadIdx.x & 31;
     int n = min(*a.S.count, a.S.capacity);
@@ -830,7 +938,7 @@ __global__ void __launch_bounds__(256) k_wf_occlude_pt(WfArgs a) {
 // per 64-spp icosphere frame. The transparent variant keeps the full budget
 // its longer walk needs.
 template <int STACK, bool L4, bool OPAQUE>
-__global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(WfArgs a) {
+__global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid_constant__ WfArgs a) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     int n = min(*a.S.count, a.S.capacity);
     if (a.shadowsort) {

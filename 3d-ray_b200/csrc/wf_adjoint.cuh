@@ -21,7 +21,7 @@
 namespace rt {
 
 template <int STACK, bool MEDIUM, bool TRANSMIT>
-__global__ void __launch_bounds__(128) k_wf_adjoint(WfArgs a) {
+__global__ void __launch_bounds__(128) k_wf_adjoint(const __grid_constant__ WfArgs a) {
     extern __shared__ float s_acc[];
     const WfAdjoint& J = a.J;
     const int nacc = J.use_local ? J.nact : (J.use_shared ? J.nparams : 0);
@@ -39,12 +39,11 @@ __global__ void __launch_bounds__(128) k_wf_adjoint(WfArgs a) {
     }
     int flags = i >= 0 ? fbits(a.P.d[i].w) : 0;
     if (flags & PF_ALIVE) {
-        int req = RT_IX(fbits(a.P.pre[i].w), a.nreq);
+        int req = RT_IX(a.P.id[i].z, a.nreq);
         const WfRequest& R = a.reqs[req];
         const SceneView& s = a.views[RT_IX(R.scene, a.nviews)];
         PathState ps;
-        int fl, pix;
-        wf_load(a, i, R, ps, fl, pix);
+        wf_load(a, i, R, ps);
         Hit h = wf_hit(a, i);
         AdjointReplay<STACK> adj;
         adj.s = &s;
@@ -84,10 +83,10 @@ __global__ void __launch_bounds__(128) k_wf_adjoint(WfArgs a) {
             for (int c = 0; c < 3; c++)
                 for (int k = 0; k < 6; k++) f[c * 6 + k] = adj.dlb[c][k];
         }
-        wf_store(a, i, ps, wf_flags(ps, alive), req, pix);
-        wf_store_media(a, i, R, ps);
+        wf_store(a, i, ps, wf_flags(ps, alive));
+        if (R.rc.dielectrics) wf_store_media(a, i, ps);
         if (adj.abs_mat != fbits(q3.w)) q[3] = make_float4(q3.x, q3.y, q3.z, ibits(adj.abs_mat));
-        if (a.raysort && alive) wf_rank_ray(a, s, ps, i);
+        if (a.raysort && alive) wf_rank_ray(a, s, ps.o, ps.d, i);
     }
     if (J.use_local) {   // warp sums of the per-thread accumulators, then the block's
         const unsigned full = 0xffffffffu;
