@@ -821,7 +821,6 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     nslots = (nslots + 255) / 256 * 256;
     int64_t cap = (int64_t)nslots * max_shadow;
     if (cap >= ((int64_t)1 << 31) || nslots >= (1 << 29)) return fail(RT_ERR_INVALID_ARG, "wavefront too large");
-    if (cfg.shadow_limit > 0) cap = std::min<int64_t>(cap, cfg.shadow_limit);
     // Workspace layout.
     size_t need = 0;
     auto add = [&](size_t b) { need = ((need + 255) & ~(size_t)255) + b; };
@@ -830,9 +829,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     add(key_base.size() * sizeof(int));
     add(sizeof(rt::WfCtl));
     for (int k = 0; k < 10; k++) add((size_t)nslots * sizeof(float4));
-    add((size_t)nslots * sizeof(int));
-    add((size_t)nslots * sizeof(int));
-    add((size_t)nslots * sizeof(int));
+    for (int k = 0; k < 5; k++) add((size_t)nslots * sizeof(int));
     if (dielectrics) {
         add((size_t)nslots * sizeof(float4));
         add((size_t)nslots * 8 * sizeof(float));
@@ -882,6 +879,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     a.P.order = cv.take<int>(nslots);
     a.P.keys = cv.take<int>(nslots);
     a.P.rrank = cv.take<int>(nslots);
+    a.P.free = cv.take<int>(nslots);
+    a.S.cnt = cv.take<int>(nslots);
     if (dielectrics) {
         a.P.ab = cv.take<float4>(nslots);
         a.P.ior = cv.take<float>((size_t)nslots * 8);
@@ -890,7 +889,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     a.S.d = cv.take<float4>(cap);
     a.S.c = cv.take<float4>(cap);
     a.S.count = cv.take<int>(1);
-    a.S.capacity = (int)cap;
+    a.S.per = max_shadow;
+    a.S.limit = cfg.shadow_limit;
     a.S.key = cv.take<int>(cap);
     a.S.rank = cv.take<int>(cap);
     a.S.order = cv.take<int>(cap);
@@ -963,6 +963,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     bool medium = false;
     for (const RtScene* sc : scenes) medium = medium || sc->host.has_medium;
     const bool transmit = !a.opaque;
+    a.replay = mode == rt::WF_REPLAY;
     a.regroup = groups == 2;
     a.raysort = groups >= 3 && !pt;
     a.shadowsort = groups == 4 && !pt && mode != rt::WF_REPLAY;   // the replay queues no shadow rays
@@ -994,9 +995,17 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         adj_shmem = (size_t)(a.J.use_local ? a.J.nact : (a.J.use_shared ? a.J.nparams : 0)) * sizeof(float);
     unsigned gs = (unsigned)((nslots + blk - 1) / blk);
     unsigned gst = (unsigned)((nslots + tblk - 1) / tblk);
-    unsigned gsh = (unsigned)((cap + tblk - 1) / tblk);
+    dim3 gsh(gst, (unsigned)max_shadow);   // occlude and the shadow scatter: (shade's threads, records of each)
     unsigned g256 = (unsigned)((nslots + 255) / 256);
-    unsigned gsh256 = (unsigned)((cap + 255) / 256);
+    dim3 gsh256(g256, (unsigned)max_shadow);
+    // the camera kernel: persistent warps, as many as are resident
+    void (*camera)(const rt::WfArgs) =
+        mode == rt::WF_RECORD ? rt::k_wf_camera<kStack, rt::WF_RECORD, true>
+                              : (one ? rt::k_wf_camera<kStack, rt::WF_RENDER, true> : rt::k_wf_camera<kStack, rt::WF_RENDER, false>);
+    int cam_sms = 148, cam_blocks = 1;
+    cudaDeviceGetAttribute(&cam_sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cam_blocks, camera, 128, 0);
+    unsigned gcam = (unsigned)std::min<int64_t>((int64_t)std::max(1, cam_blocks) * cam_sms, (nslots + 127) / 128);
     void (*shade)(const rt::WfArgs) =
         one ? (medium ? (transmit ? rt::k_wf_shade<true, true, true> : rt::k_wf_shade<true, false, true>)
                       : (transmit ? rt::k_wf_shade<false, true, true> : rt::k_wf_shade<false, false, true>))
@@ -1009,6 +1018,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         if (mode == rt::WF_RECORD) rt::k_wf_regen<rt::WF_RECORD><<<g256, 256, 0, stream>>>(a);
         else if (mode == rt::WF_REPLAY) rt::k_wf_regen<rt::WF_REPLAY><<<g256, 256, 0, stream>>>(a);
         else rt::k_wf_regen<rt::WF_RENDER><<<g256, 256, 0, stream>>>(a);
+        if (mode != rt::WF_REPLAY) camera<<<gcam, 128, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[1], stream);
         if (l4) rt::k_wf_extend<kStack, true><<<gst, tblk, 0, stream>>>(a);
         else if (pt) rt::k_wf_extend_pt<kStack><<<gpt_e, tblk, 0, stream>>>(a);
@@ -1060,7 +1070,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         // alone (everything else it reads lives in the workspace), so those
         // bytes key the cached one.
         const unsigned shape[] = {(unsigned)blk, (unsigned)tblk, (unsigned)l4, (unsigned)l4_occ, (unsigned)pt,
-                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst, gsh, g256, gsh256,
+                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst, (unsigned)max_shadow, g256, gcam,
                                   (unsigned)mode, gadj, (unsigned)adj_shmem};
         std::vector<unsigned char> key(sizeof(a) + sizeof(shape));
         std::memcpy(key.data(), &a, sizeof(a));
@@ -1083,7 +1093,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
             ws.exec_key = std::move(key);
         }
     }
-    int per_iter = (mode == rt::WF_REPLAY ? 4 : 5) + (sort ? 2 : 0) + (a.raysort ? 1 : 0) + (a.shadowsort ? 2 : 0);
+    int per_iter = (mode == rt::WF_REPLAY ? 4 : 6) + (sort ? 2 : 0) + (a.raysort ? 1 : 0) + (a.shadowsort ? 2 : 0);
     int max_depth = 1;
     for (auto& q : wreq) max_depth = std::max(max_depth, q.rc.max_depth);
     int64_t limit = (total / nslots + 2) * (int64_t)(max_depth + 2) + 64;

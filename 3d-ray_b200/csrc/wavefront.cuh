@@ -1,11 +1,12 @@
 // Persistent, request-batched wavefront form of the bounce loop.
 //
 // A fixed pool of path slots (the wavefront) is advanced one vertex per
-// iteration by four small kernels instead of one large one:
-//   regen   : resolve finished samples into their request's film, then refill
-//             the slot with the next (request, sample, pixel) work item from a
-//             global counter (warp-aggregated atomics): camera ray generation.
-//   extend  : closest hit of every live path's current ray.
+// iteration by five small kernels instead of one large one:
+//   regen   : resolve finished samples into their request's film and list the
+//             free slots.
+//   camera  : take the next (request, sample, pixel) work items, trace their
+//             camera rays and start the paths that hit something in free slots.
+//   extend  : closest hit of every other live path's current ray.
 //   shade   : one TraceRay vertex (medium, emission, NEE, BSDF sample, RR).
 //             Shadow rays go to a queue instead of being traced inline.
 //   occlude : any-hit (or the transparent walk) of the queued shadow rays;
@@ -20,9 +21,10 @@
 //
 // The same loop runs the path-replay adjoint (rt_adjoint) in two passes over
 // a range of samples: WF_RECORD renders them with the forward kernels and
-// regen stores each finished sample's end state (lp, la, pre, att0) by work id
-// instead of adding it to a film; WF_REPLAY traces the same samples again,
-// regen seeds each new path with the adjoints of its recorded resolve, and
+// regen and camera store each finished sample's end state (lp, la, pre, att0) by
+// work id instead of adding it to a film; WF_REPLAY traces the same samples
+// again, regen starts each path itself with the adjoints of its recorded
+// resolve, and
 // k_wf_adjoint (wf_adjoint.cuh) replaces shade and occlude: it runs the vertex
 // with the replay's gradient hooks and its shadow rays inline.
 #pragma once
@@ -41,6 +43,7 @@ enum : int {
     PF_FIRST = 8,
     PF_CLAMP = 16,
     PF_DEAD = 32,       // 32, 64, 128: channels of la closed by the per-frame sanitize
+    PF_TRACED = 256,    // a camera path of this iteration: its hit is in place, extend skips it
 };
 
 struct WfRequest {
@@ -72,17 +75,24 @@ struct WfPaths {
     float4* ab;     // cur_abs.xyz, ior count   (dielectric scenes)
     float* ior;     // 8 per slot                (dielectric scenes)
     float4* hit;    // t, u, v, kind << 30 | slot
+    int* free;      // free slots, for the iteration's camera paths
     int* order;     // slot order for shade (material-sorted or identity); for extend under the ray sort
     int* keys;      // material key per slot (sorting); after shade, the ray sort's key
     int* rrank;     // ray sort: the slot's rank among the rays of its key
 };
 
+// Shadow records. Thread t of shade writes its vertex's k-th record at
+// k * nslots + t and the number it wrote to cnt[t]: no queue counter (a
+// returning atomic per light sample in the middle of the vertex), and the
+// records of a warp lie side by side.
 struct WfShadow {
     float4* o;    // o.xyz, tmax
     float4* d;    // d.xyz, slot << 1 | to_la
     float4* c;    // contribution.xyz, scene
+    int* cnt;     // per shade thread: its records
+    int per;      // records a vertex can write (the most of any scene)
+    int limit;    // test only, > 0: at most this many records per iteration, counted in *count
     int* count;
-    int capacity;
     int* key;     // shadow sort: the record's ray_key
     int* rank;    // shadow sort: its rank among the records of its key
     int* order;   // shadow sort: records in key order, for occlude
@@ -98,7 +108,8 @@ struct WfCtl {
     unsigned occ_next;          // persistent occlude: next shadow record to fetch
     unsigned long long iter_first;   // ray sort: the first work id of this iteration
     int nbounce;                // ray sort: bounce rays shade continued (order[0 .. nbounce))
-    int nshadow;                // shadow sort: records counted by key (the queue's count)
+    int nshadow;                // shadow sort: records counted by key
+    int nfree, free_next;       // slots in the free list, and the first one not yet reserved
     int hist[256];              // material histogram (sorting)
 };
 
@@ -142,7 +153,8 @@ struct WfArgs {
     int nkeys;        // material keys (sum over scenes) for sorting
     const int* key_base;   // per scene: first key
     int regroup;      // extend/occlude regroup their block's rays by kind (block_group)
-    int raysort;      // extend walks bounce rays sorted by ray_key, then camera rays in pixel order
+    int replay;       // the replay pass: regen starts its camera paths, extend traces them
+    int raysort;      // extend walks the bounce rays sorted by ray_key
     int rkey_bits;    // ray_key of bounce rays: origin cell bits per axis (0 .. 4)
     int rdir_bits;    // ray_key of bounce rays: direction bits (0, 3: octant, or an even count up to 8)
     int skey_bits;    // the same two for shadow records
@@ -332,11 +344,20 @@ RT_D int find_request(const WfRequest* reqs, int n, unsigned long long id) {
     return lo;
 }
 
+// Adds a sample's clamped radiance to its request's film sums.
+RT_D void film_add(const WfRequest& R, int lx, int ly, V3 L) {
+    size_t plane = (size_t)R.ww * R.wh, k = (size_t)RT_IX(strip_index(lx, ly, R.ww, R.wh), plane);
+    atomicAdd(R.accum + k, (double)L.x);
+    atomicAdd(R.accum + plane + k, (double)L.y);
+    atomicAdd(R.accum + 2 * plane + k, (double)L.z);
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs a) {
-    // Work ids come from the global counter with one atomic per block (a
-    // ballot prefix over the block's free slots), and the live count with one
-    // more: a per-warp atomic on one address serialised in L2.
+    // The free slots go to the free list, or in the replay to the next work ids,
+    // with one atomic per block (a ballot prefix over the block's free slots),
+    // and the live count with one more: a per-warp atomic on one address
+    // serialised in L2.
     __shared__ int s_warp[8];   // blockDim 256: per-warp free-slot offsets
     __shared__ unsigned long long s_base;
     __shared__ int s_live;
@@ -378,12 +399,7 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
             ps.att0 = v3(at.x, at.y, at.z);
             ps.clamp_mode = (flags & PF_CLAMP) != 0;
             V3 L = path_resolve(ps, R.rc);
-            size_t plane = (size_t)R.ww * R.wh, k = (size_t)RT_IX(strip_index(lx, ly, R.ww, R.wh), plane);
-            if (!is_zero(L)) {   // most camera rays of an open scene see nothing
-                atomicAdd(R.accum + k, (double)L.x);
-                atomicAdd(R.accum + plane + k, (double)L.y);
-                atomicAdd(R.accum + 2 * plane + k, (double)L.z);
-            }
+            if (!is_zero(L)) film_add(R, lx, ly, L);
         }
     }
     unsigned m = __ballot_sync(full, need);
@@ -397,7 +413,9 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
             s_warp[w] = tot;
             tot += c;
         }
-        s_base = tot ? atomicAdd(&a.ctl->next, (unsigned long long)tot) : 0ull;
+        s_base = 0ull;
+        if (tot && MODE == WF_REPLAY) s_base = atomicAdd(&a.ctl->next, (unsigned long long)tot);
+        else if (tot) s_base = (unsigned long long)atomicAdd(&a.ctl->nfree, tot);
     }
     __syncthreads();
     bool live = alive;
@@ -408,7 +426,10 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
         if (pos < a.ctl->nbounce) a.P.order[pos] = i;
         else atomicExch(a.err, RT_ERR_BOUNDS);
     }
-    if (need) {
+    if (MODE != WF_REPLAY && need) {
+        a.P.d[i].w = ibits(0);
+        a.P.free[RT_IX((int)s_base + s_warp[wid] + __popc(m & ((1u << lane) - 1u)), a.nslots)] = i;
+    } else if (need) {
         unsigned long long id = s_base + (unsigned long long)(s_warp[wid] + __popc(m & ((1u << lane) - 1u)));
         if (id >= a.ctl->total) {
             a.P.d[i].w = ibits(0);
@@ -424,27 +445,26 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
             PathState ps;
             path_init(ps, R.rc, R.x0 + lx, R.y0 + ly, (uint32_t)(R.spp0 + s));
             int al = path_alive(ps);
-            if (MODE == WF_REPLAY) {   // the adjoints of the recorded resolve; no gradient, no replay
-                const WfAdjoint& J = a.J;
-                size_t plane = (size_t)J.W * J.H, fi = (size_t)(R.y0 + ly) * J.W + (R.x0 + lx);
-                V3 delta = v3(J.dimg[fi], J.dimg[plane + fi], J.dimg[2 * plane + fi]) * J.inv_spp;
-                AdjResolve ar{};
-                if (id < (unsigned long long)J.nrec && !is_zero(delta)) {
-                    const float4* r = J.rec + 4 * id;
-                    float4 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
-                    ar = adjoint_resolve(R.rc, v3(r0.x, r0.y, r0.z), v3(r1.x, r1.y, r1.z), v3(r2.x, r2.y, r2.z),
-                                         v3(r3.x, r3.y, r3.z), fbits(r0.w) != 0, delta);
-                }
-                al = al && !is_zero(ar.g_a);
-                float4* q = J.st + kAdjState * (size_t)i;
-                q[0] = make_float4(ar.tot_a.x, ar.tot_a.y, ar.tot_a.z, ar.tot_la.x);
-                q[1] = make_float4(ar.tot_la.y, ar.tot_la.z, ar.g_a.x, ar.g_a.y);
-                q[2] = make_float4(ar.g_a.z, ar.g_la.x, ar.g_la.y, ar.g_la.z);
-                q[3] = make_float4(ar.g_att0.x, ar.g_att0.y, ar.g_att0.z, ibits(-1));
-                q[4] = make_float4(ar.delta.x, ar.delta.y, ar.delta.z, ar.val);
-                if (J.gmask & 0x3Fu)
-                    for (int k = 5; k < kAdjState; k++) q[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            // the adjoints of the recorded resolve; no gradient, no replay
+            const WfAdjoint& J = a.J;
+            size_t plane = (size_t)J.W * J.H, fi = (size_t)(R.y0 + ly) * J.W + (R.x0 + lx);
+            V3 delta = v3(J.dimg[fi], J.dimg[plane + fi], J.dimg[2 * plane + fi]) * J.inv_spp;
+            AdjResolve ar{};
+            if (id < (unsigned long long)J.nrec && !is_zero(delta)) {
+                const float4* r = J.rec + 4 * id;
+                float4 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
+                ar = adjoint_resolve(R.rc, v3(r0.x, r0.y, r0.z), v3(r1.x, r1.y, r1.z), v3(r2.x, r2.y, r2.z),
+                                     v3(r3.x, r3.y, r3.z), fbits(r0.w) != 0, delta);
             }
+            al = al && !is_zero(ar.g_a);
+            float4* q = J.st + kAdjState * (size_t)i;
+            q[0] = make_float4(ar.tot_a.x, ar.tot_a.y, ar.tot_a.z, ar.tot_la.x);
+            q[1] = make_float4(ar.tot_la.y, ar.tot_la.z, ar.g_a.x, ar.g_a.y);
+            q[2] = make_float4(ar.g_a.z, ar.g_la.x, ar.g_la.y, ar.g_la.z);
+            q[3] = make_float4(ar.g_att0.x, ar.g_att0.y, ar.g_att0.z, ibits(-1));
+            q[4] = make_float4(ar.delta.x, ar.delta.y, ar.delta.z, ar.val);
+            if (J.gmask & 0x3Fu)
+                for (int k = 5; k < kAdjState; k++) q[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             a.P.o[i] = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.prev_pdf);
             a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(wf_flags(ps, al)));
             a.P.beta[i] = make_float4(1.0f, 1.0f, 1.0f, ibits(ps.depth));
@@ -452,10 +472,8 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
             a.P.id[i] = make_int4((int)ps.rng.index, lx | (ly << 16), req, (int)ps.rng.seed);
             a.P.lp[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             a.P.la[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (MODE == WF_REPLAY) {
-                a.P.pre[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-                a.P.att0[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
+            a.P.pre[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+            a.P.att0[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (R.rc.dielectrics) a.P.ab[i] = make_float4(0.0f, 0.0f, 0.0f, ibits(0));
             live = true;
             if (a.raysort) {   // camera rays after the bounce rays, in work-id (pixel) order
@@ -556,7 +574,7 @@ RT_D int ray_key(const SceneView& s, V3 o, V3 d, int cb, int db) {
 }
 
 // Stores slot i's closest hit and, when sorting, its material key.
-RT_D void extend_store(const WfArgs& a, int i, int req, const SceneView& s, const Hit& h) {
+RT_D void hit_store(const WfArgs& a, int i, int req, const SceneView& s, const Hit& h) {
     int packed = h.kind == HIT_NONE ? 0 : ((h.kind << 30) | h.slot);
     a.P.hit[i] = make_float4(h.t, h.u, h.v, ibits(packed));
     if (a.sort) {   // material key for the counting sort
@@ -572,6 +590,13 @@ RT_D void extend_store(const WfArgs& a, int i, int req, const SceneView& s, cons
     }
 }
 
+// A bounce ray's closest hit. One that leaves a scene with neither medium nor
+// sky ends its path here: shade would add nothing.
+RT_D void extend_store(const WfArgs& a, int i, int flags, int req, const SceneView& s, const Hit& h) {
+    if (h.kind == HIT_NONE && !s.has_medium && !s.sky_on) a.P.d[i].w = ibits((flags & ~PF_ALIVE) | PF_DONE);
+    else hit_store(a, i, req, s, h);
+}
+
 // One thread per slot. With regroup, the block first reorders its live slots:
 // camera rays, then bounce rays by direction octant. Regen hands a block's free
 // slots consecutive pixels, so its camera rays are coherent, but they sit
@@ -584,10 +609,13 @@ template <int STACK, bool L4>
 __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ WfArgs a) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.raysort) {
-        // order[0 .. nbounce): bounce rays by key; then this iteration's camera rays
-        unsigned long long nx = a.ctl->next < a.ctl->total ? a.ctl->next : a.ctl->total;
-        long long ncam = (long long)nx - (long long)a.ctl->iter_first;
-        long long n = (long long)a.ctl->nbounce + (ncam > 0 ? ncam : 0);
+        // order[0 .. nbounce): bounce rays by key; then, in the replay, this iteration's camera rays
+        long long n = a.ctl->nbounce;
+        if (a.replay) {
+            unsigned long long nx = a.ctl->next < a.ctl->total ? a.ctl->next : a.ctl->total;
+            long long ncam = (long long)nx - (long long)a.ctl->iter_first;
+            if (ncam > 0) n += ncam;
+        }
         if ((long long)i >= n || i >= a.nslots) return;
         i = a.P.order[i];
         if (i < 0) return;
@@ -598,7 +626,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ Wf
         if (i < a.nslots) {
             float4 d = a.P.d[i];
             int fl = fbits(d.w);
-            if (fl & PF_ALIVE) cls = (fl & PF_FIRST) ? 0 : 1 + octant(d.x, d.y, d.z);
+            if ((fl & PF_ALIVE) && !(fl & PF_TRACED)) cls = (fl & PF_FIRST) ? 0 : 1 + octant(d.x, d.y, d.z);
         }
         int n = block_group<9>(i, cls, s_idx, s_cnt, &s_tot);
         if ((int)threadIdx.x >= n) return;
@@ -607,13 +635,14 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ Wf
         return;
     }
     float4 d = a.P.d[i];
-    if (!(fbits(d.w) & PF_ALIVE)) return;
+    int flags = fbits(d.w);
+    if (!(flags & PF_ALIVE) || (flags & PF_TRACED)) return;
     float4 o = a.P.o[i];
     int req = a.nreq == 1 ? 0 : RT_IX(a.P.id[i].z, a.nreq);
     const SceneView& s = a.views[RT_IX(a.reqs[req].scene, a.nviews)];
     Hit h;
     trace<false, STACK, L4>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps, kInf, h, nullptr, a.err);
-    extend_store(a, i, req, s, h);
+    extend_store(a, i, flags, req, s, h);
 }
 
 // Persistent form with dynamic ray fetch (Aila and Laine 2009): a grid sized
@@ -629,7 +658,7 @@ __global__ void __launch_bounds__(256) k_wf_extend_pt(const __grid_constant__ Wf
     const unsigned full = 0xffffffffu;
     int lane = threadIdx.x & 31;
     Walker<false, STACK> w;
-    int slot = -1, req = 0;
+    int slot = -1, req = 0, flags = 0;
     bool exhausted = false;
     for (;;) {
         bool idle = slot < 0 && !exhausted;
@@ -647,7 +676,8 @@ __global__ void __launch_bounds__(256) k_wf_extend_pt(const __grid_constant__ Wf
                     exhausted = true;
                 } else {
                     float4 d = a.P.d[i];
-                    if (fbits(d.w) & PF_ALIVE) {
+                    flags = fbits(d.w);
+                    if ((flags & PF_ALIVE) && !(flags & PF_TRACED)) {
                         float4 o = a.P.o[i];
                         req = a.nreq == 1 ? 0 : RT_IX(a.P.id[i].z, a.nreq);
                         slot = (int)i;
@@ -661,11 +691,126 @@ __global__ void __launch_bounds__(256) k_wf_extend_pt(const __grid_constant__ Wf
         if (slot >= 0) {
             const SceneView& s = a.views[RT_IX(a.reqs[req].scene, a.nviews)];
             if (w.step(s, nullptr, a.err)) {
-                extend_store(a, slot, req, s, w.best);
+                extend_store(a, slot, flags, req, s, w.best);
                 slot = -1;
             }
         }
     }
+}
+
+// Resident blocks of 128 per SM the camera kernel is compiled for; a build knob.
+#ifndef RT_CAMERA_MIN_BLOCKS
+#define RT_CAMERA_MIN_BLOCKS 8
+#endif
+// Camera paths: generation and first hit in one kernel, on persistent warps.
+// A warp takes 32 consecutive work ids (an 8x4 block of pixels), traces their
+// camera rays and gives a slot only to the paths that go on: a ray that
+// leaves a scene without a medium is a finished sample (the sky's radiance or
+// nothing) and never touches the path state. In an open scene those are most
+// camera rays: with a slot each, they cost the state's writes and reads in
+// regen, extend and shade, and left few bounce rays per iteration to sort.
+// The paths that go on store only what their first vertex does not know: shade
+// sets the rest of a PF_FIRST path itself.
+//
+// Slots are reserved from the free list 32 at a time before the rays are
+// traced, so that every hit has one; what a warp does not use stays free until
+// the next iteration. Once the list is dry a warp goes on with what it has
+// left, down to half a warp of rays (but at least one round). Every round
+// consumes work ids, so the loop ends.
+template <int STACK, int MODE, bool ONE>
+__global__ void __launch_bounds__(128, RT_CAMERA_MIN_BLOCKS) k_wf_camera(const __grid_constant__ WfArgs a) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long total = a.ctl->total;
+    const int nfree = a.ctl->nfree;   // complete: regen has run
+    int b0 = 0, n0 = 0, b1 = 0, n1 = 0;   // the warp's reserved ranges of the free list
+    int kept = 0;
+    bool dry = false, first = true;
+    for (;;) {
+        if (!dry && n0 + n1 < 32) {
+            int b = 0;
+            if (lane == 0) b = atomicAdd(&a.ctl->free_next, 32);
+            b = __shfl_sync(full, b, 0);
+            b1 = b;
+            n1 = min(32, max(0, nfree - b));   // n1 was 0: n0 + n1 < 32 with n1 in {0, 32}
+            dry = n1 < 32;
+            if (n0 == 0) {
+                b0 = b1;
+                n0 = n1;
+                n1 = 0;
+            }
+        }
+        int n = min(32, n0 + n1);
+        if (n == 0 || (dry && n < 16 && !first)) break;
+        first = false;
+        unsigned long long id0 = 0;
+        if (lane == 0) id0 = atomicAdd(&a.ctl->next, (unsigned long long)n);
+        id0 = __shfl_sync(full, id0, 0);
+        if (id0 >= total) break;
+        unsigned long long id = id0 + (unsigned long long)lane;
+        bool keep = false;
+        int req = 0, pix = 0, seed = 0, sample = 0;
+        V3 dir = v3(0.0f);
+        Hit h;
+        h.kind = HIT_NONE;
+        if (lane < n && id < total) {
+            if (!ONE) req = RT_IX(find_request(a.reqs, a.nreq, id), a.nreq);
+            const WfRequest& R = a.reqs[req];
+            const RenderConst& rc = ONE ? c_wf_one.rc : R.rc;
+            const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(R.scene, a.nviews)];
+            long long local = (long long)(id - (unsigned long long)R.begin);
+            long long npix = (long long)R.ww * R.wh;
+            int lx, ly;
+            strip_pixel((int)(local % npix), R.ww, R.wh, lx, ly);
+            PathState ps;
+            path_init(ps, rc, R.x0 + lx, R.y0 + ly, (uint32_t)(R.spp0 + (int)(local / npix)));
+            pix = lx | (ly << 16);
+            seed = (int)ps.rng.seed;
+            sample = (int)ps.rng.index;
+            dir = ps.d;
+            V3 L = v3(0.0f);
+            if (path_alive(ps)) {
+                traverse<false, STACK>(s, ps.o, ps.d, kEps, kInf, h, nullptr, a.err);
+                keep = h.kind != HIT_NONE || s.has_medium;
+                if (!keep && s.sky_on) L = L + weight_sky(s, rc, 0.0f, 1);   // shade_vertex's sky term, w = 1
+            }
+            if (!keep && MODE == WF_RECORD) {
+                if ((long long)id < a.J.nrec) {
+                    float4* r = a.J.rec + 4 * id;
+                    r[0] = make_float4(L.x, L.y, L.z, ibits(0));
+                    r[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    r[2] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+                    r[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                } else {
+                    atomicExch(a.err, RT_ERR_BOUNDS);
+                }
+            } else if (!keep && !is_zero(L)) {
+                film_add(R, lx, ly, clamp_lum(L, rc.max_rad));
+            }
+        }
+        unsigned m = __ballot_sync(full, keep);
+        int c = __popc(m), rank = __popc(m & ((1u << lane) - 1u));
+        if (keep) {
+            int i = RT_IX(a.P.free[rank < n0 ? b0 + rank : b1 + (rank - n0)], a.nslots);
+            a.P.d[i] = make_float4(dir.x, dir.y, dir.z,
+                                   ibits(PF_ALIVE | PF_PREV_DELTA | PF_FIRST | PF_TRACED));
+            a.P.id[i] = make_int4(sample, pix, req, seed);
+            a.P.lp[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            a.P.la[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(a.reqs[req].scene, a.nviews)];
+            hit_store(a, i, req, s, h);
+        }
+        kept += c;
+        if (c >= n0) {
+            b0 = b1 + (c - n0);
+            n0 = n1 - (c - n0);
+            n1 = 0;
+        } else {
+            b0 += c;
+            n0 -= c;
+        }
+    }
+    if (lane == 0 && kept) atomicAdd(&a.ctl->live, kept);
 }
 
 // Exclusive scan of the material histogram (one block) and the scatter of
@@ -704,19 +849,20 @@ __global__ void k_wf_scatter(WfArgs a) {
 // Shadow sink of the wavefront: queue the ray with its contribution.
 struct QueueShadows : NoAdjoint {
     const WfArgs* a;
-    int slot;
-    int scene;
+    int t, slot, scene;   // shade's thread, its slot and scene
+    int n;                // records written
     template <class PS>
     RT_D void shadow(PS& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
         if (!isfinite(c.x) || !isfinite(c.y) || !isfinite(c.z)) {
             ps.add(c, to_la);   // records the per-frame sanitize in the mask
             return;
         }
-        int j = wagg_next_int(a->S.count);
-        if (j >= a->S.capacity) {
+        if (n >= a->S.per || (a->S.limit > 0 && atomicAdd(a->S.count, 1) >= a->S.limit)) {
             atomicExch(&a->ctl->overflow, 1);
             return;
         }
+        int j = n * a->nslots + t;
+        n++;
         a->S.o[j] = make_float4(o.x, o.y, o.z, tmax);
         a->S.d[j] = make_float4(d.x, d.y, d.z, ibits((slot << 1) | to_la));
         a->S.c[j] = make_float4(c.x, c.y, c.z, ibits(scene));
@@ -778,8 +924,10 @@ __global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(const __g
     }
     float4 d = a.P.d[i];
     int flags = fbits(d.w);
-    if (!(flags & PF_ALIVE)) return;
-    float4 o = a.P.o[i], b = a.P.beta[i], w = a.P.w[i];
+    if (!(flags & PF_ALIVE)) {
+        a.S.cnt[t] = 0;
+        return;
+    }
     int4 id = a.P.id[i];
     Hit h = wf_hit(a, i);
     int req = ONE ? 0 : RT_IX(id.z, a.nreq);
@@ -789,29 +937,38 @@ __global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(const __g
     LeanPath<TRANSMIT> ps;
     ps.a = &a;
     ps.slot = i;
-    ps.o = v3(o.x, o.y, o.z);
-    ps.prev_pdf = o.w;
     ps.d = v3(d.x, d.y, d.z);
-    ps.beta = v3(b.x, b.y, b.z);
-    ps.depth = fbits(b.w);
-    ps.w = v3(w.x, w.y, w.z);
-    ps.rng = Sampler{(uint32_t)id.w, (uint32_t)id.x, (uint32_t)fbits(w.w)};
     ps.prev_delta = (flags & PF_PREV_DELTA) != 0;
     ps.first = (flags & PF_FIRST) != 0;
     ps.clamp_mode = (flags & PF_CLAMP) != 0;
     ps.dead = flags & (7 * PF_DEAD);
+    // a camera path as path_init leaves it (it stored no more), else the slot's state
+    float4 o = make_float4(rc.cam.origin.x, rc.cam.origin.y, rc.cam.origin.z, 0.0f);
+    float4 b = make_float4(1.0f, 1.0f, 1.0f, ibits(rc.max_depth)), w = make_float4(1.0f, 1.0f, 1.0f, ibits(2));
+    if (!ps.first) {
+        o = a.P.o[i];
+        b = a.P.beta[i];
+        w = a.P.w[i];
+    }
+    ps.o = v3(o.x, o.y, o.z);
+    ps.prev_pdf = o.w;
+    ps.beta = v3(b.x, b.y, b.z);
+    ps.depth = fbits(b.w);
+    ps.w = v3(w.x, w.y, w.z);
+    ps.rng = Sampler{(uint32_t)id.w, (uint32_t)id.x, (uint32_t)fbits(w.w)};
     if constexpr (TRANSMIT) {
         ps.cur_abs = v3(0.0f);
         ps.iors.n = 0;
-        if (rc.dielectrics) {
+        if (rc.dielectrics && !ps.first) {
             float4 ab = a.P.ab[i];
             ps.cur_abs = v3(ab.x, ab.y, ab.z);
             ps.iors.n = fbits(ab.w);
             for (int k = 0; k < 8; k++) ps.iors.slot[k] = a.P.ior[(size_t)i * 8 + k];
         }
     }
-    QueueShadows sink{{}, &a, i, scene};
+    QueueShadows sink{{}, &a, t, i, scene, 0};
     bool alive = shade_vertex<MEDIUM, TRANSMIT>(s, rc, ps, h, sink);
+    a.S.cnt[t] = sink.n;
     a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(wf_flags(ps, alive) | ps.dead));
     if (!alive) return;   // resolve reads the flags and the radiance sums alone
     a.P.o[i] = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.prev_pdf);
@@ -872,13 +1029,20 @@ __global__ void __launch_bounds__(1024) k_wf_rscan(int* hist, int* off, int* tot
     if (t == 1023) *total = base;
 }
 
+// The record that thread t of shade wrote k-th, or -1. Under the material sort
+// shade ran the threads below the live count alone.
+RT_D int shadow_record(const WfArgs& a, int t, int k) {
+    int live = a.sort ? a.ctl->hist[a.nkeys] : a.nslots;
+    if (t >= live || k >= a.S.cnt[RT_IX(t, a.nslots)]) return -1;
+    return k * a.nslots + t;
+}
+
 // Shadow sort: each queued record goes to its key's offset plus its rank.
-__global__ void k_wf_sscatter(WfArgs a) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = min(*a.S.count, a.S.capacity);
-    if (j >= n) return;
+__global__ void k_wf_sscatter(const __grid_constant__ WfArgs a) {
+    int j = shadow_record(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+    if (j < 0) return;
     int pos = a.soff[RT_IX(a.S.key[j], kRayKeys)] + a.S.rank[j];
-    if (pos < n) a.S.order[pos] = j;
+    if (pos < a.ctl->nshadow) a.S.order[pos] = j;
     else atomicExch(a.err, RT_ERR_BOUNDS);
 }
 
@@ -888,7 +1052,7 @@ template <int STACK>
 __global__ void __launch_bounds__(256) k_wf_occlude_pt(const __grid_constant__ WfArgs a) {
     const unsigned full = 0xffffffffu;
     int lane = threadIdx.x & 31;
-    int n = min(*a.S.count, a.S.capacity);
+    unsigned n = (unsigned)a.nslots * (unsigned)a.S.per;
     Walker<true, STACK> w;
     int rec = -1;
     bool exhausted = false;
@@ -904,11 +1068,10 @@ __global__ void __launch_bounds__(256) k_wf_occlude_pt(const __grid_constant__ W
             base = __shfl_sync(full, base, leader);
             if (idle) {
                 unsigned j = base + (unsigned)__popc(need & ((1u << lane) - 1u));
-                if (j >= (unsigned)n) {
+                if (j >= n) {
                     exhausted = true;
-                } else {
-                    float4 o = a.S.o[j], d = a.S.d[j], c = a.S.c[j];
-                    rec = (int)j;
+                } else if ((rec = shadow_record(a, (int)(j % (unsigned)a.nslots), (int)(j / (unsigned)a.nslots))) >= 0) {
+                    float4 o = a.S.o[rec], d = a.S.d[rec], c = a.S.c[rec];
                     w.start(a.views[RT_IX(fbits(c.w), a.nviews)], v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps, o.w, nullptr, false, 0);
                 }
             }
@@ -939,25 +1102,27 @@ __global__ void __launch_bounds__(256) k_wf_occlude_pt(const __grid_constant__ W
 // its longer walk needs.
 template <int STACK, bool L4, bool OPAQUE>
 __global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid_constant__ WfArgs a) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = min(*a.S.count, a.S.capacity);
-    if (a.shadowsort) {
-        if (j >= n) return;
-        j = RT_IX(a.S.order[j], n);
-    } else if (a.regroup) {
-        // shadow rays by direction octant (blocks wholly past the queue leave at once)
-        if ((int)(blockIdx.x * blockDim.x) >= n) return;
-        __shared__ int s_idx[256], s_cnt[8][8], s_tot;
-        int cls = -1;
-        if (j < n) {
-            float4 d = a.S.d[j];
-            cls = octant(d.x, d.y, d.z);
+    int j;
+    if (a.shadowsort) {   // a flat grid over the sorted order
+        long long p = (long long)blockIdx.y * gridDim.x * blockDim.x + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        int n = a.ctl->nshadow;
+        if (p >= n) return;
+        j = RT_IX(a.S.order[p], a.nslots * a.S.per);
+    } else {
+        j = shadow_record(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+        if (a.regroup) {   // shadow rays by direction octant
+            __shared__ int s_idx[256], s_cnt[8][8], s_tot;
+            int cls = -1;
+            if (j >= 0) {
+                float4 d = a.S.d[j];
+                cls = octant(d.x, d.y, d.z);
+            }
+            int m = block_group<8>(j, cls, s_idx, s_cnt, &s_tot);
+            if ((int)threadIdx.x >= m) return;
+            j = s_idx[threadIdx.x];
+        } else if (j < 0) {
+            return;
         }
-        int m = block_group<8>(j, cls, s_idx, s_cnt, &s_tot);
-        if ((int)threadIdx.x >= m) return;
-        j = s_idx[threadIdx.x];
-    } else if (j >= n) {
-        return;
     }
     float4 o = a.S.o[j], d = a.S.d[j], c = a.S.c[j];
     const SceneView& s = a.views[RT_IX(fbits(c.w), a.nviews)];
@@ -982,6 +1147,8 @@ __global__ void k_wf_reset(WfArgs a) {
         a.ctl->live = 0;
         a.ctl->ext_next = 0;
         a.ctl->occ_next = 0;
+        a.ctl->nfree = 0;
+        a.ctl->free_next = 0;
         a.ctl->iter_first = a.ctl->next;
     }
     if (a.sort)
