@@ -697,31 +697,32 @@ struct HostReq {
     float* d_film;
 };
 
+// An instantiated graph: the loop of wavefront iterations (a conditional node
+// that repeats its body until k_wf_plan ends it). key: the kernel arguments and
+// launch shapes it was captured with.
+struct WfGraph {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned char> key;
+};
+constexpr size_t kMaxGraphs = 8;
+
 struct WfWorkspace {
     void* mem = nullptr;
     size_t bytes = 0;
-    unsigned long long* pinned = nullptr;   // two read-back slots of {next, live | overflow}
-    cudaEvent_t polled[2] = {nullptr, nullptr};   // each slot's read-back has landed
-    // The last instantiated iteration graph and the kernel arguments and launch
-    // shapes it was captured with: a repeated render of the same configuration
-    // replays it instead of capturing and instantiating a new one.
-    cudaGraphExec_t exec = nullptr;
-    std::vector<unsigned char> exec_key;
+    // pinned staging of the call's tables (scene views, requests, control block)
+    // and of the control block on its way back
+    char* pinned = nullptr;
+    size_t pinned_bytes = 0;
+    // The last graphs, most recent first, bounded: a call of a shape among them
+    // replays its graph instead of capturing and instantiating one.
+    std::vector<WfGraph> graphs;
+    void drop_graphs() {
+        for (WfGraph& g : graphs) cudaGraphExecDestroy(g.exec);
+        graphs.clear();
+    }
 };
 std::mutex g_wf_mu;
 WfWorkspace g_wf_ws[16];
-
-struct Carve {
-    char* base;
-    size_t off = 0;
-    template <typename T>
-    T* take(size_t n) {
-        off = (off + 255) & ~(size_t)255;
-        T* p = reinterpret_cast<T*>(base + off);
-        off += n * sizeof(T);
-        return p;
-    }
-};
 
 // Autotuned (wavefront size, block size, sort) per scene set, kept for the
 // process lifetime; filled by rt_autotune or the defaults below.
@@ -754,6 +755,39 @@ int default_groups(const std::vector<RtScene*>& scenes) {
     for (const RtScene* sc : scenes)
         if (sc->host.has_medium) return 1;
     return 4;
+}
+
+// Captures `body` (the launches of one iteration on `stream`) as the body of a
+// loop that repeats until a kernel clears the loop condition, and instantiates
+// it: the device runs the iterations without the host.
+template <class F>
+int wf_capture(cudaStream_t stream, F body, cudaGraphExec_t& exec) {
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaGraphCreate(&graph, 0);
+    if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("graph creation: ") + cudaGetErrorString(e));
+    cudaGraphConditionalHandle loop{};
+    cudaGraphNodeParams np{};
+    cudaGraphNode_t node;
+    e = cudaGraphConditionalHandleCreate(&loop, graph, 1, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) {
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = loop;
+        np.conditional.type = cudaGraphCondTypeWhile;
+        np.conditional.size = 1;
+        e = cudaGraphAddNode(&node, graph, nullptr, 0, &np);
+    }
+    if (e == cudaSuccess) {
+        cudaGraph_t inner = np.conditional.phGraph_out[0];
+        e = cudaStreamBeginCaptureToGraph(stream, inner, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            body(loop);
+            e = cudaStreamEndCapture(stream, &inner);
+        }
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);   // the executable graph does not need it
+    if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    return RT_OK;
 }
 
 // mode: rt::WF_RENDER renders the requests into their films; rt::WF_RECORD
@@ -821,95 +855,103 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     nslots = (nslots + 255) / 256 * 256;
     int64_t cap = (int64_t)nslots * max_shadow;
     if (cap >= ((int64_t)1 << 31) || nslots >= (1 << 29)) return fail(RT_ERR_INVALID_ARG, "wavefront too large");
-    // Workspace layout.
-    size_t need = 0;
-    auto add = [&](size_t b) { need = ((need + 255) & ~(size_t)255) + b; };
-    add(views.size() * sizeof(rt::SceneView));
-    add(wreq.size() * sizeof(rt::WfRequest));
-    add(key_base.size() * sizeof(int));
-    add(sizeof(rt::WfCtl));
-    for (int k = 0; k < 10; k++) add((size_t)nslots * sizeof(float4));
-    for (int k = 0; k < 5; k++) add((size_t)nslots * sizeof(int));
-    if (dielectrics) {
-        add((size_t)nslots * sizeof(float4));
-        add((size_t)nslots * 8 * sizeof(float));
-    }
-    for (int k = 0; k < 3; k++) add((size_t)cap * sizeof(float4));
-    add(sizeof(int));
-    for (int k = 0; k < 3; k++) add((size_t)cap * sizeof(int));
-    for (int k = 0; k < 4; k++) add((size_t)rt::kRayKeys * sizeof(int));
-    for (auto& q : wreq) add((size_t)3 * q.ww * q.wh * sizeof(double));
-    add(reqs.size() * sizeof(float*));
-    add(reqs.size() * sizeof(int) * 2);
-    if (mode == rt::WF_REPLAY) add((size_t)nslots * rt::kAdjState * sizeof(float4));
-    need += 1024;
+    // Workspace layout: the call's tables first (one upload), then what one
+    // memset clears, then the rest.
+    auto align = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    rt::WfArgs a;
+    std::memset(&a, 0, sizeof(a));   // padding too: the bytes key the cached graph
+    rt::SceneView* d_views;
+    rt::WfRequest* d_reqs;
+    int *d_kb, *d_fdims;
+    rt::WfCtl* d_ctl;
+    float** d_films;
+    rt::WfOne* d_one;
+    rt::WfAdjoint* d_adj;
+    rt::WfAdjoint J{};
+    if (adj) J = *adj;
+    size_t off_views, off_reqs, off_kb, off_ctl, off_films, off_fdims, off_one, off_adj, table_bytes, clear_begin, clear_end;
+    auto layout = [&](char* base) {
+        size_t off = 0;
+        auto take = [&](auto*& p, size_t n) {
+            off = align(off);
+            size_t at = off;
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + off);
+            off += n * sizeof(*p);
+            return at;
+        };
+        off_views = take(d_views, views.size());
+        off_reqs = take(d_reqs, wreq.size());
+        off_kb = take(d_kb, key_base.size());
+        off_ctl = take(d_ctl, 1);
+        off_films = take(d_films, reqs.size());
+        off_fdims = take(d_fdims, 2 * reqs.size());
+        off_one = take(d_one, 1);
+        off_adj = take(d_adj, 1);
+        table_bytes = off;
+        clear_begin = align(off);
+        take(a.rhist, rt::kRayKeys);
+        take(a.roff, rt::kRayKeys);
+        take(a.shist, rt::kRayKeys);
+        take(a.soff, rt::kRayKeys);
+        take(a.P.d, nslots);
+        for (auto& q : wreq) take(q.accum, (size_t)3 * q.ww * q.wh);
+        clear_end = off;
+        take(a.P.o, nslots);
+        take(a.P.beta, nslots);
+        take(a.P.w, nslots);
+        take(a.P.id, nslots);
+        take(a.P.lp, nslots);
+        take(a.P.la, nslots);
+        take(a.P.pre, nslots);
+        take(a.P.att0, nslots);
+        take(a.P.hit, nslots);
+        take(a.P.order, nslots);
+        take(a.P.keys, nslots);
+        take(a.P.rrank, nslots);
+        take(a.P.free, nslots);
+        take(a.S.cnt, nslots);
+        if (dielectrics) {
+            take(a.P.ab, nslots);
+            take(a.P.ior, (size_t)nslots * 8);
+        }
+        take(a.S.o, cap);
+        take(a.S.d, cap);
+        take(a.S.c, cap);
+        take(a.S.key, cap);
+        take(a.S.rank, cap);
+        take(a.S.order, cap);
+        if (mode == rt::WF_REPLAY) take(J.st, (size_t)nslots * rt::kAdjState);
+        return off;
+    };
     WfWorkspace& ws = g_wf_ws[dev];
+    size_t need = layout(nullptr) + 1024;
     if (ws.bytes < need) {
-        if (ws.exec) cudaGraphExecDestroy(ws.exec);   // captured with pointers into the old workspace
-        ws.exec = nullptr;
-        ws.exec_key.clear();
+        ws.drop_graphs();   // captured with pointers into the old workspace
         if (ws.mem) cudaFree(ws.mem);
         ws.mem = nullptr;
         ws.bytes = 0;
         if (cudaMalloc(&ws.mem, need) != cudaSuccess) return fail(RT_ERR_OOM, "wavefront workspace allocation failed");
         ws.bytes = need;
     }
-    if (!ws.pinned && cudaMallocHost(&ws.pinned, 4 * sizeof(unsigned long long)) != cudaSuccess)
-        return fail(RT_ERR_OOM, "pinned read-back allocation failed");
-    for (cudaEvent_t& e : ws.polled)
-        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
-            return fail(RT_ERR_CUDA, "event creation failed");
-    Carve cv{static_cast<char*>(ws.mem)};
-    rt::WfArgs a;
-    std::memset(&a, 0, sizeof(a));   // padding too: the bytes key the cached graph
-    auto* d_views = cv.take<rt::SceneView>(views.size());
-    auto* d_reqs = cv.take<rt::WfRequest>(wreq.size());
-    auto* d_kb = cv.take<int>(key_base.size());
-    auto* d_ctl = cv.take<rt::WfCtl>(1);
-    a.P.o = cv.take<float4>(nslots);
-    a.P.d = cv.take<float4>(nslots);
-    a.P.beta = cv.take<float4>(nslots);
-    a.P.w = cv.take<float4>(nslots);
-    a.P.id = cv.take<int4>(nslots);
-    a.P.lp = cv.take<float4>(nslots);
-    a.P.la = cv.take<float4>(nslots);
-    a.P.pre = cv.take<float4>(nslots);
-    a.P.att0 = cv.take<float4>(nslots);
-    a.P.hit = cv.take<float4>(nslots);
-    a.P.order = cv.take<int>(nslots);
-    a.P.keys = cv.take<int>(nslots);
-    a.P.rrank = cv.take<int>(nslots);
-    a.P.free = cv.take<int>(nslots);
-    a.S.cnt = cv.take<int>(nslots);
-    if (dielectrics) {
-        a.P.ab = cv.take<float4>(nslots);
-        a.P.ior = cv.take<float>((size_t)nslots * 8);
+    layout(static_cast<char*>(ws.mem));
+    size_t pin_need = align(table_bytes) + sizeof(rt::WfCtl);
+    if (ws.pinned_bytes < pin_need) {
+        if (ws.pinned) cudaFreeHost(ws.pinned);
+        ws.pinned = nullptr;
+        ws.pinned_bytes = 0;
+        if (cudaMallocHost(&ws.pinned, pin_need) != cudaSuccess)
+            return fail(RT_ERR_OOM, "pinned staging allocation failed");
+        ws.pinned_bytes = pin_need;
     }
-    a.S.o = cv.take<float4>(cap);
-    a.S.d = cv.take<float4>(cap);
-    a.S.c = cv.take<float4>(cap);
-    a.S.count = cv.take<int>(1);
-    a.S.per = max_shadow;
-    a.S.limit = cfg.shadow_limit;
-    a.S.key = cv.take<int>(cap);
-    a.S.rank = cv.take<int>(cap);
-    a.S.order = cv.take<int>(cap);
-    a.rhist = cv.take<int>(rt::kRayKeys);
-    a.roff = cv.take<int>(rt::kRayKeys);
-    a.shist = cv.take<int>(rt::kRayKeys);
-    a.soff = cv.take<int>(rt::kRayKeys);
     std::vector<float*> films(reqs.size());
     std::vector<int> fdims(2 * reqs.size());
     for (size_t r = 0; r < reqs.size(); r++) {
-        wreq[r].accum = cv.take<double>((size_t)3 * wreq[r].ww * wreq[r].wh);
         films[r] = reqs[r].d_film;
         fdims[r] = reqs[r].W;
         fdims[reqs.size() + r] = reqs[r].H;
     }
-    auto* d_films = cv.take<float*>(reqs.size());
-    auto* d_fdims = cv.take<int>(2 * reqs.size());
-    if (adj) a.J = *adj;
-    if (mode == rt::WF_REPLAY) a.J.st = cv.take<float4>((size_t)nslots * rt::kAdjState);
+    a.S.per = max_shadow;
+    a.S.limit = cfg.shadow_limit;
     a.views = d_views;
     a.nviews = (int)views.size();
     a.reqs = d_reqs;
@@ -920,28 +962,33 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     a.nkeys = nkeys;
     a.key_base = d_kb;
     a.ctl = d_ctl;
-    a.err = s0->d_err;
+    a.err = &d_ctl->err;
+    a.J = adj ? d_adj : nullptr;
+    int max_depth = 1;
+    for (auto& q : wreq) max_depth = std::max(max_depth, q.rc.max_depth);
+    // Twice the iterations of batches that each wait for their longest path: an
+    // iteration starts at least half as many paths as there are free slots.
+    int64_t limit = 2 * (total / nslots + 2) * (int64_t)(max_depth + 2) + 64;
+    if (cfg.iter_limit > 0) limit = std::min<int64_t>(limit, cfg.iter_limit);
+    const bool one = reqs.size() == 1;
     rt::WfCtl ctl0{};
     ctl0.total = (unsigned long long)total;
-    CUDA_TRY(cudaMemcpyAsync(d_views, views.data(), views.size() * sizeof(rt::SceneView), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(d_reqs, wreq.data(), wreq.size() * sizeof(rt::WfRequest), cudaMemcpyHostToDevice, stream));
-    const bool one = reqs.size() == 1;
+    ctl0.limit = (int)std::min<int64_t>(limit, INT32_MAX);
+    std::memcpy(ws.pinned + off_views, views.data(), views.size() * sizeof(rt::SceneView));
+    std::memcpy(ws.pinned + off_reqs, wreq.data(), wreq.size() * sizeof(rt::WfRequest));
+    std::memcpy(ws.pinned + off_kb, key_base.data(), key_base.size() * sizeof(int));
+    std::memcpy(ws.pinned + off_ctl, &ctl0, sizeof(ctl0));
+    std::memcpy(ws.pinned + off_adj, &J, sizeof(J));
+    std::memcpy(ws.pinned + off_films, films.data(), films.size() * sizeof(float*));
+    std::memcpy(ws.pinned + off_fdims, fdims.data(), fdims.size() * sizeof(int));
+    CUDA_TRY(cudaMemcpyAsync(ws.mem, ws.pinned, table_bytes, cudaMemcpyHostToDevice, stream));
     if (one) {
         rt::WfOne c{views[0], wreq[0].rc};
-        CUDA_TRY(cudaMemcpyToSymbolAsync(rt::c_wf_one, &c, sizeof(c), 0, cudaMemcpyHostToDevice, stream));
+        std::memcpy(ws.pinned + off_one, &c, sizeof(c));
+        CUDA_TRY(cudaMemcpyToSymbolAsync(rt::c_wf_one, ws.pinned + off_one, sizeof(c), 0, cudaMemcpyHostToDevice, stream));
     }
-    CUDA_TRY(cudaMemcpyAsync(d_kb, key_base.data(), key_base.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(d_ctl, &ctl0, sizeof(ctl0), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(d_films, films.data(), films.size() * sizeof(float*), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(d_fdims, fdims.data(), fdims.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemsetAsync(a.P.d, 0, (size_t)nslots * sizeof(float4), stream));
-    CUDA_TRY(cudaMemsetAsync(a.S.count, 0, sizeof(int), stream));
-    for (int* h : {a.rhist, a.roff, a.shist, a.soff})
-        CUDA_TRY(cudaMemsetAsync(h, 0, (size_t)rt::kRayKeys * sizeof(int), stream));
-    for (auto& q : wreq) CUDA_TRY(cudaMemsetAsync(q.accum, 0, (size_t)3 * q.ww * q.wh * sizeof(double), stream));
-    CUDA_TRY(cudaMemsetAsync(s0->d_err, 0, sizeof(int), stream));
-    CUDA_TRY(cudaStreamSynchronize(stream));   // host vectors above go out of scope
-    // One iteration: reset, regen, extend, [scan, scatter], shade, occlude.
+    CUDA_TRY(cudaMemsetAsync(static_cast<char*>(ws.mem) + clear_begin, 0, clear_end - clear_begin, stream));
+    // One iteration: regen, camera, extend, [scatter], shade, plan, [sscatter], occlude.
     int blk = cfg.block;
     int tblk = cfg.tblock > 0 ? cfg.tblock : blk;
     bool l4 = cfg.layout == 4;
@@ -992,7 +1039,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     unsigned gadj = (unsigned)((nslots + adj_blk - 1) / adj_blk);
     size_t adj_shmem = 0;
     if (mode == rt::WF_REPLAY)
-        adj_shmem = (size_t)(a.J.use_local ? a.J.nact : (a.J.use_shared ? a.J.nparams : 0)) * sizeof(float);
+        adj_shmem = (size_t)(J.use_local ? J.nact : (J.use_shared ? J.nparams : 0)) * sizeof(float);
     unsigned gs = (unsigned)((nslots + blk - 1) / blk);
     unsigned gst = (unsigned)((nslots + tblk - 1) / tblk);
     dim3 gsh(gst, (unsigned)max_shadow);   // occlude and the shadow scatter: (shade's threads, records of each)
@@ -1011,10 +1058,11 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
                       : (transmit ? rt::k_wf_shade<false, true, true> : rt::k_wf_shade<false, false, true>))
             : (medium ? (transmit ? rt::k_wf_shade<true, true, false> : rt::k_wf_shade<true, false, false>)
                       : (transmit ? rt::k_wf_shade<false, true, false> : rt::k_wf_shade<false, false, false>));
+    // the plan's blocks: the bookkeeping, the bounce rays' scan, the shadow records' scan
+    const unsigned gplan = a.shadowsort ? 3 : (a.raysort ? 2 : 1);
     // ev (profiling only): boundaries between the kernel groups of one iteration.
-    auto launch_iter = [&](cudaEvent_t* ev) {
+    auto launch_iter = [&](cudaEvent_t* ev, cudaGraphConditionalHandle loop) {
         if (ev) cudaEventRecord(ev[0], stream);
-        rt::k_wf_reset<<<1, 256, 0, stream>>>(a);
         if (mode == rt::WF_RECORD) rt::k_wf_regen<rt::WF_RECORD><<<g256, 256, 0, stream>>>(a);
         else if (mode == rt::WF_REPLAY) rt::k_wf_regen<rt::WF_REPLAY><<<g256, 256, 0, stream>>>(a);
         else rt::k_wf_regen<rt::WF_RENDER><<<g256, 256, 0, stream>>>(a);
@@ -1024,162 +1072,114 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         else if (pt) rt::k_wf_extend_pt<kStack><<<gpt_e, tblk, 0, stream>>>(a);
         else rt::k_wf_extend<kStack, false><<<gst, tblk, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[2], stream);
-        if (sort) {
-            rt::k_wf_scan<<<1, 256, 0, stream>>>(a);
-            rt::k_wf_scatter<<<g256, 256, 0, stream>>>(a);
-        }
+        if (sort) rt::k_wf_scatter<<<g256, 256, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[3], stream);
         if (mode == rt::WF_REPLAY) {   // the adjoint vertex, shadow rays inline: no occlude
             if (medium && transmit) rt::k_wf_adjoint<kStack, true, true><<<gadj, adj_blk, adj_shmem, stream>>>(a);
             else if (medium) rt::k_wf_adjoint<kStack, true, false><<<gadj, adj_blk, adj_shmem, stream>>>(a);
             else if (transmit) rt::k_wf_adjoint<kStack, false, true><<<gadj, adj_blk, adj_shmem, stream>>>(a);
             else rt::k_wf_adjoint<kStack, false, false><<<gadj, adj_blk, adj_shmem, stream>>>(a);
-            if (ev) cudaEventRecord(ev[4], stream);
-            if (a.raysort) rt::k_wf_rscan<<<1, 1024, 0, stream>>>(a.rhist, a.roff, &d_ctl->nbounce);
-            if (ev) {
-                cudaEventRecord(ev[5], stream);
-                cudaEventRecord(ev[6], stream);
-            }
-            return;
+        } else {
+            shade<<<gs, blk, 0, stream>>>(a);
         }
-        shade<<<gs, blk, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[4], stream);   // the ray sorts' scans and scatter count as sorting
-        if (a.raysort) rt::k_wf_rscan<<<1, 1024, 0, stream>>>(a.rhist, a.roff, &d_ctl->nbounce);
-        if (a.shadowsort) {
-            rt::k_wf_rscan<<<1, 1024, 0, stream>>>(a.shist, a.soff, &d_ctl->nshadow);
-            rt::k_wf_sscatter<<<gsh256, 256, 0, stream>>>(a);
-        }
+        rt::k_wf_plan<<<gplan, 1024, 0, stream>>>(a, loop);
+        if (a.shadowsort) rt::k_wf_sscatter<<<gsh256, 256, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[5], stream);
-        if (l4_occ && a.opaque) rt::k_wf_occlude<kStack, true, true><<<gsh, tblk, 0, stream>>>(a);
-        else if (l4) rt::k_wf_occlude<kStack, true, false><<<gsh, tblk, 0, stream>>>(a);
-        else if (pt && a.opaque) rt::k_wf_occlude_pt<kStack><<<gpt_o, tblk, 0, stream>>>(a);
-        else if (a.opaque) rt::k_wf_occlude<kStack, false, true><<<gsh, tblk, 0, stream>>>(a);
-        else rt::k_wf_occlude<kStack, false, false><<<gsh, tblk, 0, stream>>>(a);
+        if (mode != rt::WF_REPLAY) {
+            if (l4_occ && a.opaque) rt::k_wf_occlude<kStack, true, true><<<gsh, tblk, 0, stream>>>(a);
+            else if (l4) rt::k_wf_occlude<kStack, true, false><<<gsh, tblk, 0, stream>>>(a);
+            else if (pt && a.opaque) rt::k_wf_occlude_pt<kStack><<<gpt_o, tblk, 0, stream>>>(a);
+            else if (a.opaque) rt::k_wf_occlude<kStack, false, true><<<gsh, tblk, 0, stream>>>(a);
+            else rt::k_wf_occlude<kStack, false, false><<<gsh, tblk, 0, stream>>>(a);
+        }
         if (ev) cudaEventRecord(ev[6], stream);
     };
-    constexpr int kEv = 7;   // profiling events per iteration
-    const int batch = 4;
+    int per_iter = (mode == rt::WF_REPLAY ? 4 : 6) + (sort ? 1 : 0) + (a.shadowsort ? 1 : 0);
+    double t_regen = 0, t_extend = 0, t_sort = 0, t_shade = 0, t_occlude = 0;
+    int rc = RT_OK;
+    rt::WfCtl* back = reinterpret_cast<rt::WfCtl*>(ws.pinned + align(table_bytes));
     cudaGraphExec_t exec = nullptr;
-    std::vector<cudaEvent_t> pev;
-    if (cfg.profile) {
-        pev.resize(batch * kEv);
-        for (auto& e : pev)
-            if (cudaEventCreate(&e) != cudaSuccess) return fail(RT_ERR_CUDA, "event creation failed");
-    } else {
+    if (!cfg.profile) {
         // The graph is a function of the kernels' arguments and launch shapes
         // alone (everything else it reads lives in the workspace), so those
-        // bytes key the cached one.
+        // bytes key the cached ones.
         const unsigned shape[] = {(unsigned)blk, (unsigned)tblk, (unsigned)l4, (unsigned)l4_occ, (unsigned)pt,
-                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst, (unsigned)max_shadow, g256, gcam,
-                                  (unsigned)mode, gadj, (unsigned)adj_shmem};
+                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst,
+                                  (unsigned)max_shadow, g256, gcam, gplan, (unsigned)mode, gadj, (unsigned)adj_shmem};
         std::vector<unsigned char> key(sizeof(a) + sizeof(shape));
         std::memcpy(key.data(), &a, sizeof(a));
         std::memcpy(key.data() + sizeof(a), shape, sizeof(shape));
-        if (ws.exec && ws.exec_key == key) {
-            exec = ws.exec;
+        size_t at = 0;
+        while (at < ws.graphs.size() && ws.graphs[at].key != key) at++;
+        if (at < ws.graphs.size()) {
+            std::rotate(ws.graphs.begin(), ws.graphs.begin() + at, ws.graphs.begin() + at + 1);
         } else {
-            if (ws.exec) cudaGraphExecDestroy(ws.exec);
-            ws.exec = nullptr;
-            ws.exec_key.clear();
-            cudaGraph_t graph = nullptr;
-            CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            launch_iter(nullptr);
-            cudaError_t ce = cudaStreamEndCapture(stream, &graph);
-            if (ce != cudaSuccess) return fail(RT_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-            ce = cudaGraphInstantiate(&exec, graph, 0);
-            cudaGraphDestroy(graph);   // the executable graph does not need it
-            if (ce != cudaSuccess) return fail(RT_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-            ws.exec = exec;
-            ws.exec_key = std::move(key);
+            WfGraph g;
+            g.key = std::move(key);
+            rc = wf_capture(stream, [&](cudaGraphConditionalHandle h) { launch_iter(nullptr, h); }, g.exec);
+            if (rc != RT_OK) return rc;
+            if (ws.graphs.size() >= kMaxGraphs) {
+                cudaGraphExecDestroy(ws.graphs.back().exec);
+                ws.graphs.pop_back();
+            }
+            ws.graphs.insert(ws.graphs.begin(), std::move(g));
         }
+        exec = ws.graphs.front().exec;
     }
-    int per_iter = (mode == rt::WF_REPLAY ? 4 : 6) + (sort ? 2 : 0) + (a.raysort ? 1 : 0) + (a.shadowsort ? 2 : 0);
-    int max_depth = 1;
-    for (auto& q : wreq) max_depth = std::max(max_depth, q.rc.max_depth);
-    int64_t limit = (total / nslots + 2) * (int64_t)(max_depth + 2) + 64;
-    if (cfg.iter_limit > 0) limit = std::min<int64_t>(limit, cfg.iter_limit);
-    int64_t iters = 0;
-    double t_regen = 0, t_extend = 0, t_sort = 0, t_shade = 0, t_occlude = 0;
-    int rc = RT_OK;
-    // The poll is pipelined: batch k+1 is queued before the host waits for
-    // batch k's read-back, so the device does not idle while the host turns
-    // around. Replays after the wavefront has drained find no work and write
-    // nothing (the polled batches already ran up to batch-1 of them).
-    // Profiling waits for each batch itself, so its events are read before the
-    // next batch records them again.
-    int cur = 0, waiting = -1;
     CUDA_TRY(cudaEventRecord(s0->ev0, stream));
-    for (;;) {
-        for (int k = 0; k < batch; k++) {
-            if (cfg.profile) {
-                launch_iter(&pev[k * kEv]);
-            } else if (cudaGraphLaunch(exec, stream) != cudaSuccess) {
-                rc = fail(RT_ERR_CUDA, "graph launch failed");
+    if (exec) {
+        // the whole loop is one launch: k_wf_plan ends it on the device, at the
+        // latest at ctl->limit
+        if (cudaGraphLaunch(exec, stream) != cudaSuccess) rc = fail(RT_ERR_CUDA, "graph launch failed");
+    } else {
+        // profiling: the host runs the iterations, with events between the kernels
+        constexpr int kEv = 7;
+        cudaEvent_t pev[kEv] = {};
+        for (auto& e : pev)
+            if (rc == RT_OK && cudaEventCreate(&e) != cudaSuccess) rc = fail(RT_ERR_CUDA, "event creation failed");
+        while (rc == RT_OK) {
+            launch_iter(pev, cudaGraphConditionalHandle{});
+            cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
+            if (cudaStreamSynchronize(stream) != cudaSuccess) {
+                rc = fail(RT_ERR_CUDA, std::string("wavefront iteration failed: ") + cudaGetErrorString(cudaGetLastError()));
                 break;
             }
+            float m[kEv - 1];
+            for (int e = 0; e < kEv - 1; e++) cudaEventElapsedTime(&m[e], pev[e], pev[e + 1]);
+            t_regen += m[0];
+            t_extend += m[1];
+            t_sort += m[2] + m[4];   // the material sort, then the ray sorts' scans and scatter
+            t_shade += m[3];
+            t_occlude += m[5];
+            if (back->done || back->overflow || back->iters >= back->limit) break;
         }
-        if (rc != RT_OK) break;
-        iters += batch;
-        unsigned long long* slot = ws.pinned + 2 * cur;
-        cudaMemcpyAsync(slot, &d_ctl->next, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream);
-        cudaMemcpyAsync(slot + 1, &d_ctl->live, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream);
-        cudaEventRecord(ws.polled[cur], stream);
-        int check = cur;
-        if (!cfg.profile) {
-            check = waiting;
-            waiting = cur;
-            cur ^= 1;
-            if (check < 0) continue;   // first batch: queue the second before waiting
-        }
-        if (cudaEventSynchronize(ws.polled[check]) != cudaSuccess) {
-            rc = fail(RT_ERR_CUDA, std::string("wavefront iteration failed: ") + cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
-        if (cfg.profile) {
-            for (int k = 0; k < batch; k++) {
-                float m[kEv - 1];
-                for (int e = 0; e < kEv - 1; e++)
-                    cudaEventElapsedTime(&m[e], pev[k * kEv + e], pev[k * kEv + e + 1]);
-                t_regen += m[0];
-                t_extend += m[1];
-                t_sort += m[2] + m[4];   // the material sort, then the ray sorts' scans and scatter
-                t_shade += m[3];
-                t_occlude += m[5];
-            }
-        }
-        unsigned long long next = ws.pinned[2 * check];
-        int live = reinterpret_cast<int*>(ws.pinned + 2 * check + 1)[0];
-        int overflow = reinterpret_cast<int*>(ws.pinned + 2 * check + 1)[1];
-        if (overflow) {
-            rc = fail(RT_ERR_BOUNDS, "shadow queue overflow");
-            break;
-        }
-        if (next >= (unsigned long long)total && live == 0) break;
-        if (iters > limit) {
-            rc = fail(RT_ERR_TIMEOUT, "wavefront did not drain within its iteration bound");
-            break;
-        }
+        for (auto e : pev)
+            if (e) cudaEventDestroy(e);
     }
     if (rc == RT_OK) {
         dim3 g(std::max<unsigned>(1, std::min<unsigned>(4096, (unsigned)((wreq[0].ww * (int64_t)wreq[0].wh + 255) / 256))),
                (unsigned)wreq.size());
         if (mode == rt::WF_RENDER)
             rt::k_wf_finalize<<<g, 256, 0, stream>>>(d_reqs, (int)wreq.size(), d_films, d_fdims, d_fdims + reqs.size());
-        CUDA_TRY(cudaEventRecord(s0->ev1, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        rc = check_err(s0);
+        cudaError_t e = cudaEventRecord(s0->ev1, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) rc = fail(RT_ERR_CUDA, std::string("wavefront failed: ") + cudaGetErrorString(e));
     }
-    // On an error exit up to two batches of replays may still be queued; they
-    // write the shared workspace and the films, so let them finish before the
-    // graph goes away and the next call reuses the workspace.
-    if (rc != RT_OK) cudaStreamSynchronize(stream);
-    if (rc == RT_ERR_CUDA && ws.exec) {   // a failed launch: do not replay that graph again
-        cudaGraphExecDestroy(ws.exec);
-        ws.exec = nullptr;
-        ws.exec_key.clear();
+    if (rc == RT_OK) {
+        if (back->overflow) rc = fail(RT_ERR_BOUNDS, "shadow queue overflow");
+        else if (back->err == RT_ERR_STACK) rc = fail(RT_ERR_STACK, "traversal stack bound exceeded");
+        else if (back->err != 0) rc = fail(RT_ERR_BOUNDS, "device error " + std::to_string(back->err));
+        else if (!back->done) rc = fail(RT_ERR_TIMEOUT, "wavefront did not drain within its iteration bound");
+        else rc = checked_flag(stream);
     }
-    for (auto e : pev) cudaEventDestroy(e);
+    if (rc == RT_ERR_CUDA) {   // a failed launch: finish what is queued, and replay no graph again
+        cudaStreamSynchronize(stream);
+        ws.drop_graphs();
+    }
     if (rc != RT_OK) return rc;
+    const int64_t iters = back->iters;
     if (st) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, s0->ev0, s0->ev1);

@@ -91,8 +91,7 @@ struct WfShadow {
     float4* c;    // contribution.xyz, scene
     int* cnt;     // per shade thread: its records
     int per;      // records a vertex can write (the most of any scene)
-    int limit;    // test only, > 0: at most this many records per iteration, counted in *count
-    int* count;
+    int limit;    // test only, > 0: at most this many records per iteration, counted in ctl->nrec
     int* key;     // shadow sort: the record's ray_key
     int* rank;    // shadow sort: its rank among the records of its key
     int* order;   // shadow sort: records in key order, for occlude
@@ -101,16 +100,21 @@ struct WfShadow {
 struct WfCtl {
     unsigned long long next;    // next global work id
     unsigned long long total;   // total work ids
-    int live;                   // slots alive or done after the last regen
-    int overflow;               // shadow queue overflow (never expected: sized by the host)
-    // (the host reads next, then live and overflow as one 8-byte copy: keep them adjacent)
+    unsigned long long iter_first;   // replay: the first work id of this iteration
+    int live;                   // slots alive after the last regen and camera
+    int nlive;                  // live slots in order[] (the material sort's total)
+    int err;                    // a kernel's RT_ERR_* (traversal stack, index checks)
+    int overflow;               // shadow queue overflow (its arrays hold every record: a test's limit)
+    int iters, limit;           // iterations run, and the host's bound on them
+    int done;                   // every work id resolved
     unsigned ext_next;          // persistent extend: next slot to fetch
     unsigned occ_next;          // persistent occlude: next shadow record to fetch
-    unsigned long long iter_first;   // ray sort: the first work id of this iteration
     int nbounce;                // ray sort: bounce rays shade continued (order[0 .. nbounce))
     int nshadow;                // shadow sort: records counted by key
     int nfree, free_next;       // slots in the free list, and the first one not yet reserved
+    int nrec;                   // records written this iteration (counted under a test's limit alone)
     int hist[256];              // material histogram (sorting)
+    int cursor[256];            // live slots placed so far, per material
 };
 
 // Buckets of the bounce-ray sort.
@@ -122,7 +126,7 @@ enum : int { WF_RENDER = 0, WF_RECORD = 1, WF_REPLAY = 2 };
 // throughput's log derivatives (dlb) while a medium slot is differentiated
 constexpr int kAdjState = 10;
 
-// The adjoint passes' buffers and parameters (zero in WF_RENDER).
+// The adjoint passes' buffers and parameters.
 struct WfAdjoint {
     float4* rec;            // per work id, 4 float4: {lp, clamp flag}, la, pre, att0 of the finished sample
     long long nrec;         // work ids the record holds
@@ -169,7 +173,7 @@ struct WfArgs {
     WfCtl* ctl;
     int* err;
     int any4;         // opaque shadow rays may walk the four-wide records (their stack bound fits)
-    WfAdjoint J;
+    const WfAdjoint* J;   // the adjoint passes' buffers and parameters (null in WF_RENDER)
 };
 
 // The scene and constants of a batch of one request, in constant memory: the
@@ -382,8 +386,8 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
         if (MODE == WF_RECORD) {   // keep its end state
             long long rid = R.begin + (long long)(id.x - R.spp0) * ((long long)R.ww * R.wh) +
                             strip_index(lx, ly, R.ww, R.wh);
-            if (rid >= 0 && rid < a.J.nrec) {
-                float4* r = a.J.rec + 4 * rid;
+            if (rid >= 0 && rid < a.J->nrec) {
+                float4* r = a.J->rec + 4 * rid;
                 r[0] = make_float4(lp.x, lp.y, lp.z, ibits(flags & PF_CLAMP));
                 r[1] = la;
                 r[2] = pre;
@@ -446,7 +450,7 @@ __global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs
             path_init(ps, R.rc, R.x0 + lx, R.y0 + ly, (uint32_t)(R.spp0 + s));
             int al = path_alive(ps);
             // the adjoints of the recorded resolve; no gradient, no replay
-            const WfAdjoint& J = a.J;
+            const WfAdjoint& J = *a.J;
             size_t plane = (size_t)J.W * J.H, fi = (size_t)(R.y0 + ly) * J.W + (R.x0 + lx);
             V3 delta = v3(J.dimg[fi], J.dimg[plane + fi], J.dimg[2 * plane + fi]) * J.inv_spp;
             AdjResolve ar{};
@@ -775,8 +779,8 @@ __global__ void __launch_bounds__(128, RT_CAMERA_MIN_BLOCKS) k_wf_camera(const _
                 if (!keep && s.sky_on) L = L + weight_sky(s, rc, 0.0f, 1);   // shade_vertex's sky term, w = 1
             }
             if (!keep && MODE == WF_RECORD) {
-                if ((long long)id < a.J.nrec) {
-                    float4* r = a.J.rec + 4 * id;
+                if ((long long)id < a.J->nrec) {
+                    float4* r = a.J->rec + 4 * id;
                     r[0] = make_float4(L.x, L.y, L.z, ibits(0));
                     r[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     r[2] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
@@ -813,25 +817,40 @@ __global__ void __launch_bounds__(128, RT_CAMERA_MIN_BLOCKS) k_wf_camera(const _
     if (lane == 0 && kept) atomicAdd(&a.ctl->live, kept);
 }
 
-// Exclusive scan of the material histogram (one block) and the scatter of
-// live slots into material order.
-__global__ void k_wf_scan(WfArgs a) {
-    __shared__ int s[257];
-    int t = threadIdx.x;
-    if (t <= a.nkeys) s[t] = a.ctl->hist[t];
+// Exclusive scan over the block of one value per thread (blockDim.x a multiple
+// of 32, at most 1024); *total receives the sum. s_w holds 32 ints.
+RT_D int block_scan(int v, int* s_w, int* total) {
+    const unsigned full = 0xffffffffu;
+    int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        int x = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) s_w[w] = incl;
     __syncthreads();
-    if (t == 0) {
-        int acc = 0;
-        for (int k = 0; k <= a.nkeys; k++) {
-            int c = s[k];
-            s[k] = acc;
-            acc += c;
+    if (w == 0) {
+        int x = lane < nw ? s_w[lane] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(full, x, o);
+            if (lane >= o) x += y;
         }
+        s_w[lane] = x;
     }
     __syncthreads();
-    if (t <= a.nkeys) a.ctl->hist[t] = s[t];
+    *total = s_w[nw - 1];
+    return (w ? s_w[w - 1] : 0) + incl - v;
 }
-__global__ void k_wf_scatter(WfArgs a) {
+
+// Counting sort of the live slots by material. Every block scans the histogram
+// itself (at most 256 keys), so the sort is one launch.
+__global__ void __launch_bounds__(256) k_wf_scatter(const __grid_constant__ WfArgs a) {
+    __shared__ int s_w[32], s_off[256];
+    int v = (int)threadIdx.x <= a.nkeys ? a.ctl->hist[threadIdx.x] : 0;
+    int live;
+    s_off[threadIdx.x] = block_scan(v, s_w, &live);
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->nlive = live;
+    __syncthreads();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nslots) return;
     if (!(fbits(a.P.d[i].w) & PF_ALIVE)) return;
@@ -841,8 +860,8 @@ __global__ void k_wf_scatter(WfArgs a) {
     int leader = __ffs(grp) - 1;
     int rank = __popc(grp & ((1u << lane) - 1u));
     int base = 0;
-    if (lane == leader) base = atomicAdd(&a.ctl->hist[key], __popc(grp));
-    base = __shfl_sync(grp, base, leader);
+    if (lane == leader) base = atomicAdd(&a.ctl->cursor[key], __popc(grp));
+    base = __shfl_sync(grp, base, leader) + s_off[key];
     a.P.order[RT_IX(base + rank, a.nslots)] = i;
 }
 
@@ -857,7 +876,7 @@ struct QueueShadows : NoAdjoint {
             ps.add(c, to_la);   // records the per-frame sanitize in the mask
             return;
         }
-        if (n >= a->S.per || (a->S.limit > 0 && atomicAdd(a->S.count, 1) >= a->S.limit)) {
+        if (n >= a->S.per || (a->S.limit > 0 && atomicAdd(&a->ctl->nrec, 1) >= a->S.limit)) {
             atomicExch(&a->ctl->overflow, 1);
             return;
         }
@@ -916,7 +935,7 @@ __global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(const __g
     int i;
     if (a.sort) {
         // the scatter left the live slots in material order in order[0 .. live)
-        if (t >= a.ctl->hist[a.nkeys]) return;
+        if (t >= a.ctl->nlive) return;
         i = RT_IX(a.P.order[RT_IX(t, a.nslots)], a.nslots);
     } else {
         if (t >= a.nslots) return;
@@ -983,38 +1002,20 @@ __global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(const __g
 // Exclusive scan of a ray-sort key histogram (kRayKeys counts) into off (one
 // block of 1024 threads, a run of kRayKeys / 1024 keys each), clearing the
 // histogram for the next shade; *total receives the sum.
-__global__ void __launch_bounds__(1024) k_wf_rscan(int* hist, int* off, int* total) {
+RT_D void key_scan(int* hist, int* off, int* total) {
     constexpr int kPer = kRayKeys / 1024;
     static_assert(kPer % 4 == 0, "whole int4 runs per thread");
     __shared__ int s_w[32];
-    const unsigned full = 0xffffffffu;
-    int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    int4* h4 = reinterpret_cast<int4*>(hist) + t * (kPer / 4);
-    int4* o4 = reinterpret_cast<int4*>(off) + t * (kPer / 4);
+    int4* h4 = reinterpret_cast<int4*>(hist) + threadIdx.x * (kPer / 4);
+    int4* o4 = reinterpret_cast<int4*>(off) + threadIdx.x * (kPer / 4);
     int4 v[kPer / 4];
-    int sum = 0;
+    int sum = 0, all;
 #pragma unroll
     for (int k = 0; k < kPer / 4; k++) {
         v[k] = h4[k];
         sum += v[k].x + v[k].y + v[k].z + v[k].w;
     }
-    int incl = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-        int x = __shfl_up_sync(full, incl, o);
-        if (lane >= o) incl += x;
-    }
-    if (lane == 31) s_w[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-        int x = s_w[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(full, x, o);
-            if (lane >= o) x += y;
-        }
-        s_w[lane] = x;
-    }
-    __syncthreads();
-    int base = (w ? s_w[w - 1] : 0) + incl - sum;
+    int base = block_scan(sum, s_w, &all);
 #pragma unroll
     for (int k = 0; k < kPer / 4; k++) {
         int4 r;
@@ -1026,13 +1027,44 @@ __global__ void __launch_bounds__(1024) k_wf_rscan(int* hist, int* off, int* tot
         o4[k] = r;
         h4[k] = make_int4(0, 0, 0, 0);
     }
-    if (t == 1023) *total = base;
+    if (threadIdx.x == 0) *total = all;
+}
+
+// Between shade and occlude, one launch of up to three blocks: block 0 ends the
+// iteration's bookkeeping (whether the loop goes on, and the counters that the
+// next iteration accumulates; occlude reads none of them), block 1 scans the
+// bounce rays' keys, block 2 the shadow records'. loop: the graph's loop
+// condition, 0 when the host runs the iterations itself.
+__global__ void __launch_bounds__(1024) k_wf_plan(const __grid_constant__ WfArgs a, cudaGraphConditionalHandle loop) {
+    WfCtl* c = a.ctl;
+    if (blockIdx.x == 1) {
+        key_scan(a.rhist, a.roff, &c->nbounce);
+    } else if (blockIdx.x == 2) {
+        key_scan(a.shist, a.soff, &c->nshadow);
+    } else {
+        if (threadIdx.x == 0) {
+            c->iters++;
+            c->done = c->next >= c->total && c->live == 0;
+            if (loop && (c->done || c->overflow || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
+            c->iter_first = c->next;
+            c->live = 0;
+            c->ext_next = 0;
+            c->occ_next = 0;
+            c->nfree = 0;
+            c->free_next = 0;
+            c->nrec = 0;
+        }
+        if (threadIdx.x < 256) {
+            c->hist[threadIdx.x] = 0;
+            c->cursor[threadIdx.x] = 0;
+        }
+    }
 }
 
 // The record that thread t of shade wrote k-th, or -1. Under the material sort
 // shade ran the threads below the live count alone.
 RT_D int shadow_record(const WfArgs& a, int t, int k) {
-    int live = a.sort ? a.ctl->hist[a.nkeys] : a.nslots;
+    int live = a.sort ? a.ctl->nlive : a.nslots;
     if (t >= live || k >= a.S.cnt[RT_IX(t, a.nslots)]) return -1;
     return k * a.nslots + t;
 }
@@ -1137,22 +1169,6 @@ __global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid
     atomicAdd(f, v.x);
     atomicAdd(f + 1, v.y);
     atomicAdd(f + 2, v.z);
-}
-
-// Per-iteration reset of the counters the next iteration accumulates.
-__global__ void k_wf_reset(WfArgs a) {
-    int t = threadIdx.x;
-    if (t == 0) {
-        *a.S.count = 0;
-        a.ctl->live = 0;
-        a.ctl->ext_next = 0;
-        a.ctl->occ_next = 0;
-        a.ctl->nfree = 0;
-        a.ctl->free_next = 0;
-        a.ctl->iter_first = a.ctl->next;
-    }
-    if (a.sort)
-        for (int k = t; k <= a.nkeys; k += blockDim.x) a.ctl->hist[k] = 0;
 }
 
 // Mean of the accumulated sums into the films (Renderer.cs:711).

@@ -23,7 +23,7 @@ namespace rt {
 template <int STACK, bool MEDIUM, bool TRANSMIT>
 __global__ void __launch_bounds__(128) k_wf_adjoint(const __grid_constant__ WfArgs a) {
     extern __shared__ float s_acc[];
-    const WfAdjoint& J = a.J;
+    const WfAdjoint& J = *a.J;
     const int nacc = J.use_local ? J.nact : (J.use_shared ? J.nparams : 0);
     for (int k = threadIdx.x; k < nacc; k += blockDim.x) s_acc[k] = 0.0f;
     float loc[kAdjLocal];
@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(128) k_wf_adjoint(const __grid_constant__ WfAr
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     int i = -1;
     if (a.sort) {   // the scatter left the live slots in material order in order[0 .. live)
-        if (t < a.ctl->hist[a.nkeys]) i = RT_IX(a.P.order[RT_IX(t, a.nslots)], a.nslots);
+        if (t < a.ctl->nlive) i = RT_IX(a.P.order[RT_IX(t, a.nslots)], a.nslots);
     } else if (t < a.nslots) {
         i = t;
     }
