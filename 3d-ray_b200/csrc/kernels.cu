@@ -1040,7 +1040,10 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     size_t adj_shmem = 0;
     if (mode == rt::WF_REPLAY)
         adj_shmem = (size_t)(J.use_local ? J.nact : (J.use_shared ? J.nparams : 0)) * sizeof(float);
-    unsigned gs = (unsigned)((nslots + blk - 1) / blk);
+    // shade: smaller blocks where the slots would not give every SM one
+    int sblk = rt::kShadeBlock;
+    while (sblk > 64 && (int64_t)sblk * 148 > nslots) sblk /= 2;
+    unsigned gs = (unsigned)((nslots + sblk - 1) / sblk);
     unsigned gst = (unsigned)((nslots + tblk - 1) / tblk);
     dim3 gsh(gst, (unsigned)max_shadow);   // occlude and the shadow scatter: (shade's threads, records of each)
     unsigned g256 = (unsigned)((nslots + 255) / 256);
@@ -1080,7 +1083,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
             else if (transmit) rt::k_wf_adjoint<kStack, false, true><<<gadj, adj_blk, adj_shmem, stream>>>(a);
             else rt::k_wf_adjoint<kStack, false, false><<<gadj, adj_blk, adj_shmem, stream>>>(a);
         } else {
-            shade<<<gs, blk, 0, stream>>>(a);
+            shade<<<gs, sblk, 0, stream>>>(a);
         }
         if (ev) cudaEventRecord(ev[4], stream);   // the ray sorts' scans and scatter count as sorting
         rt::k_wf_plan<<<gplan, 1024, 0, stream>>>(a, loop);

@@ -925,12 +925,15 @@ RT_D Hit wf_hit(const WfArgs& a, int i) {
     return h;
 }
 
-// Minimum resident blocks of 256 for shade (a register budget); a build knob.
-#ifndef RT_SHADE_MIN_BLOCKS
-#define RT_SHADE_MIN_BLOCKS 2
-#endif
+// Threads of a shade block: 512 at 128 registers fill an SM. Shade waits for
+// instructions, and the warps of one block start together and share what they
+// fetch: with two blocks of 256 instead, shade took 29.4 against 26.7 ms on a
+// full-HD icosphere frame of 64 samples and 44.0 against 39.2 ms on four foggy
+// views; blocks of 768 and 1024 threads (80 and 64 registers) spill and took
+// 26.8 and 27.6, 42.5 and 45.5 ms.
+constexpr int kShadeBlock = 512;
 template <bool MEDIUM, bool TRANSMIT, bool ONE>
-__global__ void __launch_bounds__(256, RT_SHADE_MIN_BLOCKS) k_wf_shade(const __grid_constant__ WfArgs a) {
+__global__ void __launch_bounds__(kShadeBlock, 1) k_wf_shade(const __grid_constant__ WfArgs a) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     int i;
     if (a.sort) {
