@@ -136,7 +136,7 @@ RT_D Df lut_e_dual(const float* e, float mu, Df alpha) {
     return Df{x0 + (x1 - x0) * tu, dx0 + (dx1 - dx0) * tu};
 }
 
-RT_NI DMat dual_material(const SceneView& s, const Material& m, const float* p, int k) {
+RT_D DMat dual_material(const SceneView& s, const Material& m, const float* p, int k) {
     auto seed = [&](int i) { return Df{p[i], i == k ? 1.0f : 0.0f}; };
     DMat r;
     D3 bc = D3{seed(0), seed(1), seed(2)};
@@ -194,6 +194,16 @@ RT_NI DMat dual_material(const SceneView& s, const Material& m, const float* p, 
     r.sheen = sheen;
     r.clearcoat = clearcoat;
     return r;
+}
+
+// The dual materials of every differentiated (material, BSDF slot) pair, one
+// thread each, once per rt_adjoint call: they depend on the parameters alone.
+// The hooks used to build theirs at every NEE sample and every bounce.
+__global__ void k_dual_materials(SceneView s, const float* params, const unsigned* mmask, int nmat, DMat* out) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int mat = i / kAdjBsdfDirs, k = i % kAdjBsdfDirs;
+    if (mat >= nmat || !((mmask[mat] >> k) & 1u) || s.materials[mat].type != 0) return;
+    out[i] = dual_material(s, s.materials[mat], params + mat * kAdjPerMat, k);
 }
 
 // ---------------------------------------------------------------------------
@@ -459,6 +469,7 @@ struct AdjointSink {
     const SceneView* s;
     const float* params;   // raw parameter vector (device), 16 per material
     const unsigned* mmask; // per material: bit k = slot k is differentiated
+    const DMat* dmat;      // per material and BSDF slot: the dual material (k_dual_materials)
     unsigned gmask;        // the 6 global (medium) slots
     float* loc;            // per-thread accumulators (kAdjLocal), or null
     float* acc;            // block accumulators in shared memory, or null
@@ -520,11 +531,11 @@ struct AdjointSink {
 
     // The transparent walk of shadow_transmittance, recording the absorption
     // lengths and surface crossings that the gradient needs.
-    template <int STACK>
+    template <int STACK, bool TRANSMIT>
     RT_D V3 walk(V3 o, V3 d, float tmin, float tmax) {
         sh_n = 0;
         Hit h;
-        if (opaque) {
+        if (!TRANSMIT || opaque) {
             if (any4) traverse4_any<STACK>(*s, o, d, tmin, tmax, h, err);
             else traverse<true, STACK>(*s, o, d, tmin, tmax, h, nullptr, err);
             return h.kind == HIT_NONE ? v3(1.0f) : v3(0.0f);
@@ -617,9 +628,9 @@ struct AdjointSink {
     }
 
     // ---- the hooks of shade_vertex
-    template <int STACK>
+    template <int STACK, bool TRANSMIT>
     RT_D void shadow_impl(PathState& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
-        V3 tr = walk<STACK>(o, d, kEps, tmax);
+        V3 tr = walk<STACK, TRANSMIT>(o, d, kEps, tmax);
         sh_added = !near_zero(tr);
         if (!sh_added) return;
         sh_tr = tr;
@@ -771,10 +782,9 @@ struct AdjointSink {
         if (!bits) return;
         V3 w = gain(ps, to_la) * coef * tr_m * sh_tr * term;
         if (is_zero(w)) return;
-        const float* p = params + rec.material * kAdjPerMat;
         for (; bits; bits &= bits - 1u) {
             int k = __ffs(bits) - 1;
-            DMat dm = dual_material(*s, m, p, k);
+            const DMat& dm = dmat[rec.material * kAdjBsdfDirs + k];
             add(rec.material * kAdjPerMat + k, dot(w, dpart(eval_direct_dual(*s, m, dm, rec, L, V))));
         }
     }
@@ -807,10 +817,9 @@ struct AdjointSink {
         if (is_zero(coef)) return;
         float cw = 1.0f;
         if (mode == SCATTER_SAMPLED) cw = fabsf(dot(rec.n, dir)) / pdf;
-        const float* p = params + rec.material * kAdjPerMat;
         for (; bits; bits &= bits - 1u) {
             int k = __ffs(bits) - 1;
-            DMat dm = dual_material(*s, m, p, k);
+            const DMat& dm = dmat[rec.material * kAdjBsdfDirs + k];
             V3 da = mode == SCATTER_SAMPLED ? dpart(eval_dual(*s, m, dm, rec, V, dir)) * cw
                                             : dpart(lobe_att_dual(*s, m, dm, rec, V, dir, lobe));
             if (mode != SCATTER_SAMPLED) {
@@ -824,7 +833,9 @@ struct AdjointSink {
     }
 };
 
-template <int STACK>
+// TRANSMIT = false: a scene of opaque materials, whose shadow rays are any-hit
+// walks; the transparent walk and its records compile away.
+template <int STACK, bool TRANSMIT>
 struct AdjointReplay : AdjointSink {
     // the adjoint captures no AOVs
     RT_D void aov_ray(const Hit&, V3) {}
@@ -833,7 +844,7 @@ struct AdjointReplay : AdjointSink {
     RT_D void aov_surface(V3, const Material&) {}
     RT_D void aov_bounce(bool, V3) {}
     RT_D void shadow(PathState& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
-        shadow_impl<STACK>(ps, o, d, tmax, c, to_la);
+        shadow_impl<STACK, TRANSMIT>(ps, o, d, tmax, c, to_la);
     }
 };
 

@@ -313,6 +313,7 @@ struct AdjArgs {
     const float* dimg;     // 3*H*W planar dLoss/dfilm
     const float* params;   // raw parameter vector
     const unsigned* mmask; // per material slot masks
+    const rt::DMat* dmat;  // per material and BSDF slot: the dual material
     unsigned gmask;        // global slot mask
     double* grad;          // accumulators, nparams
     int nparams;
@@ -381,10 +382,11 @@ __global__ void RT_ADJ_BOUNDS k_adjoint(rt::SceneView s, rt::RenderConst rc, Adj
             }
         }
         // adjoints of the resolve (path_resolve)
-        rt::AdjointReplay<STACK> adj;
+        rt::AdjointReplay<STACK, true> adj;
         adj.s = &s;
         adj.params = a.params;
         adj.mmask = a.mmask;
+        adj.dmat = a.dmat;
         adj.gmask = a.gmask;
         adj.loc = a.use_local ? loc : nullptr;
         adj.acc = a.use_shared ? sacc : nullptr;
@@ -1035,7 +1037,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         gpt_e = (unsigned)std::max(1, nb_e * sms);
         gpt_o = (unsigned)std::max(1, nb_o * sms);
     }
-    const int adj_blk = 128;
+    int adj_blk = rt::kAdjBlock;
+    while (adj_blk > 64 && (int64_t)adj_blk * 148 > nslots) adj_blk /= 2;
     unsigned gadj = (unsigned)((nslots + adj_blk - 1) / adj_blk);
     size_t adj_shmem = 0;
     if (mode == rt::WF_REPLAY)
@@ -1109,7 +1112,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         // bytes key the cached ones.
         const unsigned shape[] = {(unsigned)blk, (unsigned)tblk, (unsigned)l4, (unsigned)l4_occ, (unsigned)pt,
                                   (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst,
-                                  (unsigned)max_shadow, g256, gcam, gplan, (unsigned)mode, gadj, (unsigned)adj_shmem};
+                                  (unsigned)max_shadow, g256, gcam, gplan, (unsigned)mode, gadj, (unsigned)adj_blk, (unsigned)adj_shmem};
         std::vector<unsigned char> key(sizeof(a) + sizeof(shape));
         std::memcpy(key.data(), &a, sizeof(a));
         std::memcpy(key.data() + sizeof(a), shape, sizeof(shape));
@@ -2121,11 +2124,13 @@ int rt_adjoint(RtScene* sc, const RtRenderParams* p, const float* dimg, const ui
         bool on = i < nm * kPerMat ? ((hm[(size_t)(i / kPerMat)] >> (i % kPerMat)) & 1u) : ((gm >> (i - nm * kPerMat)) & 1u);
         if (on) act.push_back(i);
     }
-    size_t bytes = (size_t)np * sizeof(double) + (size_t)np * sizeof(float) + film * sizeof(float) +
+    const size_t nd = (size_t)nm * rt::kAdjBsdfDirs;
+    size_t bytes = nd * sizeof(rt::DMat) + (size_t)np * sizeof(double) + (size_t)np * sizeof(float) + film * sizeof(float) +
                    (size_t)nm * sizeof(unsigned) + (size_t)(act.size() + 1) * sizeof(int) + 256;
     void* mem = nullptr;
     if (cudaMalloc(&mem, bytes) != cudaSuccess) return fail(RT_ERR_OOM, "adjoint buffers");
-    char* base = static_cast<char*>(mem);
+    rt::DMat* d_dmat = static_cast<rt::DMat*>(mem);
+    char* base = static_cast<char*>(mem) + nd * sizeof(rt::DMat);
     double* d_grad = reinterpret_cast<double*>(base);
     float* d_params = reinterpret_cast<float*>(base + (size_t)np * sizeof(double));
     float* d_img = d_params + np;
@@ -2145,7 +2150,12 @@ int rt_adjoint(RtScene* sc, const RtRenderParams* p, const float* dimg, const ui
              "slot list copy");
     step(cudaMemsetAsync(d_grad, 0, (size_t)np * sizeof(double), sc->stream), "gradient clear");
     step(cudaMemsetAsync(sc->d_err, 0, sizeof(int), sc->stream), "error clear");
+    if (rc == RT_OK) {
+        rt::k_dual_materials<<<(unsigned)((nd + 63) / 64), 64, 0, sc->stream>>>(sc->view, d_params, d_mask, nm, d_dmat);
+        step(cudaGetLastError(), "dual materials launch");
+    }
     AdjArgs a;
+    a.dmat = d_dmat;
     a.x0 = p->pixel_x0;
     a.y0 = p->pixel_y0;
     a.ww = ww;
@@ -2179,6 +2189,7 @@ int rt_adjoint(RtScene* sc, const RtRenderParams* p, const float* dimg, const ui
         J.inv_spp = 1.0f / (float)p->spp;
         J.params = d_params;
         J.mmask = d_mask;
+        J.dmat = d_dmat;
         J.gmask = gm;
         J.nparams = np;
         J.medium_base = nm * kPerMat;

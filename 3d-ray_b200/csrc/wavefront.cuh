@@ -137,6 +137,7 @@ struct WfAdjoint {
     float inv_spp;          // 1 / the request's spp: the film is the mean of its samples
     const float* params;    // raw parameter vector, 16 per material, then the medium's 6
     const unsigned* mmask;  // per material: bit k = slot k is differentiated
+    const DMat* dmat;       // per material and BSDF slot: the dual material
     unsigned gmask;         // the medium's slots
     int nparams, medium_base;
     const int* act;         // the differentiated slots, nact of them

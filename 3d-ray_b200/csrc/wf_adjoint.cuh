@@ -20,8 +20,14 @@
 
 namespace rt {
 
+// Threads of a block: 512 at 128 registers, an SM's worth, for the reason of
+// kShadeBlock. The replay's registers (177 to 195 without a bound) spill 164 to
+// 404 bytes at that size and it is still the fastest: on a fit step of
+// 256x256x32 samples the adjoint took 18.3 ms in blocks of 128, 18.2 in blocks
+// of 256 (8 warps an SM each) and 16.6 in blocks of 512.
+constexpr int kAdjBlock = 512;
 template <int STACK, bool MEDIUM, bool TRANSMIT>
-__global__ void __launch_bounds__(128) k_wf_adjoint(const __grid_constant__ WfArgs a) {
+__global__ void __launch_bounds__(kAdjBlock, 1) k_wf_adjoint(const __grid_constant__ WfArgs a) {
     extern __shared__ float s_acc[];
     const WfAdjoint& J = *a.J;
     const int nacc = J.use_local ? J.nact : (J.use_shared ? J.nparams : 0);
@@ -45,10 +51,11 @@ __global__ void __launch_bounds__(128) k_wf_adjoint(const __grid_constant__ WfAr
         PathState ps;
         wf_load(a, i, R, ps);
         Hit h = wf_hit(a, i);
-        AdjointReplay<STACK> adj;
+        AdjointReplay<STACK, TRANSMIT> adj;
         adj.s = &s;
         adj.params = J.params;
         adj.mmask = J.mmask;
+        adj.dmat = J.dmat;
         adj.gmask = J.gmask;
         adj.loc = J.use_local ? loc : nullptr;
         adj.acc = (!J.use_local && J.use_shared) ? s_acc : nullptr;
