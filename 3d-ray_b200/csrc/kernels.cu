@@ -1358,6 +1358,8 @@ int rt_scene_create_ex(const RtWorldDesc* world, const RtSceneOptions* options, 
     v.top_is_bvh = h.top_is_bvh;
     v.top_root = h.top_root_code;
     v.top_root4 = h.top_root4;
+    v.walk_root = h.walk_root;
+    v.walk_root4 = h.walk_root4;
     v.num_top_items = (int)h.top_items.size();
     v.n_cnodes = (int)(h.cnodes.size() / 4);
     v.n_cnodes4 = (int)(h.cnodes4.size() / 8);

@@ -179,6 +179,14 @@ struct SceneView {
     int top_root;               // child code of the top-level root (top_is_bvh only)
     int top_root4;              // the same in the four-wide layout
     int num_top_items;          // flat list: entity count
+    // Where the walks start (the counting build and Walker start at top_root or
+    // the flat list). A copy of the top level in which a leaf's entities are
+    // children of records: a mesh BVH's root stands there with its entity box,
+    // so entering a mesh costs no leaf, no entity record and no second box
+    // test; a quad, sphere or list mesh, which the reference tests without a box
+    // of its own, stands there with an unbounded one. Order 3 (in place of an
+    // axis) visits the children first to last, as the list is. May be a leaf code.
+    int walk_root, walk_root4;
     int has_medium;
     V3 sigma_a, sigma_s, sigma_t;
     float hg_g;

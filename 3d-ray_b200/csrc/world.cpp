@@ -380,6 +380,132 @@ bool make_smooth(const RtWorldDesc* w, int64_t i, SmoothTri& st) {
     return true;
 }
 
+// Appends the kernels' top level (SceneView::walk_root) to both record arrays,
+// once the entities' mesh roots are child codes.
+struct WalkBuilder {
+    HostScene& sc;
+    struct Kid {
+        Box box;
+        int code = INT_MIN, code4 = INT_MIN;
+    };
+    static Box unbounded() {
+        const float inf = std::numeric_limits<float>::infinity();
+        return {v3(-inf), v3(inf)};
+    }
+    static float bits(int i) {
+        float f;
+        std::memcpy(&f, &i, 4);
+        return f;
+    }
+    // One entity of a list. `tested`: its own box was tested where its leaf's was.
+    Kid entity(int e) const {
+        const Entity& en = sc.entities[e];
+        if (en.kind != ENT_MESH) {
+            int c = leaf_code(e, LEAF_ENT1, 1);
+            return {unbounded(), c, c};
+        }
+        Kid k{unbounded(), en.index, sc.mesh_root4[(size_t)e]};
+        if (en.index >= 0) {
+            const float4 &lo = sc.ent_box[2 * (size_t)e], &hi = sc.ent_box[2 * (size_t)e + 1];
+            k.box = {v3(lo.x, lo.y, lo.z), v3(hi.x, hi.y, hi.z)};
+        }
+        return k;
+    }
+    int record2(const Kid& l, const Kid& r, int axis) const {
+        int i = (int)(sc.cnodes.size() / 4);
+        sc.cnodes.push_back(float4{l.box.mn.x, l.box.mn.y, l.box.mn.z, bits(l.code)});
+        sc.cnodes.push_back(float4{l.box.mx.x, l.box.mx.y, l.box.mx.z, bits(r.code)});
+        sc.cnodes.push_back(float4{r.box.mn.x, r.box.mn.y, r.box.mn.z, bits(axis)});
+        sc.cnodes.push_back(float4{r.box.mx.x, r.box.mx.y, r.box.mx.z, 0.0f});
+        return i;
+    }
+    int record4(const Kid k[4], const int axes[3]) const {
+        int i = (int)(sc.cnodes4.size() / 8);
+        const float inf = std::numeric_limits<float>::infinity();
+        float lo[3][4], hi[3][4], cf[4];
+        for (int j = 0; j < 4; j++) {
+            bool used = k[j].code4 != INT_MIN;
+            for (int a = 0; a < 3; a++) {
+                lo[a][j] = used ? axis_of(k[j].box.mn, a) : inf;
+                hi[a][j] = used ? axis_of(k[j].box.mx, a) : inf;
+            }
+            cf[j] = bits(k[j].code4);
+        }
+        for (int a = 0; a < 3; a++) sc.cnodes4.push_back(float4{lo[a][0], lo[a][1], lo[a][2], lo[a][3]});
+        for (int a = 0; a < 3; a++) sc.cnodes4.push_back(float4{hi[a][0], hi[a][1], hi[a][2], hi[a][3]});
+        sc.cnodes4.push_back(float4{cf[0], cf[1], cf[2], cf[3]});
+        sc.cnodes4.push_back(float4{bits(axes[0]), bits(axes[1]), bits(axes[2]), 0.0f});
+        return i;
+    }
+    // A list of entities in order (a top-level leaf, at most 4, or the flat list).
+    Kid list(const int* items, int n) const {
+        if (n == 1) return entity(items[0]);
+        Kid out{unbounded(), 0, 0};
+        out.code = record2(entity(items[0]), list2(items + 1, n - 1), 3);
+        Kid k[4];
+        for (int j = 0; j < n; j++) k[j] = entity(items[j]);
+        const int order[3] = {3, 3, 3};
+        out.code4 = record4(k, order);
+        return out;
+    }
+    Kid list2(const int* items, int n) const {   // the rest of a list, in the two-wide layout alone
+        if (n == 1) return entity(items[0]);
+        Kid out{unbounded(), 0, INT_MIN};
+        out.code = record2(entity(items[0]), list2(items + 1, n - 1), 3);
+        return out;
+    }
+    // The binary top-level tree, its leaves as lists; kids4 of a record are the
+    // node's grandchildren where a child is an interior node itself.
+    struct Node {
+        Kid self;
+        bool inner = false;
+        int axis = 0;
+        Kid l, r;
+    };
+    Node node(int n) const {
+        const NodeF& f = sc.nodes[n];
+        int a, b;
+        std::memcpy(&a, &f.lo[3], 4);
+        std::memcpy(&b, &f.hi[3], 4);
+        Node out;
+        Box box{v3(f.lo[0], f.lo[1], f.lo[2]), v3(f.hi[0], f.hi[1], f.hi[2])};
+        if (a < 0) {
+            out.self = list(&sc.top_items[~a], b & 0xFFFF);
+            out.self.box = box;   // the leaf's own box guards the list
+            return out;
+        }
+        Node L = node(a), R = node(b & 0x3FFFFFFF);
+        out.inner = true;
+        out.axis = (int)((unsigned)b >> 30);
+        out.l = L.self;
+        out.r = R.self;
+        out.self.box = box;
+        out.self.code = record2(L.self, R.self, out.axis);
+        Kid k[4];
+        int axes[3] = {out.axis, 0, 0};
+        for (int side = 0; side < 2; side++) {
+            const Node& c = side == 0 ? L : R;
+            if (c.inner) {
+                k[2 * side] = c.l;
+                k[2 * side + 1] = c.r;
+                axes[1 + side] = c.axis;
+            } else {
+                k[2 * side] = c.self;
+            }
+        }
+        out.self.code4 = record4(k, axes);
+        return out;
+    }
+};
+
+void build_walk(HostScene& sc) {
+    WalkBuilder b{sc};
+    WalkBuilder::Kid root = sc.top_is_bvh ? b.node(sc.top_root).self
+                                          : b.list(sc.top_items.data(), (int)sc.top_items.size());
+    sc.walk_root = root.code;
+    sc.walk_root4 = root.code4;
+}
+
 }  // namespace
 
 int build_world(const RtWorldDesc* w, HostScene& sc, std::string& err, const BuildOptions& opt) {
@@ -703,6 +829,7 @@ int build_world(const RtWorldDesc* w, HostScene& sc, std::string& err, const Bui
         }
         for (int e : mesh_ids) sc.entities[e].index = code_of(sc.entities[e].index);
     }
+    build_walk(sc);
     // --- explicit lights (SceneLoader.cs:446-458)
     for (int i = 0; i < w->num_lights; i++) {
         const RtLightDesc& d = w->lights[i];
