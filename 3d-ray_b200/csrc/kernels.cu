@@ -2,12 +2,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
 #include <functional>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/rt3d.h"
@@ -72,6 +74,8 @@ struct RtScene {
     int* d_err = nullptr;
     float* film = nullptr;         // rt_render's device film, kept between calls
     size_t film_bytes = 0;
+    void* rec = nullptr;           // the wavefront adjoint's sample record, kept between calls up to a bound
+    size_t rec_bytes = 0;
     int tuned = 0;                 // rt_autotune ran: use the fields below
     int tuned_slots = 0, tuned_block = 0, tuned_sort = 0, tuned_layout = 2, tuned_fetch = 1, tuned_tblock = 0, tuned_groups = 0;
     // Copy of the world description: rt_scene_set_params rebuilds from it.
@@ -155,6 +159,93 @@ int ensure_scratch(RtScene* sc, size_t bytes) {
     if (cudaMalloc(&sc->scratch, bytes) != cudaSuccess) return fail(RT_ERR_OOM, "scratch allocation failed");
     sc->scratch_bytes = bytes;
     return RT_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Large copies between the device and a caller's pageable memory. The driver
+// stages such a copy through its own pinned buffers on one host thread, which
+// also takes the page faults of a fresh destination: a full-HD film (25 MB) took
+// 4 to 8 ms each way, the link needs 0.5. Here four threads move the chunks of
+// a pinned window (one per device, 32 MiB, kept) while the next ones are on the
+// link. A copy below 1 MiB, or one that finds the window in use by another
+// thread's call, goes the driver's way. Both return with the copy done.
+// ---------------------------------------------------------------------------
+constexpr size_t kStageChunk = size_t(1) << 20, kStageChunks = 32;
+constexpr int kStageThreads = 4;
+struct Stage {
+    std::mutex mu;
+    char* mem = nullptr;
+    cudaEvent_t landed[kStageChunks] = {};
+};
+Stage g_stage[16];
+
+cudaError_t stage_copy(int dev, cudaStream_t stream, char* host, char* device, size_t n, bool to_host) {
+    auto plain = [&] {
+        cudaError_t e = to_host ? cudaMemcpyAsync(host, device, n, cudaMemcpyDeviceToHost, stream)
+                                : cudaMemcpyAsync(device, host, n, cudaMemcpyHostToDevice, stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+    };
+    if (n < kStageChunk || dev < 0 || dev >= 16) return plain();
+    cudaPointerAttributes at_host{};
+    if (cudaPointerGetAttributes(&at_host, host) == cudaSuccess && at_host.type != cudaMemoryTypeUnregistered)
+        return plain();   // pinned or device-accessible memory: the link takes it as it is
+    Stage& st = g_stage[dev];
+    std::unique_lock<std::mutex> lk(st.mu, std::try_to_lock);
+    if (!lk.owns_lock()) return plain();
+    if (!st.mem) {
+        if (cudaMallocHost(&st.mem, kStageChunk * kStageChunks) != cudaSuccess) {
+            st.mem = nullptr;
+            cudaGetLastError();   // no window: the driver's way
+            return plain();
+        }
+        for (cudaEvent_t& e : st.landed) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    }
+    for (size_t w = 0; w < n; w += kStageChunk * kStageChunks) {   // one window at a time
+        const size_t bytes = std::min(n - w, kStageChunk * kStageChunks);
+        const size_t chunks = (bytes + kStageChunk - 1) / kStageChunk;
+        std::atomic<int> err{cudaSuccess};
+        auto note = [&](cudaError_t e) {
+            int none = cudaSuccess;
+            if (e != cudaSuccess) err.compare_exchange_strong(none, e);
+        };
+        auto len = [&](size_t c) { return std::min(kStageChunk, bytes - c * kStageChunk); };
+        if (to_host)
+            for (size_t c = 0; c < chunks; c++) {
+                note(cudaMemcpyAsync(st.mem + c * kStageChunk, device + w + c * kStageChunk, len(c),
+                                     cudaMemcpyDeviceToHost, stream));
+                note(cudaEventRecord(st.landed[c], stream));
+            }
+        std::atomic<size_t> at{0};
+        auto work = [&] {
+            cudaSetDevice(dev);
+            for (size_t c; (c = at.fetch_add(1)) < chunks;) {
+                char *mine = st.mem + c * kStageChunk, *theirs = host + w + c * kStageChunk;
+                if (to_host) {
+                    note(cudaEventSynchronize(st.landed[c]));
+                    std::memcpy(theirs, mine, len(c));
+                } else {
+                    std::memcpy(mine, theirs, len(c));
+                    note(cudaMemcpyAsync(device + w + c * kStageChunk, mine, len(c), cudaMemcpyHostToDevice, stream));
+                }
+            }
+        };
+        std::vector<std::thread> pool;
+        try {
+            for (size_t k = 1; k < std::min<size_t>(kStageThreads, chunks); k++) pool.emplace_back(work);
+        } catch (const std::exception&) {   // no more threads: this one does the rest
+        }
+        work();
+        for (std::thread& t : pool) t.join();
+        note(cudaStreamSynchronize(stream));   // before the window is used again
+        if (err != cudaSuccess) return static_cast<cudaError_t>(err.load());
+    }
+    return cudaSuccess;
+}
+cudaError_t copy_to_host(int dev, cudaStream_t stream, void* dst, const void* src, size_t n) {
+    return stage_copy(dev, stream, static_cast<char*>(dst), static_cast<char*>(const_cast<void*>(src)), n, true);
+}
+cudaError_t copy_to_device(int dev, cudaStream_t stream, void* dst, const void* src, size_t n) {
+    return stage_copy(dev, stream, static_cast<char*>(const_cast<void*>(src)), static_cast<char*>(dst), n, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -696,7 +787,8 @@ struct HostReq {
     rt::RenderConst rc;
     int x0, y0, ww, wh, spp, spp0;
     int W, H;
-    float* d_film;
+    float* d_film;          // the device film, or null: one from the workspace,
+    float* host_film = nullptr;   // copied here (3*W*H floats) when the render is done
 };
 
 // An instantiated graph: the loop of wavefront iterations (a conditional node
@@ -868,6 +960,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     rt::WfCtl* d_ctl;
     float** d_films;
     rt::WfOne* d_one;
+    std::vector<float*> films(reqs.size());
+    for (size_t r = 0; r < reqs.size(); r++) films[r] = reqs[r].d_film;
     rt::WfAdjoint* d_adj;
     rt::WfAdjoint J{};
     if (adj) J = *adj;
@@ -898,6 +992,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         take(a.P.d, nslots);
         for (auto& q : wreq) take(q.accum, (size_t)3 * q.ww * q.wh);
         clear_end = off;
+        for (size_t r = 0; r < reqs.size(); r++)
+            if (reqs[r].host_film) take(films[r], (size_t)3 * reqs[r].W * reqs[r].H);
         take(a.P.o, nslots);
         take(a.P.beta, nslots);
         take(a.P.w, nslots);
@@ -945,10 +1041,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
             return fail(RT_ERR_OOM, "pinned staging allocation failed");
         ws.pinned_bytes = pin_need;
     }
-    std::vector<float*> films(reqs.size());
     std::vector<int> fdims(2 * reqs.size());
     for (size_t r = 0; r < reqs.size(); r++) {
-        films[r] = reqs[r].d_film;
         fdims[r] = reqs[r].W;
         fdims[reqs.size() + r] = reqs[r].H;
     }
@@ -1169,6 +1263,10 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         if (mode == rt::WF_RENDER)
             rt::k_wf_finalize<<<g, 256, 0, stream>>>(d_reqs, (int)wreq.size(), d_films, d_fdims, d_fdims + reqs.size());
         cudaError_t e = cudaEventRecord(s0->ev1, stream);
+        for (size_t r = 0; r < reqs.size() && e == cudaSuccess; r++)
+            if (reqs[r].host_film)
+                e = copy_to_host(dev, stream, reqs[r].host_film, films[r],
+                                 (size_t)3 * reqs[r].W * reqs[r].H * sizeof(float));
         if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) rc = fail(RT_ERR_CUDA, std::string("wavefront failed: ") + cudaGetErrorString(e));
@@ -1405,6 +1503,7 @@ int rt_scene_destroy(RtScene* sc) {
     if (sc->scratch) cudaFree(sc->scratch);
     if (sc->d_err) cudaFree(sc->d_err);
     if (sc->film) cudaFree(sc->film);
+    if (sc->rec) cudaFree(sc->rec);
     if (sc->ev0) cudaEventDestroy(sc->ev0);
     if (sc->ev1) cudaEventDestroy(sc->ev1);
     if (sc->stream) cudaStreamDestroy(sc->stream);
@@ -1522,7 +1621,7 @@ int rt_render_capture(RtScene* sc, const RtRenderParams* p, float* out, const Rt
     for (int k = 0; k < 9; k++) {
         if (!dst[k]) continue;
         size_t nb = (size_t)(k < 7 ? 3 : 1) * npix * sizeof(float);
-        CUDA_TRY(cudaMemcpyAsync(dst[k], res + (size_t)first[k] * npix, nb, cudaMemcpyDeviceToHost, sc->stream));
+        CUDA_TRY(copy_to_host(sc->device, sc->stream, dst[k], res + (size_t)first[k] * npix, nb));
     }
     CUDA_TRY(cudaStreamSynchronize(sc->stream));
     rc_ = check_err(sc);
@@ -1672,8 +1771,7 @@ int rt_render(RtScene* sc, const RtRenderParams* p, float* out, RtStats* st) {
     }
     int rc = render_to_device(sc, p, sc->host.camera, sc->film, st);
     if (rc == RT_OK) {
-        if (cudaMemcpyAsync(out, sc->film, film_bytes, cudaMemcpyDeviceToHost, sc->stream) != cudaSuccess ||
-            cudaStreamSynchronize(sc->stream) != cudaSuccess)
+        if (copy_to_host(sc->device, sc->stream, out, sc->film, film_bytes) != cudaSuccess)
             rc = fail(RT_ERR_CUDA, "film copy failed");
     }
     if (st && rc == RT_OK)
@@ -1702,7 +1800,6 @@ int rt_render_batch(RtScene* const* scenes, int32_t num_scenes, const RtRequest*
     guards.reserve(locked.size());
     for (RtScene* sc : locked) guards.emplace_back(sc->mu);
     std::vector<HostReq> hq((size_t)n);
-    std::vector<float*> d_films((size_t)n, nullptr);
     int rc = RT_OK;
     for (int i = 0; i < n && rc == RT_OK; i++) {
         const RtRequest& q = reqs[i];
@@ -1720,11 +1817,6 @@ int rt_render_batch(RtScene* const* scenes, int32_t num_scenes, const RtRequest*
         p.spp_offset = 0;
         rc = validate_params(sc, &p);
         if (rc != RT_OK) break;
-        if (cudaSetDevice(sc->device) != cudaSuccess ||
-            cudaMalloc(&d_films[i], (size_t)3 * q.width * q.height * sizeof(float)) != cudaSuccess) {
-            rc = fail(RT_ERR_OOM, "film allocation failed");
-            break;
-        }
         HostReq& h = hq[i];
         h.scene = sc;
         h.rc = make_rc(sc, &p, q.camera);
@@ -1735,7 +1827,8 @@ int rt_render_batch(RtScene* const* scenes, int32_t num_scenes, const RtRequest*
         h.spp0 = 0;
         h.W = q.width;
         h.H = q.height;
-        h.d_film = d_films[i];
+        h.d_film = nullptr;
+        h.host_film = outs[i];
     }
     if (rc == RT_OK) {
         WfConfig cfg = g_wf_default;
@@ -1759,13 +1852,6 @@ int rt_render_batch(RtScene* const* scenes, int32_t num_scenes, const RtRequest*
         cfg.profile = common->profile_kernels != 0;
         apply_test_limits(cfg, common);
         rc = wf_render(hq, cfg, st);
-    }
-    for (int i = 0; i < n; i++) {
-        if (rc == RT_OK &&
-            cudaMemcpy(outs[i], d_films[i], (size_t)3 * reqs[i].width * reqs[i].height * sizeof(float),
-                       cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = fail(RT_ERR_CUDA, "film copy failed");
-        if (d_films[i]) cudaFree(d_films[i]);
     }
     if (st && rc == RT_OK)
         st->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -2004,6 +2090,7 @@ void put_params(RtScene* sc, const float* in) {
 // gradient hooks (WF_REPLAY). base carries the parameter, mask and gradient
 // buffers; ms and launches add up the passes.
 constexpr long long kAdjRecord = 1LL << 24;   // 64 B per recorded sample: 1 GiB
+constexpr size_t kAdjRecordKept = 256u << 20; // the most a scene keeps between calls
 
 int wf_adjoint(RtScene* sc, const RtRenderParams* p, const rt::WfAdjoint& base, double& ms, long long& launches) {
     WfConfig cfg;
@@ -2023,10 +2110,15 @@ int wf_adjoint(RtScene* sc, const RtRenderParams* p, const rt::WfAdjoint& base, 
     int per = (int)std::max<long long>(1, std::min<long long>(p->spp, kAdjRecord / std::max<long long>(npix, 1)));
     rt::WfAdjoint J = base;
     J.nrec = npix * per;
-    void* mem = nullptr;
-    if (cudaMalloc(&mem, (size_t)J.nrec * 4 * sizeof(float4)) != cudaSuccess)
-        return fail(RT_ERR_OOM, "adjoint sample record");
-    J.rec = static_cast<float4*>(mem);
+    const size_t rec_bytes = (size_t)J.nrec * 4 * sizeof(float4);
+    if (sc->rec_bytes < rec_bytes) {
+        if (sc->rec) cudaFree(sc->rec);
+        sc->rec = nullptr;
+        sc->rec_bytes = 0;
+        if (cudaMalloc(&sc->rec, rec_bytes) != cudaSuccess) return fail(RT_ERR_OOM, "adjoint sample record");
+        sc->rec_bytes = rec_bytes;
+    }
+    J.rec = static_cast<float4*>(sc->rec);
     for (int s0 = 0; s0 < p->spp && rc == RT_OK; s0 += per) {
         q.spp = std::min(per, p->spp - s0);
         q.spp0 = p->spp_offset + s0;
@@ -2038,7 +2130,11 @@ int wf_adjoint(RtScene* sc, const RtRenderParams* p, const rt::WfAdjoint& base, 
             launches += one.kernel_launches;
         }
     }
-    cudaFree(mem);
+    if (sc->rec_bytes > kAdjRecordKept) {   // a large record goes back at once
+        cudaFree(sc->rec);
+        sc->rec = nullptr;
+        sc->rec_bytes = 0;
+    }
     return rc;
 }
 
@@ -2129,8 +2225,9 @@ int rt_adjoint(RtScene* sc, const RtRenderParams* p, const float* dimg, const ui
     const size_t nd = (size_t)nm * rt::kAdjBsdfDirs;
     size_t bytes = nd * sizeof(rt::DMat) + (size_t)np * sizeof(double) + (size_t)np * sizeof(float) + film * sizeof(float) +
                    (size_t)nm * sizeof(unsigned) + (size_t)(act.size() + 1) * sizeof(int) + 256;
-    void* mem = nullptr;
-    if (cudaMalloc(&mem, bytes) != cudaSuccess) return fail(RT_ERR_OOM, "adjoint buffers");
+    rc_ = ensure_scratch(sc, bytes);   // kept by the scene: an optimiser calls this every step
+    if (rc_ != RT_OK) return rc_;
+    void* mem = sc->scratch;
     rt::DMat* d_dmat = static_cast<rt::DMat*>(mem);
     char* base = static_cast<char*>(mem) + nd * sizeof(rt::DMat);
     double* d_grad = reinterpret_cast<double*>(base);
@@ -2219,7 +2316,6 @@ int rt_adjoint(RtScene* sc, const RtRenderParams* p, const float* dimg, const ui
     float ms = 0.0f;
     if (rc == RT_OK && !wavefront) cudaEventElapsedTime(&ms, sc->ev0, sc->ev1);
     if (wavefront) ms = (float)wf_ms;
-    cudaFree(mem);
     if (rc != RT_OK) return rc;
     for (int i = 0; i < np; i++) grad[i] = (float)hg[(size_t)i];
     if (st) {
@@ -2355,14 +2451,17 @@ int rt_tonemap(const float* hdr, int32_t width, int32_t height, float exposure_e
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(RT_ERR_NO_DEVICE, "no CUDA device");
     size_t n = (size_t)width * height, b = n * 3 * sizeof(float);
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
     float* d = nullptr;
     if (cudaMalloc(&d, 2 * b) != cudaSuccess) return fail(RT_ERR_OOM, "allocation failed");
     int rc = RT_OK;
-    if (cudaMemcpy(d, hdr, b, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (copy_to_device(dev, cudaStreamPerThread, d, hdr, b) != cudaSuccess) {
         rc = fail(RT_ERR_CUDA, "copy failed");
     } else {
-        k_tonemap<<<(unsigned)((n + 255) / 256), 256>>>(d, (int)n, powf(2.0f, exposure_ev), d + n * 3);
-        if (cudaGetLastError() != cudaSuccess || cudaMemcpy(rgb, d + n * 3, b, cudaMemcpyDeviceToHost) != cudaSuccess)
+        k_tonemap<<<(unsigned)((n + 255) / 256), 256, 0, cudaStreamPerThread>>>(d, (int)n, powf(2.0f, exposure_ev),
+                                                                                d + n * 3);
+        if (cudaGetLastError() != cudaSuccess || copy_to_host(dev, cudaStreamPerThread, rgb, d + n * 3, b) != cudaSuccess)
             rc = fail(RT_ERR_CUDA, "tonemap failed");
     }
     cudaFree(d);
