@@ -1066,7 +1066,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     // iteration starts at least half as many paths as there are free slots.
     int64_t limit = 2 * (total / nslots + 2) * (int64_t)(max_depth + 2) + 64;
     if (cfg.iter_limit > 0) limit = std::min<int64_t>(limit, cfg.iter_limit);
-    const bool one = reqs.size() == 1;
+    const bool one = reqs.size() == 1, one_scene = views.size() == 1;   // what is in constant memory
     rt::WfCtl ctl0{};
     ctl0.total = (unsigned long long)total;
     ctl0.limit = (int)std::min<int64_t>(limit, INT32_MAX);
@@ -1078,7 +1078,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     std::memcpy(ws.pinned + off_films, films.data(), films.size() * sizeof(float*));
     std::memcpy(ws.pinned + off_fdims, fdims.data(), fdims.size() * sizeof(int));
     CUDA_TRY(cudaMemcpyAsync(ws.mem, ws.pinned, table_bytes, cudaMemcpyHostToDevice, stream));
-    if (one) {
+    if (one_scene) {
         rt::WfOne c{views[0], wreq[0].rc};
         std::memcpy(ws.pinned + off_one, &c, sizeof(c));
         CUDA_TRY(cudaMemcpyToSymbolAsync(rt::c_wf_one, ws.pinned + off_one, sizeof(c), 0, cudaMemcpyHostToDevice, stream));
@@ -1148,11 +1148,21 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     // the camera kernel: persistent warps, as many as are resident
     void (*camera)(const rt::WfArgs) =
         mode == rt::WF_RECORD ? rt::k_wf_camera<kStack, rt::WF_RECORD, true>
-                              : (one ? rt::k_wf_camera<kStack, rt::WF_RENDER, true> : rt::k_wf_camera<kStack, rt::WF_RENDER, false>);
+                              : (one_scene ? rt::k_wf_camera<kStack, rt::WF_RENDER, true> : rt::k_wf_camera<kStack, rt::WF_RENDER, false>);
     int cam_sms = 148, cam_blocks = 1;
     cudaDeviceGetAttribute(&cam_sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cam_blocks, camera, 128, 0);
     unsigned gcam = (unsigned)std::min<int64_t>((int64_t)std::max(1, cam_blocks) * cam_sms, (nslots + 127) / 128);
+    void (*extend)(const rt::WfArgs) =
+        one_scene ? (l4 ? rt::k_wf_extend<kStack, true, true> : rt::k_wf_extend<kStack, false, true>)
+                  : (l4 ? rt::k_wf_extend<kStack, true, false> : rt::k_wf_extend<kStack, false, false>);
+    const bool occ4 = a.opaque ? l4_occ : l4;
+    void (*occlude)(const rt::WfArgs) =
+        one_scene
+            ? (a.opaque ? (occ4 ? rt::k_wf_occlude<kStack, true, true, true> : rt::k_wf_occlude<kStack, false, true, true>)
+                        : (occ4 ? rt::k_wf_occlude<kStack, true, false, true> : rt::k_wf_occlude<kStack, false, false, true>))
+            : (a.opaque ? (occ4 ? rt::k_wf_occlude<kStack, true, true, false> : rt::k_wf_occlude<kStack, false, true, false>)
+                        : (occ4 ? rt::k_wf_occlude<kStack, true, false, false> : rt::k_wf_occlude<kStack, false, false, false>));
     void (*shade)(const rt::WfArgs) =
         one ? (medium ? (transmit ? rt::k_wf_shade<true, true, true> : rt::k_wf_shade<true, false, true>)
                       : (transmit ? rt::k_wf_shade<false, true, true> : rt::k_wf_shade<false, false, true>))
@@ -1168,9 +1178,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         else rt::k_wf_regen<rt::WF_RENDER><<<g256, 256, 0, stream>>>(a);
         if (mode != rt::WF_REPLAY) camera<<<gcam, 128, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[1], stream);
-        if (l4) rt::k_wf_extend<kStack, true><<<gst, tblk, 0, stream>>>(a);
-        else if (pt) rt::k_wf_extend_pt<kStack><<<gpt_e, tblk, 0, stream>>>(a);
-        else rt::k_wf_extend<kStack, false><<<gst, tblk, 0, stream>>>(a);
+        if (pt) rt::k_wf_extend_pt<kStack><<<gpt_e, tblk, 0, stream>>>(a);
+        else extend<<<gst, tblk, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[2], stream);
         if (sort) rt::k_wf_scatter<<<g256, 256, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[3], stream);
@@ -1187,11 +1196,8 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         if (a.shadowsort) rt::k_wf_sscatter<<<gsh256, 256, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[5], stream);
         if (mode != rt::WF_REPLAY) {
-            if (l4_occ && a.opaque) rt::k_wf_occlude<kStack, true, true><<<gsh, tblk, 0, stream>>>(a);
-            else if (l4) rt::k_wf_occlude<kStack, true, false><<<gsh, tblk, 0, stream>>>(a);
-            else if (pt && a.opaque) rt::k_wf_occlude_pt<kStack><<<gpt_o, tblk, 0, stream>>>(a);
-            else if (a.opaque) rt::k_wf_occlude<kStack, false, true><<<gsh, tblk, 0, stream>>>(a);
-            else rt::k_wf_occlude<kStack, false, false><<<gsh, tblk, 0, stream>>>(a);
+            if (pt && a.opaque) rt::k_wf_occlude_pt<kStack><<<gpt_o, tblk, 0, stream>>>(a);
+            else occlude<<<gsh, tblk, 0, stream>>>(a);
         }
         if (ev) cudaEventRecord(ev[6], stream);
     };
@@ -1205,7 +1211,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         // alone (everything else it reads lives in the workspace), so those
         // bytes key the cached ones.
         const unsigned shape[] = {(unsigned)blk, (unsigned)tblk, (unsigned)l4, (unsigned)l4_occ, (unsigned)pt,
-                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, gpt_e, gpt_o, gs, gst,
+                                  (unsigned)medium, (unsigned)transmit, (unsigned)one, (unsigned)one_scene, gpt_e, gpt_o, gs, gst,
                                   (unsigned)max_shadow, g256, gcam, gplan, (unsigned)mode, gadj, (unsigned)adj_blk, (unsigned)adj_shmem};
         std::vector<unsigned char> key(sizeof(a) + sizeof(shape));
         std::memcpy(key.data(), &a, sizeof(a));

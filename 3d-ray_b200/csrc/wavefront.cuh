@@ -177,11 +177,15 @@ struct WfArgs {
     const WfAdjoint* J;   // the adjoint passes' buffers and parameters (null in WF_RENDER)
 };
 
-// The scene and constants of a batch of one request, in constant memory: the
-// kernels' ONE variants read them as instruction operands instead of through
-// two dependent loads (request, then scene view) per thread. wf_render, which
-// holds a process-wide lock until its kernels are done, writes them on the
-// stream before the first iteration.
+// The scene of a call with one scene, and the constants of one with one
+// request, in constant memory: the kernels' ONE variants read them as
+// instruction operands instead of through two dependent loads (request, then
+// scene view) per thread. wf_render, which holds a process-wide lock until its
+// kernels are done, writes them on the stream before the first iteration. Shade
+// takes them for one request alone (with the view constant and the request's
+// constants in global memory it lost 2% on a Cornell box); extend and occlude
+// for one scene (extend 1.29 to 1.23 ms, occlude 0.78 to 0.73 ms on a Cornell
+// box of 256x256x64 samples).
 struct WfOne {
     SceneView view;
     RenderConst rc;
@@ -610,7 +614,7 @@ RT_D void extend_store(const WfArgs& a, int i, int flags, int req, const SceneVi
 // The register budget of 5 blocks of 256 (48 registers) lets 10 blocks of the
 // autotuned 128 threads share an SM instead of 9: extend -2.5% per 64-spp
 // icosphere frame, for an 8-byte spill.
-template <int STACK, bool L4>
+template <int STACK, bool L4, bool ONE>
 __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ WfArgs a) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.raysort) {
@@ -643,8 +647,8 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ Wf
     int flags = fbits(d.w);
     if (!(flags & PF_ALIVE) || (flags & PF_TRACED)) return;
     float4 o = a.P.o[i];
-    int req = a.nreq == 1 ? 0 : RT_IX(a.P.id[i].z, a.nreq);
-    const SceneView& s = a.views[RT_IX(a.reqs[req].scene, a.nviews)];
+    int req = ONE && a.nreq == 1 ? 0 : RT_IX(a.P.id[i].z, a.nreq);
+    const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(a.reqs[req].scene, a.nviews)];
     Hit h;
     trace<false, STACK, L4>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps, kInf, h, nullptr, a.err);
     extend_store(a, i, flags, req, s, h);
@@ -759,9 +763,9 @@ __global__ void __launch_bounds__(128, RT_CAMERA_MIN_BLOCKS) k_wf_camera(const _
         Hit h;
         h.kind = HIT_NONE;
         if (lane < n && id < total) {
-            if (!ONE) req = RT_IX(find_request(a.reqs, a.nreq, id), a.nreq);
+            req = RT_IX(find_request(a.reqs, a.nreq, id), a.nreq);
             const WfRequest& R = a.reqs[req];
-            const RenderConst& rc = ONE ? c_wf_one.rc : R.rc;
+            const RenderConst& rc = R.rc;
             const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(R.scene, a.nviews)];
             long long local = (long long)(id - (unsigned long long)R.begin);
             long long npix = (long long)R.ww * R.wh;
@@ -1136,7 +1140,7 @@ __global__ void __launch_bounds__(256) k_wf_occlude_pt(const __grid_constant__ W
 // 10 blocks of the autotuned 128 threads per SM instead of 8, occlude -7.8%
 // per 64-spp icosphere frame. The transparent variant keeps the full budget
 // its longer walk needs.
-template <int STACK, bool L4, bool OPAQUE>
+template <int STACK, bool L4, bool OPAQUE, bool ONE>
 __global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid_constant__ WfArgs a) {
     int j;
     if (a.shadowsort) {   // a flat grid over the sorted order
@@ -1161,7 +1165,7 @@ __global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid
         }
     }
     float4 o = a.S.o[j], d = a.S.d[j], c = a.S.c[j];
-    const SceneView& s = a.views[RT_IX(fbits(c.w), a.nviews)];
+    const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(fbits(c.w), a.nviews)];
     V3 tr = shadow_transmittance<STACK, L4>(s, OPAQUE ? 1 : a.opaque, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps,
                                             o.w, nullptr, a.err);
     if (near_zero(tr)) return;
