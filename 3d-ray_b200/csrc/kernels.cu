@@ -1168,20 +1168,23 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
                       : (transmit ? rt::k_wf_shade<false, true, true> : rt::k_wf_shade<false, false, true>))
             : (medium ? (transmit ? rt::k_wf_shade<true, true, false> : rt::k_wf_shade<true, false, false>)
                       : (transmit ? rt::k_wf_shade<false, true, false> : rt::k_wf_shade<false, false, false>));
-    // the plan's blocks: the bookkeeping, the bounce rays' scan, the shadow records' scan
-    const unsigned gplan = a.shadowsort ? 3 : (a.raysort ? 2 : 1);
+    // the plan's clusters: the bookkeeping with the bounce rays' scan, the shadow records' scan
+    const unsigned gplan = rt::kPlanCluster * (a.shadowsort ? 2 : 1);
+    void (*regen)(const rt::WfArgs) = mode == rt::WF_RECORD   ? rt::k_wf_regen<rt::WF_RECORD>
+                                      : mode == rt::WF_REPLAY ? rt::k_wf_regen<rt::WF_REPLAY>
+                                                              : rt::k_wf_regen<rt::WF_RENDER>;
+    const unsigned grg = (unsigned)((nslots + rt::kRegenBlock - 1) / rt::kRegenBlock);
+    const unsigned gsort = (unsigned)((nslots + rt::kSortChunk - 1) / rt::kSortChunk) * rt::kSortCluster;
     // ev (profiling only): boundaries between the kernel groups of one iteration.
     auto launch_iter = [&](cudaEvent_t* ev, cudaGraphConditionalHandle loop) {
         if (ev) cudaEventRecord(ev[0], stream);
-        if (mode == rt::WF_RECORD) rt::k_wf_regen<rt::WF_RECORD><<<g256, 256, 0, stream>>>(a);
-        else if (mode == rt::WF_REPLAY) rt::k_wf_regen<rt::WF_REPLAY><<<g256, 256, 0, stream>>>(a);
-        else rt::k_wf_regen<rt::WF_RENDER><<<g256, 256, 0, stream>>>(a);
+        regen<<<grg, rt::kRegenBlock, 0, stream>>>(a);
         if (mode != rt::WF_REPLAY) camera<<<gcam, 128, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[1], stream);
         if (pt) rt::k_wf_extend_pt<kStack><<<gpt_e, tblk, 0, stream>>>(a);
         else extend<<<gst, tblk, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[2], stream);
-        if (sort) rt::k_wf_scatter<<<g256, 256, 0, stream>>>(a);
+        if (sort) rt::k_wf_scatter<<<gsort, rt::kSortThreads, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[3], stream);
         if (mode == rt::WF_REPLAY) {   // the adjoint vertex, shadow rays inline: no occlude
             if (medium && transmit) rt::k_wf_adjoint<kStack, true, true><<<gadj, adj_blk, adj_shmem, stream>>>(a);

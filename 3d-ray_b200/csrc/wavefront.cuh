@@ -29,6 +29,8 @@
 // with the replay's gradient hooks and its shadow rays inline.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 #include "adjoint.cuh"
@@ -103,6 +105,7 @@ struct WfCtl {
     unsigned long long iter_first;   // replay: the first work id of this iteration
     int live;                   // slots alive after the last regen and camera
     int nlive;                  // live slots in order[] (the material sort's total)
+    int shaded;                 // nlive of the iteration's shade, for occlude
     int err;                    // a kernel's RT_ERR_* (traversal stack, index checks)
     int overflow;               // shadow queue overflow (its arrays hold every record: a test's limit)
     int iters, limit;           // iterations run, and the host's bound on them
@@ -113,8 +116,6 @@ struct WfCtl {
     int nshadow;                // shadow sort: records counted by key
     int nfree, free_next;       // slots in the free list, and the first one not yet reserved
     int nrec;                   // records written this iteration (counted under a test's limit alone)
-    int hist[256];              // material histogram (sorting)
-    int cursor[256];            // live slots placed so far, per material
 };
 
 // Buckets of the bounce-ray sort.
@@ -361,13 +362,16 @@ RT_D void film_add(const WfRequest& R, int lx, int ly, V3 L) {
     atomicAdd(R.accum + 2 * plane + k, (double)L.z);
 }
 
+// Threads of a regen block: one atomic per counter and block, on addresses that
+// every block shares.
+constexpr int kRegenBlock = 512;
 template <int MODE>
-__global__ void __launch_bounds__(256) k_wf_regen(const __grid_constant__ WfArgs a) {
+__global__ void __launch_bounds__(kRegenBlock) k_wf_regen(const __grid_constant__ WfArgs a) {
     // The free slots go to the free list, or in the replay to the next work ids,
     // with one atomic per block (a ballot prefix over the block's free slots),
     // and the live count with one more: a per-warp atomic on one address
     // serialised in L2.
-    __shared__ int s_warp[8];   // blockDim 256: per-warp free-slot offsets
+    __shared__ int s_warp[kRegenBlock / 32];   // per-warp free-slot offsets
     __shared__ unsigned long long s_base;
     __shared__ int s_live;
     const unsigned full = 0xffffffffu;
@@ -586,16 +590,13 @@ RT_D int ray_key(const SceneView& s, V3 o, V3 d, int cb, int db) {
 RT_D void hit_store(const WfArgs& a, int i, int req, const SceneView& s, const Hit& h) {
     int packed = h.kind == HIT_NONE ? 0 : ((h.kind << 30) | h.slot);
     a.P.hit[i] = make_float4(h.t, h.u, h.v, ibits(packed));
-    if (a.sort) {   // material key for the counting sort
+    if (a.sort) {   // material key for the scatter
         int key = a.nkeys;   // misses and emitters sort last
         if (h.kind != HIT_NONE) {
             int ent = h.kind == HIT_TRI ? s.tri_entity[RT_IX(h.slot, s.n_tris)] : h.slot;
             key = RT_IX(a.key_base[a.reqs[req].scene] + s.entities[RT_IX(ent, s.n_entities)].material, a.nkeys);
         }
         a.P.keys[i] = key;
-        // one atomic per distinct key in the warp (__match_any_sync groups lanes)
-        unsigned grp = __match_any_sync(__activemask(), key);
-        if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&a.ctl->hist[key], __popc(grp));
     }
 }
 
@@ -847,27 +848,60 @@ RT_D int block_scan(int v, int* s_w, int* total) {
     return (w ? s_w[w - 1] : 0) + incl - v;
 }
 
-// Counting sort of the live slots by material. Every block scans the histogram
-// itself (at most 256 keys), so the sort is one launch.
-__global__ void __launch_bounds__(256) k_wf_scatter(const __grid_constant__ WfArgs a) {
-    __shared__ int s_w[32], s_off[256];
-    int v = (int)threadIdx.x <= a.nkeys ? a.ctl->hist[threadIdx.x] : 0;
-    int live;
-    s_off[threadIdx.x] = block_scan(v, s_w, &live);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->nlive = live;
+// Sorts the live slots by material, chunk by chunk: a cluster of blocks orders
+// its run of kSortChunk slots through shared memory and appends it to order[]
+// with one atomic. Shade wants warps of one material, not one global order: a
+// material's run in a chunk is long enough for that, and there is no global
+// histogram, whose few hot counters took an atomic per warp and material in
+// extend, in camera and twice here. (Chunks of 8192 slots, one block's: shade
+// 27.1 to 30.4 ms on the full-HD icosphere frame with its 65 materials.)
+constexpr int kSortThreads = 1024, kSortPer = 8, kSortCluster = 8;
+constexpr int kSortChunk = kSortThreads * kSortPer * kSortCluster;
+__global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThreads)
+    k_wf_scatter(const __grid_constant__ WfArgs a) {
+    __shared__ int s_w[32], s_cnt[256], s_all[kSortCluster][256], s_base;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank();
+    const int tid = threadIdx.x, first = blockIdx.x * (kSortThreads * kSortPer) + tid;
+    if (tid < 256) s_cnt[tid] = 0;
     __syncthreads();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.nslots) return;
-    if (!(fbits(a.P.d[i].w) & PF_ALIVE)) return;
-    int key = RT_IX(a.P.keys[i], a.nkeys + 1);
-    unsigned grp = __match_any_sync(__activemask(), key);
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(grp) - 1;
-    int rank = __popc(grp & ((1u << lane) - 1u));
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&a.ctl->cursor[key], __popc(grp));
-    base = __shfl_sync(grp, base, leader) + s_off[key];
-    a.P.order[RT_IX(base + rank, a.nslots)] = i;
+    int key[kSortPer], pos[kSortPer];
+#pragma unroll
+    for (int k = 0; k < kSortPer; k++) {
+        int i = first + k * kSortThreads;
+        key[k] = i < a.nslots && (fbits(a.P.d[i].w) & PF_ALIVE) ? RT_IX(a.P.keys[i], a.nkeys + 1) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kSortPer; k++) {
+        // one shared-memory atomic per distinct key of the warp
+        unsigned grp = __match_any_sync(0xffffffffu, key[k]);
+        int lane = tid & 31, leader = __ffs(grp) - 1, base = 0;
+        if (key[k] >= 0 && lane == leader) base = atomicAdd(&s_cnt[key[k]], __popc(grp));
+        pos[k] = __shfl_sync(0xffffffffu, base, leader) + __popc(grp & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    // every block gets every block's counts: a key's slots of the earlier blocks go first
+    if (tid < 256)
+        for (int q = 0; q < kSortCluster; q++) cluster.map_shared_rank(&s_all[0][0], q)[rank * 256 + tid] = s_cnt[tid];
+    cluster.sync();
+    int sum = 0, before = 0, live;
+    if (tid < 256)
+        for (int q = 0; q < kSortCluster; q++) {
+            int c = s_all[q][tid];
+            if (q < (int)rank) before += c;
+            sum += c;
+        }
+    int off = block_scan(sum, s_w, &live);
+    if (tid < 256) s_cnt[tid] = off + before;
+    if (rank == 0 && tid == 0) {
+        int b = live ? atomicAdd(&a.ctl->nlive, live) : 0;
+        for (int q = 0; q < kSortCluster; q++) *cluster.map_shared_rank(&s_base, q) = b;
+    }
+    cluster.sync();
+#pragma unroll
+    for (int k = 0; k < kSortPer; k++)
+        if (key[k] >= 0) a.P.order[RT_IX(s_base + s_cnt[key[k]] + pos[k], a.nslots)] = first + k * kSortThreads;
 }
 
 // Shadow sink of the wavefront: queue the ray with its contribution.
@@ -1007,72 +1041,70 @@ __global__ void __launch_bounds__(kShadeBlock, 1) k_wf_shade(const __grid_consta
     if (a.raysort) wf_rank_ray(a, s, ps.o, ps.d, i);
 }
 
-// Exclusive scan of a ray-sort key histogram (kRayKeys counts) into off (one
-// block of 1024 threads, a run of kRayKeys / 1024 keys each), clearing the
-// histogram for the next shade; *total receives the sum.
+// Exclusive scan of a ray-sort key histogram (kRayKeys counts) into off by one
+// cluster of kPlanCluster blocks of 1024 threads, four neighbouring keys a
+// thread, clearing the histogram for the next shade; *total receives the sum.
+// Blocks exchange their sums through distributed shared memory. (One block
+// whose threads each read a run of 32 keys took about 10 us longer.)
+constexpr int kPlanCluster = 8;
 RT_D void key_scan(int* hist, int* off, int* total) {
-    constexpr int kPer = kRayKeys / 1024;
-    static_assert(kPer % 4 == 0, "whole int4 runs per thread");
-    __shared__ int s_w[32];
-    int4* h4 = reinterpret_cast<int4*>(hist) + threadIdx.x * (kPer / 4);
-    int4* o4 = reinterpret_cast<int4*>(off) + threadIdx.x * (kPer / 4);
-    int4 v[kPer / 4];
-    int sum = 0, all;
+    static_assert(kRayKeys == kPlanCluster * 1024 * 4, "four keys a thread");
+    __shared__ int s_w[32], s_sum[kPlanCluster];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank();
+    const int at = (int)rank * 1024 + threadIdx.x;
+    int4 v = reinterpret_cast<int4*>(hist)[at];
+    reinterpret_cast<int4*>(hist)[at] = make_int4(0, 0, 0, 0);
+    int sum;
+    int base = block_scan(v.x + v.y + v.z + v.w, s_w, &sum);
+    if (threadIdx.x < kPlanCluster) *cluster.map_shared_rank(&s_sum[rank], threadIdx.x) = sum;
+    cluster.sync();
+    int all = 0;
 #pragma unroll
-    for (int k = 0; k < kPer / 4; k++) {
-        v[k] = h4[k];
-        sum += v[k].x + v[k].y + v[k].z + v[k].w;
+    for (unsigned k = 0; k < kPlanCluster; k++) {
+        if (k < rank) base += s_sum[k];
+        all += s_sum[k];
     }
-    int base = block_scan(sum, s_w, &all);
-#pragma unroll
-    for (int k = 0; k < kPer / 4; k++) {
-        int4 r;
-        r.x = base;
-        r.y = r.x + v[k].x;
-        r.z = r.y + v[k].y;
-        r.w = r.z + v[k].z;
-        base = r.w + v[k].w;
-        o4[k] = r;
-        h4[k] = make_int4(0, 0, 0, 0);
-    }
-    if (threadIdx.x == 0) *total = all;
+    int4 r;
+    r.x = base;
+    r.y = r.x + v.x;
+    r.z = r.y + v.y;
+    r.w = r.z + v.z;
+    reinterpret_cast<int4*>(off)[at] = r;
+    if (rank == 0 && threadIdx.x == 0) *total = all;
 }
 
-// Between shade and occlude, one launch of up to three blocks: block 0 ends the
-// iteration's bookkeeping (whether the loop goes on, and the counters that the
-// next iteration accumulates; occlude reads none of them), block 1 scans the
-// bounce rays' keys, block 2 the shadow records'. loop: the graph's loop
-// condition, 0 when the host runs the iterations itself.
-__global__ void __launch_bounds__(1024) k_wf_plan(const __grid_constant__ WfArgs a, cudaGraphConditionalHandle loop) {
+// Between shade and occlude, one launch: block 0 ends the iteration's
+// bookkeeping (whether the loop goes on, and the counters that the next
+// iteration accumulates; occlude reads none of them), the first cluster scans
+// the bounce rays' keys and the second the shadow records'. loop: the graph's
+// loop condition, 0 when the host runs the iterations itself.
+__global__ void __cluster_dims__(kPlanCluster, 1, 1) __launch_bounds__(1024)
+    k_wf_plan(const __grid_constant__ WfArgs a, cudaGraphConditionalHandle loop) {
     WfCtl* c = a.ctl;
-    if (blockIdx.x == 1) {
-        key_scan(a.rhist, a.roff, &c->nbounce);
-    } else if (blockIdx.x == 2) {
-        key_scan(a.shist, a.soff, &c->nshadow);
-    } else {
-        if (threadIdx.x == 0) {
-            c->iters++;
-            c->done = c->next >= c->total && c->live == 0;
-            if (loop && (c->done || c->overflow || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
-            c->iter_first = c->next;
-            c->live = 0;
-            c->ext_next = 0;
-            c->occ_next = 0;
-            c->nfree = 0;
-            c->free_next = 0;
-            c->nrec = 0;
-        }
-        if (threadIdx.x < 256) {
-            c->hist[threadIdx.x] = 0;
-            c->cursor[threadIdx.x] = 0;
-        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        c->iters++;
+        c->done = c->next >= c->total && c->live == 0;
+        if (loop && (c->done || c->overflow || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
+        c->iter_first = c->next;
+        c->live = 0;
+        c->ext_next = 0;
+        c->occ_next = 0;
+        c->nfree = 0;
+        c->free_next = 0;
+        c->nrec = 0;
+        c->shaded = c->nlive;
+        c->nlive = 0;
     }
+    if (blockIdx.x >= kPlanCluster) key_scan(a.shist, a.soff, &c->nshadow);
+    else if (a.raysort) key_scan(a.rhist, a.roff, &c->nbounce);
 }
 
 // The record that thread t of shade wrote k-th, or -1. Under the material sort
 // shade ran the threads below the live count alone.
 RT_D int shadow_record(const WfArgs& a, int t, int k) {
-    int live = a.sort ? a.ctl->nlive : a.nslots;
+    int live = a.sort ? a.ctl->shaded : a.nslots;
     if (t >= live || k >= a.S.cnt[RT_IX(t, a.nslots)]) return -1;
     return k * a.nslots + t;
 }
