@@ -41,13 +41,6 @@ RT_D long long checked_index(long long i, long long n) {
 // ---------------------------------------------------------------------------
 // Owen-scrambled Sobol (Core/Sampling/OwenSobol.cs:48-210)
 // ---------------------------------------------------------------------------
-__constant__ uint32_t c_dim1_dirs[32] = {
-    0x80000000u, 0xc0000000u, 0xa0000000u, 0xf0000000u, 0x88000000u, 0xcc000000u, 0xaa000000u, 0xff000000u,
-    0x80800000u, 0xc0c00000u, 0xa0a00000u, 0xf0f00000u, 0x88880000u, 0xcccc0000u, 0xaaaa0000u, 0xffff0000u,
-    0x80008000u, 0xc000c000u, 0xa000a000u, 0xf000f000u, 0x88008800u, 0xcc00cc00u, 0xaa00aa00u, 0xff00ff00u,
-    0x80808080u, 0xc0c0c0c0u, 0xa0a0a0a0u, 0xf0f0f0f0u, 0x88888888u, 0xccccccccu, 0xaaaaaaaau, 0xffffffffu,
-};
-
 RT_D uint32_t hash_u32(uint32_t x) {
     x ^= x >> 16;
     x *= 0x7feb352du;
@@ -66,15 +59,21 @@ RT_D uint32_t lk_permute(uint32_t v, uint32_t seed) {
 }
 RT_D uint32_t owen_scramble(uint32_t v, uint32_t seed) { return __brev(lk_permute(__brev(v), seed)); }
 
-// Dimensions 0 and 1, which only the camera jitter draws: out of line, so that
-// every other draw site carries the padded-dimension code alone.
-__device__ __noinline__ uint32_t sobol_dim01(uint32_t index, uint32_t dim) {
-    if (dim == 0u) return __brev(index);
-    uint32_t v = 0u, i = index;
-#pragma unroll 1
-    for (int k = 0; i != 0u; k++, i >>= 1)
-        if (i & 1u) v ^= c_dim1_dirs[k];
-    return v;
+// Dimensions 0 and 1, which only the camera jitter draws. The direction
+// numbers of dimension 1 are the rows of Pascal's triangle mod 2: bit j of row
+// k (from the top) is set when j's bits are a subset of k's (Lucas' theorem).
+// The xor of the index's rows is therefore a superset sum over its bits, five
+// shift-and-mask steps, and then the bits reversed.
+RT_D uint32_t sobol_dim01(uint32_t index, uint32_t dim) {
+    uint32_t x = index;
+    if (dim != 0u) {
+        x ^= (x >> 1) & 0x55555555u;
+        x ^= (x >> 2) & 0x33333333u;
+        x ^= (x >> 4) & 0x0f0f0f0fu;
+        x ^= (x >> 8) & 0x00ff00ffu;
+        x ^= (x >> 16) & 0x0000ffffu;
+    }
+    return __brev(x);
 }
 
 RT_D float sobol_sample(uint32_t index, uint32_t dim, uint32_t pixel_seed) {

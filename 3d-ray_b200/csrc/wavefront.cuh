@@ -251,6 +251,18 @@ RT_D void strip_pixel(int p, int ww, int wh, int& lx, int& ly) {
     lx = kStripW * strip + in % sw;
     ly = in / sw;
 }
+// A request's local work id as (sample, pixel in strip order): samples outermost.
+// 32-bit division where the request's ids fit.
+RT_D void split_id(unsigned long long local, int npix, int& s, int& p) {
+    if (local >> 32) {
+        s = (int)(local / (unsigned)npix);
+        p = (int)(local % (unsigned)npix);
+    } else {
+        unsigned q = (unsigned)local / (unsigned)npix;
+        s = (int)q;
+        p = (int)((unsigned)local - q * (unsigned)npix);
+    }
+}
 RT_D int strip_index(int lx, int ly, int ww, int wh) {
     int strip = lx / kStripW;
     int sw = min(kStripW, ww - kStripW * strip);
@@ -449,11 +461,8 @@ __global__ void __launch_bounds__(kRegenBlock) k_wf_regen(const __grid_constant_
         } else {
             int req = RT_IX(find_request(a.reqs, a.nreq, id), a.nreq);
             const WfRequest& R = a.reqs[req];
-            long long local = (long long)(id - (unsigned long long)R.begin);
-            long long npix = (long long)R.ww * R.wh;
-            int s = (int)(local / npix);
-            int p = (int)(local % npix);
-            int lx, ly;
+            int lx, ly, s, p;
+            split_id(id - (unsigned long long)R.begin, R.ww * R.wh, s, p);
             strip_pixel(p, R.ww, R.wh, lx, ly);
             PathState ps;
             path_init(ps, R.rc, R.x0 + lx, R.y0 + ly, (uint32_t)(R.spp0 + s));
@@ -768,12 +777,11 @@ __global__ void __launch_bounds__(128, RT_CAMERA_MIN_BLOCKS) k_wf_camera(const _
             const WfRequest& R = a.reqs[req];
             const RenderConst& rc = R.rc;
             const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(R.scene, a.nviews)];
-            long long local = (long long)(id - (unsigned long long)R.begin);
-            long long npix = (long long)R.ww * R.wh;
-            int lx, ly;
-            strip_pixel((int)(local % npix), R.ww, R.wh, lx, ly);
+            int lx, ly, si, p;
+            split_id(id - (unsigned long long)R.begin, R.ww * R.wh, si, p);
+            strip_pixel(p, R.ww, R.wh, lx, ly);
             PathState ps;
-            path_init(ps, rc, R.x0 + lx, R.y0 + ly, (uint32_t)(R.spp0 + (int)(local / npix)));
+            path_init(ps, rc, R.x0 + lx, R.y0 + ly, (uint32_t)(R.spp0 + si));
             pix = lx | (ly << 16);
             seed = (int)ps.rng.seed;
             sample = (int)ps.rng.index;
