@@ -1351,9 +1351,10 @@ RT_D float sphere_cone_pdf(V3 center, float radius, V3 p, V3 wi) {
 
 // The sphere and sky samplers of light_sample, out of line: most scenes have
 // none of these lights, and the shade kernel is bound by instruction fetch.
-__device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, const Light& l, V3 p, V3 sn, int si,
-                                                         Sampler& rng) {
-    LightSample r;
+// The caller hands in copies of its sampler and sample: the address of a
+// variable passed to a call keeps it in local memory for its whole life.
+__device__ __noinline__ void light_sample_sphere_env(const SceneView& s, const Light& l, V3 p, V3 sn, int si,
+                                                     Sampler& rng, LightSample& r) {
     r.occluded = 0;
     r.has_ray = 0;
     r.color = v3(0.0f);
@@ -1397,28 +1398,28 @@ __device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, 
         if (pdf <= 0.0f) {
             r.occluded = 1;
             r.dir = v3(0.0f, 1.0f, 0.0f);
-            return r;
+            return;
         }
         V3 tl = sp - p;
         float d2 = length_sq(tl);
         if (d2 < kEps * kEps) {
             r.occluded = 1;
             r.dir = v3(0.0f, 1.0f, 0.0f);
-            return r;
+            return;
         }
         float dist = sqrtf(d2);
         V3 dir = tl / dist;
         r.dir = dir;
         r.dist = dist;
         float cl = fmaxf(0.0f, dot(-dir, ln));
-        if (cl <= 0.0f) return r;   // not in shadow, zero colour
+        if (cl <= 0.0f) return;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
         r.ray_o = so;
         r.ray_tmax = length(sp - so) - kEps;
         float atten = 1.0f / (pdf * (float)l.shadow_samples);
         r.color = l.emission * atten;
-        return r;
+        return;
     }
     if (l.type == LIGHT_SPHERE) {   // SphereLight.IlluminateAndTestStratified (:72-141)
         V3 tc = l.center - p;
@@ -1426,7 +1427,7 @@ __device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, 
         if (d2c < kEps * kEps) {
             r.occluded = 1;
             r.dir = v3(0.0f, 1.0f, 0.0f);
-            return r;
+            return;
         }
         float dc = sqrtf(d2c);
         V3 wd = tc / dc;
@@ -1444,20 +1445,20 @@ __device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, 
         if (disc < 0.0f) {
             r.occluded = 1;
             r.dist = length(l.center + normalize(dw) * l.radius - p);
-            return r;
+            return;
         }
         float sq = sqrtf(disc);
         float t = -b - sq;
         if (t < kEps) t = -b + sq;
         if (t < kEps) {
             r.occluded = 1;
-            return r;
+            return;
         }
         V3 sp = p + t * dw;
         r.dist = t;
         V3 ln = (sp - l.center) / l.radius;
         float cl = fmaxf(0.0f, dot(-dw, ln));
-        if (cl <= 0.0f) return r;   // not in shadow, zero colour
+        if (cl <= 0.0f) return;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
         r.ray_o = so;
@@ -1465,7 +1466,7 @@ __device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, 
         float sa = 2.0f * kPi * (1.0f - cmax);
         float atten = l.intensity * sa / (float)l.shadow_samples;
         r.color = l.color * atten;
-        return r;
+        return;
     }
     if (l.type == LIGHT_ENV) {   // EnvironmentLight.IlluminateAndTest (:54-90) over FlatSky.ImportanceSample
         V3 dir = random_unit_vector(rng);
@@ -1474,15 +1475,15 @@ __device__ __noinline__ LightSample light_sample_sphere_env(const SceneView& s, 
         r.dist = kInf;
         if (length_sq(sn) > 0.0f && dot(sn, dir) <= 0.0f) {   // below a surface's horizon
             r.occluded = 1;
-            return r;
+            return;
         }
         r.has_ray = 1;
         r.ray_o = offset_origin(p, sn);
         r.ray_tmax = kInf;
         r.color = l.color / (pdf * (float)l.shadow_samples);
-        return r;
+        return;
     }
-    return r;   // not reached: the caller passes only these three types
+    // not reached: the caller passes only these three types
 }
 
 // Draws the light sample (all RNG draws happen here, before any shadow test):
@@ -1567,8 +1568,20 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         r.color = l.emission * atten;
         return r;
     }
-    if (l.type == LIGHT_GEOM_SPHERE || l.type == LIGHT_SPHERE || l.type == LIGHT_ENV)
-        return light_sample_sphere_env(s, l, p, sn, si, rng);
+    if (l.type == LIGHT_GEOM_SPHERE || l.type == LIGHT_SPHERE || l.type == LIGHT_ENV) {
+        Sampler rc = rng;
+        LightSample t = r;
+        light_sample_sphere_env(s, l, p, sn, si, rc, t);
+        rng = rc;
+        r.occluded = t.occluded;
+        r.has_ray = t.has_ray;
+        r.color = t.color;
+        r.dir = t.dir;
+        r.dist = t.dist;
+        r.ray_o = t.ray_o;
+        r.ray_tmax = t.ray_tmax;
+        return r;
+    }
     if (l.type == LIGHT_AREA) {
         int su = si % l.sqrt_samples, sv = si / l.sqrt_samples;
         float ru = ((float)su + u1) * l.inv_sqrt;

@@ -139,6 +139,10 @@ struct PathState {
         if (!isfinite(x.z)) mask.z = 0.0f;
         la = la + v3(mask.x != 0.0f ? x.x : 0.0f, mask.y != 0.0f ? x.y : 0.0f, mask.z != 0.0f ? x.z : 0.0f);
     }
+    RT_D float ior_top() const { return iors.top(); }
+    RT_D float ior_enclosing() const { return iors.enclosing(); }
+    RT_D void ior_push(float v) { iors.push(v); }
+    RT_D void ior_pop() { iors.pop(); }
     // The first surface vertex: its weight and attenuation, for the primary clamp.
     RT_D void set_primary(V3 att) {
         pre = w;
@@ -334,7 +338,7 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
         view = normalize(-ps.d);
         if constexpr (TRANSMIT) {
             dielectric = !mp->thin_walled && mp->spec_trans_raw > 0.0f;
-            if (dielectric) rel_eta = rec.front ? (ps.iors.top() / mp->ior_raw) : (mp->ior_raw / ps.iors.enclosing());
+            if (dielectric) rel_eta = rec.front ? (ps.ior_top() / mp->ior_raw) : (mp->ior_raw / ps.ior_enclosing());
         }
         bv = bsdf_view(*mp, rec, view);
     }
@@ -492,8 +496,8 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
                 ps.cur_abs = bs.next_absorption;
                 sink.interior(near_zero(bs.next_absorption) ? -1 : rec.material);
             }
-            if (rc.dielectrics && bs.transition == 1) ps.iors.push(dielectric ? m.ior_raw : ps.iors.top());
-            if (rc.dielectrics && bs.transition == 2) ps.iors.pop();
+            if (rc.dielectrics && bs.transition == 1) ps.ior_push(dielectric ? m.ior_raw : ps.ior_top());
+            if (rc.dielectrics && bs.transition == 2) ps.ior_pop();
         }
     } else {
         sink.scatter(ps, m, rec, view, sdir, lobe, SCATTER_LEGACY, 1.0f, att_pre, att, bs.lobe, bs.tried);
@@ -502,8 +506,8 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
         ps.prev_delta = 0;
         if constexpr (TRANSMIT) {
             if (rc.dielectrics && dielectric && dot(sdir, rec.n) < 0.0f) {
-                if (rec.front) ps.iors.push(m.ior_raw);
-                else ps.iors.pop();
+                if (rec.front) ps.ior_push(m.ior_raw);
+                else ps.ior_pop();
             }
         }
     }

@@ -45,6 +45,7 @@ enum : int {
     PF_FIRST = 8,
     PF_CLAMP = 16,
     PF_DEAD = 32,       // 32, 64, 128: channels of la closed by the per-frame sanitize
+    PF_INSIDE = 512,    // the slot's interior state (ab, ior) is set: absorption or a non-empty IOR stack
     PF_TRACED = 256,    // a camera path of this iteration: its hit is in place, extend skips it
 };
 
@@ -303,8 +304,7 @@ RT_D void wf_load(const WfArgs& a, int i, const WfRequest& R, PathState& ps) {
     }
 }
 
-template <class PS>
-RT_D void wf_store_media(const WfArgs& a, int i, const PS& ps) {
+RT_D void wf_store_media(const WfArgs& a, int i, const PathState& ps) {
     a.P.ab[i] = make_float4(ps.cur_abs.x, ps.cur_abs.y, ps.cur_abs.z, ibits(ps.iors.n));
     for (int k = 0; k < 8; k++) a.P.ior[(size_t)i * 8 + k] = ps.iors.slot[k];
 }
@@ -324,9 +324,13 @@ __device__ __noinline__ void wf_add(float4* dst, float x, float y, float z) {
 // and the primary clamp's terms stay in their slot and are written where they
 // change: a whole PathState held 15 more registers through the vertex and
 // moved 128 B more per slot.
-struct LeanMedia {   // a batch with transmissive materials
+// A batch with transmissive materials: the interior absorption and the depth of
+// the IOR stack. The stack's entries stay in the slot (a dielectric surface
+// alone reads them), and outside every dielectric (PF_INSIDE clear) there is
+// nothing to load or store.
+struct LeanMedia {
     V3 cur_abs;
-    IorStackD iors;
+    int ior_n;
 };
 struct NoMedia {};
 template <bool TRANSMIT>
@@ -339,6 +343,21 @@ struct LeanPath : std::conditional_t<TRANSMIT, LeanMedia, NoMedia> {
     const WfArgs* a;
     int slot;
 
+    // Volumetrics/IorStack.cs (capacity 8), as IorStackD
+    RT_D float* ior_at(int k) const { return a->P.ior + (size_t)slot * 8 + k; }
+    RT_D float ior_top() const { return this->ior_n == 0 ? 1.0f : *ior_at(this->ior_n - 1); }
+    RT_D float ior_enclosing() const { return this->ior_n >= 2 ? *ior_at(this->ior_n - 2) : 1.0f; }
+    RT_D void ior_push(float v) {
+        if (this->ior_n >= 8) {
+            for (int k = 0; k < 7; k++) *ior_at(k) = *ior_at(k + 1);
+            *ior_at(7) = v;
+            return;
+        }
+        *ior_at(this->ior_n++) = v;
+    }
+    RT_D void ior_pop() {
+        if (this->ior_n > 0) this->ior_n--;
+    }
     RT_D void add(V3 x, int to_la) {   // PathState::add
         if (!to_la) {
             wf_add(a->P.lp + slot, x.x, x.y, x.z);
@@ -1027,25 +1046,28 @@ __global__ void __launch_bounds__(kShadeBlock, 1) k_wf_shade(const __grid_consta
     ps.rng = Sampler{(uint32_t)id.w, (uint32_t)id.x, (uint32_t)fbits(w.w)};
     if constexpr (TRANSMIT) {
         ps.cur_abs = v3(0.0f);
-        ps.iors.n = 0;
-        if (rc.dielectrics && !ps.first) {
+        ps.ior_n = 0;
+        if (flags & PF_INSIDE) {
             float4 ab = a.P.ab[i];
             ps.cur_abs = v3(ab.x, ab.y, ab.z);
-            ps.iors.n = fbits(ab.w);
-            for (int k = 0; k < 8; k++) ps.iors.slot[k] = a.P.ior[(size_t)i * 8 + k];
+            ps.ior_n = fbits(ab.w);
         }
     }
     QueueShadows sink{{}, &a, t, i, scene, 0};
     bool alive = shade_vertex<MEDIUM, TRANSMIT>(s, rc, ps, h, sink);
     a.S.cnt[t] = sink.n;
-    a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(wf_flags(ps, alive) | ps.dead));
+    int keep = wf_flags(ps, alive) | ps.dead;
+    if constexpr (TRANSMIT) {
+        if (alive && rc.dielectrics && (ps.ior_n > 0 || !is_zero(ps.cur_abs))) {
+            keep |= PF_INSIDE;
+            a.P.ab[i] = make_float4(ps.cur_abs.x, ps.cur_abs.y, ps.cur_abs.z, ibits(ps.ior_n));
+        }
+    }
+    a.P.d[i] = make_float4(ps.d.x, ps.d.y, ps.d.z, ibits(keep));
     if (!alive) return;   // resolve reads the flags and the radiance sums alone
     a.P.o[i] = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.prev_pdf);
     a.P.beta[i] = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, ibits(ps.depth));
     a.P.w[i] = make_float4(ps.w.x, ps.w.y, ps.w.z, ibits((int)ps.rng.dim));
-    if constexpr (TRANSMIT) {
-        if (rc.dielectrics) wf_store_media(a, i, ps);
-    }
     if (a.raysort) wf_rank_ray(a, s, ps.o, ps.d, i);
 }
 
