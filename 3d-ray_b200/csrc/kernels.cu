@@ -818,12 +818,12 @@ struct WfWorkspace {
 std::mutex g_wf_mu;
 WfWorkspace g_wf_ws[16];
 
-// Autotuned (wavefront size, block size, sort) per scene set, kept for the
-// process lifetime; filled by rt_autotune or the defaults below.
+// The wavefront's configuration: a scene's autotuned values (rt_autotune) or
+// the defaults below, overridden by a request's own.
 struct WfConfig {
     int slots = 1 << 22;
-    int block = 256;
-    int sort = 1;
+    int block = 128;   // block of extend/occlude when tblock is 0 (shade has its own: kShadeBlock)
+    int sort = -1;     // material sort: 1 on, 0 off, -1 by size (default_sort)
     int profile = 0;   // per-kernel events instead of the graph
     int layout = 2;    // BVH records of extend/occlude: 2 or 4 wide
     int fetch = 1;     // 1 one ray per thread, 2 persistent warps with dynamic fetch (two-wide only)
@@ -839,17 +839,33 @@ void apply_test_limits(WfConfig& cfg, const RtRenderParams* p) {
     cfg.shadow_limit = std::max(0, p->shadow_queue_limit);
 }
 
-// Untuned ray order: bounce and shadow rays sorted, except with a
-// participating medium. There nearly every slot is a bounce ray scattered in
-// mid-air and the scene is small, so the sorts' keys and ranks in shade cost
-// more than the coherence wins back (measured, bounce rays sorted: icosphere
-// field +12%, Cornell box +12%, mixed batch +10%, the medium scene -3%; shadow
-// rays sorted as well: a further +3%, +1% and -3%).
-int default_groups(const std::vector<RtScene*>& scenes) {
+// Untuned ray order: bounce and shadow rays sorted, except
+//   - with a participating medium: nearly every slot is then a bounce ray
+//     scattered in mid-air and the scene is small, so the sorts' keys and ranks
+//     in shade cost more than the coherence wins back (-3% on the foggy box);
+//   - in a wavefront of up to 256 K slots: the sorts' two launches an iteration
+//     cost more than traversal gains. Slot order against sorted, Cornell box /
+//     33 icospheres / open sky, ms a render: 12 K samples 0.60 and 0.68 / 0.64
+//     and 0.74 / 0.50 and 0.57; 160 K 0.82 and 0.84 / 0.98 and 1.17 / 0.65 and
+//     0.71; 390 K 1.21 and 1.16 / 1.25 and 1.44 / 0.82 and 0.87; 1.3 M 3.07 and
+//     2.74 / 2.00 and 2.19 / 1.55 and 1.60; 3.1 M 6.2 and 5.4 / 3.4 and 3.5 /
+//     3.06 and 3.05. The Cornell box has the line at 300 K, icospheres past 3 M
+//     (a full-HD frame of 133 M samples gains 10%): it lies where the first of
+//     them starts to gain.
+constexpr int kSortRaysSlots = 1 << 18;
+int default_groups(const std::vector<RtScene*>& scenes, int nslots) {
+    if (nslots <= kSortRaysSlots) return 1;
     for (const RtScene* sc : scenes)
         if (sc->host.has_medium) return 1;
     return 4;
 }
+
+// Untuned material sort: on, except in a wavefront too small to fill the SMs
+// with whole warps of one material (slot order, off against on: 12 K samples
+// 0.53 and 0.60 ms on a Cornell box, 0.53 and 0.64 on icospheres; 49 K 0.57 and
+// 0.63, 0.71 and 0.85; 160 K 0.90 and 0.82, 0.91 and 0.98).
+constexpr int kSortMaterialSlots = 1 << 16;
+int default_sort(int nslots) { return nslots > kSortMaterialSlots; }
 
 // Captures `body` (the launches of one iteration on `stream`) as the body of a
 // loop that repeats until a kernel clears the loop condition, and instantiates
@@ -925,7 +941,6 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         opaque &= sc->opaque;
         dielectrics |= sc->dielectrics;
     }
-    int sort = cfg.sort && nkeys < 255;
     int64_t total = 0;
     std::vector<rt::WfRequest> wreq(reqs.size());
     for (size_t r = 0; r < reqs.size(); r++) {
@@ -947,6 +962,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     }
     int nslots = (int)std::max<int64_t>(1024, std::min<int64_t>(cfg.slots, total));
     nslots = (nslots + 255) / 256 * 256;
+    int sort = (cfg.sort < 0 ? default_sort(nslots) : cfg.sort) && nkeys < 255;
     int64_t cap = (int64_t)nslots * max_shadow;
     if (cap >= ((int64_t)1 << 31) || nslots >= (1 << 29)) return fail(RT_ERR_INVALID_ARG, "wavefront too large");
     // Workspace layout: the call's tables first (one upload), then what one
@@ -1100,7 +1116,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         for (const HostReq& q : reqs) l4_occ = l4_occ && q.scene->host.max_stack4 <= kStack;
     }
     a.any4 = l4_occ && opaque;
-    int groups = cfg.groups > 0 ? cfg.groups : default_groups(scenes);
+    int groups = cfg.groups > 0 ? cfg.groups : default_groups(scenes, nslots);
     // shade is compiled with the volumetric branch and the transmission lobe
     // only when a scene of the batch needs them
     bool medium = false;
