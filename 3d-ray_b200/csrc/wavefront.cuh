@@ -614,15 +614,26 @@ RT_D int ray_key(const SceneView& s, V3 o, V3 d, int cb, int db) {
     return (int)((cell << db) | dir) & (kRayKeys - 1);
 }
 
-// Stores slot i's closest hit and, when sorting, its material key.
-RT_D void hit_store(const WfArgs& a, int i, int req, const SceneView& s, const Hit& h) {
+// Stores slot i's closest hit and, when sorting, its material key: misses and
+// emitters sort after the materials, and a path whose free flight ends in the
+// medium before the hit after those. The flight's two draws are the vertex's
+// first (rng as shade will have it), so its outcome is known here; a warp of
+// shade that held both kinds of vertex ran the medium's and the surface's code,
+// which in a foggy box, where 19 of 20 vertices are in mid-air, most warps did.
+RT_D void hit_store(const WfArgs& a, int i, int req, const SceneView& s, const Hit& h, const Sampler& rng) {
     int packed = h.kind == HIT_NONE ? 0 : ((h.kind << 30) | h.slot);
     a.P.hit[i] = make_float4(h.t, h.u, h.v, ibits(packed));
-    if (a.sort) {   // material key for the scatter
-        int key = a.nkeys;   // misses and emitters sort last
+    if (a.sort) {
+        int key = a.nkeys;
         if (h.kind != HIT_NONE) {
             int ent = h.kind == HIT_TRI ? s.tri_entity[RT_IX(h.slot, s.n_tris)] : h.slot;
             key = RT_IX(a.key_base[a.reqs[req].scene] + s.entities[RT_IX(ent, s.n_entities)].material, a.nkeys);
+        }
+        if (s.has_medium) {
+            Sampler r = rng;
+            float t;
+            V3 beta;
+            if (medium_sample(s, h.kind != HIT_NONE ? h.t : 1e30f, r, t, beta)) key = a.nkeys + 1;
         }
         a.P.keys[i] = key;
     }
@@ -631,8 +642,16 @@ RT_D void hit_store(const WfArgs& a, int i, int req, const SceneView& s, const H
 // A bounce ray's closest hit. One that leaves a scene with neither medium nor
 // sky ends its path here: shade would add nothing.
 RT_D void extend_store(const WfArgs& a, int i, int flags, int req, const SceneView& s, const Hit& h) {
-    if (h.kind == HIT_NONE && !s.has_medium && !s.sky_on) a.P.d[i].w = ibits((flags & ~PF_ALIVE) | PF_DONE);
-    else hit_store(a, i, req, s, h);
+    if (h.kind == HIT_NONE && !s.has_medium && !s.sky_on) {
+        a.P.d[i].w = ibits((flags & ~PF_ALIVE) | PF_DONE);
+        return;
+    }
+    Sampler rng{0u, 0u, 0u};
+    if (a.sort && s.has_medium) {
+        int4 id = a.P.id[i];
+        rng = Sampler{(uint32_t)id.w, (uint32_t)id.x, (uint32_t)fbits(a.P.w[i].w)};
+    }
+    hit_store(a, i, req, s, h, rng);
 }
 
 // One thread per slot. With regroup, the block first reorders its live slots:
@@ -835,7 +854,7 @@ __global__ void __launch_bounds__(128, RT_CAMERA_MIN_BLOCKS) k_wf_camera(const _
             a.P.lp[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             a.P.la[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(a.reqs[req].scene, a.nviews)];
-            hit_store(a, i, req, s, h);
+            hit_store(a, i, req, s, h, Sampler{(uint32_t)seed, (uint32_t)sample, 2u});
         }
         kept += c;
         if (c >= n0) {
@@ -897,7 +916,7 @@ __global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThre
 #pragma unroll
     for (int k = 0; k < kSortPer; k++) {
         int i = first + k * kSortThreads;
-        key[k] = i < a.nslots && (fbits(a.P.d[i].w) & PF_ALIVE) ? RT_IX(a.P.keys[i], a.nkeys + 1) : -1;
+        key[k] = i < a.nslots && (fbits(a.P.d[i].w) & PF_ALIVE) ? RT_IX(a.P.keys[i], a.nkeys + 2) : -1;
     }
 #pragma unroll
     for (int k = 0; k < kSortPer; k++) {
