@@ -843,7 +843,7 @@ struct AdjointReplay : AdjointSink {
     RT_D void aov_miss(V3) {}
     RT_D void aov_surface(V3, const Material&) {}
     RT_D void aov_bounce(bool, V3) {}
-    RT_D void shadow(PathState& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
+    RT_D void shadow(PathState& ps, int, V3 o, V3 d, float tmax, V3 c, int to_la) {
         shadow_impl<STACK, TRANSMIT>(ps, o, d, tmax, c, to_la);
     }
 };

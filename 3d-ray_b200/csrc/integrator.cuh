@@ -436,7 +436,7 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
         V3 wc = wgt * ls.color;
         V3 c = (MEDIUM && med) ? wc * pb : wc * f;
         if (MEDIUM) c = c * tr_m;
-        sink.shadow(ps, ls.ray_o, L, ls.ray_tmax, ps.w * c, to_la);
+        sink.shadow(ps, li, ls.ray_o, L, ls.ray_tmax, ps.w * c, to_la);
         if (MEDIUM && med) sink.nee_medium(ps, li, ls.dist, to_la);
         else sink.nee_surface(ps, li, m, rec, L, view, term, ps.w * wc, ls.dist, tr_m, to_la);
     }
@@ -532,7 +532,7 @@ struct InlineShadows : NoAdjoint {
     int opaque;
     Counters* cnt;
     int* err;
-    RT_D void shadow(PathState& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
+    RT_D void shadow(PathState& ps, int, V3 o, V3 d, float tmax, V3 c, int to_la) {
         V3 tr = shadow_transmittance<STACK>(*s, opaque, o, d, kEps, tmax, cnt, err);
         if (near_zero(tr)) return;
         ps.add(c * tr, to_la);

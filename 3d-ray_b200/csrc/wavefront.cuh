@@ -956,7 +956,7 @@ struct QueueShadows : NoAdjoint {
     int t, slot, scene;   // shade's thread, its slot and scene
     int n;                // records written
     template <class PS>
-    RT_D void shadow(PS& ps, V3 o, V3 d, float tmax, V3 c, int to_la) {
+    RT_D void shadow(PS& ps, int li, V3 o, V3 d, float tmax, V3 c, int to_la) {
         if (!isfinite(c.x) || !isfinite(c.y) || !isfinite(c.z)) {
             ps.add(c, to_la);   // records the per-frame sanitize in the mask
             return;
@@ -971,7 +971,10 @@ struct QueueShadows : NoAdjoint {
         a->S.d[j] = make_float4(d.x, d.y, d.z, ibits((slot << 1) | to_la));
         a->S.c[j] = make_float4(c.x, c.y, c.z, ibits(scene));
         if (a->shadowsort) {   // the record's sort key and its rank in the key's count
-            int key = ray_key(a->views[scene], o, d, a->skey_bits, a->sdir_bits);
+            // above the origin's cell: the light, among up to eight, else the direction's octant
+            const SceneView& s = a->views[scene];
+            int key = ray_key(s, o, d, a->skey_bits, a->sdir_bits);
+            if (s.num_lights > 1 && s.num_lights <= 8) key = (key & ~7) | li;
             unsigned grp = __match_any_sync(__activemask(), key);
             int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
             int base = 0;
