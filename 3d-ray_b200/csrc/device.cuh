@@ -1313,8 +1313,7 @@ struct LightSample {
     V3 color;         // contribution before the shadow transmittance
     V3 dir;
     float dist;
-    V3 ray_o;
-    float ray_tmax;
+    float ray_tmax;   // of the shadow ray, which starts at offset_origin(p, sn)
 };
 
 // A direction in the cone of half-angle acos(cos_max) around w, uniform in
@@ -1415,8 +1414,7 @@ __device__ __noinline__ void light_sample_sphere_env(const SceneView& s, const L
         if (cl <= 0.0f) return;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-        r.ray_o = so;
-        r.ray_tmax = length(sp - so) - kEps;
+            r.ray_tmax = length(sp - so) - kEps;
         float atten = 1.0f / (pdf * (float)l.shadow_samples);
         r.color = l.emission * atten;
         return;
@@ -1461,8 +1459,7 @@ __device__ __noinline__ void light_sample_sphere_env(const SceneView& s, const L
         if (cl <= 0.0f) return;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-        r.ray_o = so;
-        r.ray_tmax = length(sp - so) - kEps;
+            r.ray_tmax = length(sp - so) - kEps;
         float sa = 2.0f * kPi * (1.0f - cmax);
         float atten = l.intensity * sa / (float)l.shadow_samples;
         r.color = l.color * atten;
@@ -1478,7 +1475,6 @@ __device__ __noinline__ void light_sample_sphere_env(const SceneView& s, const L
             return;
         }
         r.has_ray = 1;
-        r.ray_o = offset_origin(p, sn);
         r.ray_tmax = kInf;
         r.color = l.color / (pdf * (float)l.shadow_samples);
         return;
@@ -1562,8 +1558,7 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         }
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-        r.ray_o = so;
-        r.ray_tmax = length(sp - so) - kEps;
+            r.ray_tmax = length(sp - so) - kEps;
         float atten = area * cl / (d2 * (float)l.shadow_samples);
         r.color = l.emission * atten;
         return r;
@@ -1578,7 +1573,6 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         r.color = t.color;
         r.dir = t.dir;
         r.dist = t.dist;
-        r.ray_o = t.ray_o;
         r.ray_tmax = t.ray_tmax;
         return r;
     }
@@ -1602,8 +1596,7 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         if (cl <= 0.0f) return r;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-        r.ray_o = so;
-        r.ray_tmax = length(sp - so) - kEps;
+            r.ray_tmax = length(sp - so) - kEps;
         float ad2 = d2;
         if (l.soft_radius > 0.0f) ad2 = fmaxf(ad2, l.soft_radius * l.soft_radius);
         float atten = l.intensity * l.area * cl / (ad2 * (float)l.shadow_samples);
@@ -1634,7 +1627,6 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
     r.dir = tl;
     r.dist = kInf;
     r.has_ray = 1;
-    r.ray_o = offset_origin(p, sn);
     r.ray_tmax = kInf;
     float e = l.intensity / (float)l.shadow_samples;
     r.color = l.color * e;

@@ -421,7 +421,7 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
             term = shadow_terminator(rec.n, rec.n, view) * shadow_terminator(rec.n, rec.n, L);
             f = f * term;
             if (is_zero(f)) {
-                sink.skipped(ls.ray_o, L, ls.ray_tmax);
+                sink.skipped(offset_origin(rec.p, rec.n), L, ls.ray_tmax);
                 continue;
             }
         }
@@ -436,7 +436,7 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& s, const RenderCon
         V3 wc = wgt * ls.color;
         V3 c = (MEDIUM && med) ? wc * pb : wc * f;
         if (MEDIUM) c = c * tr_m;
-        sink.shadow(ps, li, ls.ray_o, L, ls.ray_tmax, ps.w * c, to_la);
+        sink.shadow(ps, li, offset_origin(rec.p, rec.n), L, ls.ray_tmax, ps.w * c, to_la);
         if (MEDIUM && med) sink.nee_medium(ps, li, ls.dist, to_la);
         else sink.nee_surface(ps, li, m, rec, L, view, term, ps.w * wc, ls.dist, tr_m, to_la);
     }
