@@ -248,6 +248,15 @@ cudaError_t copy_to_device(int dev, cudaStream_t stream, void* dst, const void* 
     return stage_copy(dev, stream, static_cast<char*>(const_cast<void*>(src)), static_cast<char*>(dst), n, false);
 }
 
+// rt_tonemap's device buffer, one per device, kept between calls up to a size.
+constexpr size_t kToneKept = size_t(256) << 20;
+struct ToneBuffer {
+    std::mutex mu;
+    void* mem = nullptr;
+    size_t bytes = 0;
+};
+ToneBuffer g_tone[16];
+
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
@@ -2478,8 +2487,28 @@ int rt_tonemap(const float* hdr, int32_t width, int32_t height, float exposure_e
     size_t n = (size_t)width * height, b = n * 3 * sizeof(float);
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
+    // The images' device buffer is kept per device (up to kToneKept): allocating
+    // and freeing it took 1 to 15 ms of a call, which every Renderer.render makes.
+    // A call that finds it in use by another thread allocates its own.
+    std::unique_lock<std::mutex> lk;
+    ToneBuffer* kept = dev >= 0 && dev < 16 && 2 * b <= kToneKept ? &g_tone[dev] : nullptr;
+    if (kept) {
+        lk = std::unique_lock<std::mutex>(kept->mu, std::try_to_lock);
+        if (!lk.owns_lock()) kept = nullptr;
+    }
     float* d = nullptr;
-    if (cudaMalloc(&d, 2 * b) != cudaSuccess) return fail(RT_ERR_OOM, "allocation failed");
+    if (kept && kept->bytes < 2 * b) {
+        if (kept->mem) cudaFree(kept->mem);
+        kept->mem = nullptr;
+        kept->bytes = 0;
+        if (cudaMalloc(&kept->mem, 2 * b) != cudaSuccess) {
+            kept->mem = nullptr;
+            return fail(RT_ERR_OOM, "allocation failed");
+        }
+        kept->bytes = 2 * b;
+    }
+    if (kept) d = static_cast<float*>(kept->mem);
+    else if (cudaMalloc(&d, 2 * b) != cudaSuccess) return fail(RT_ERR_OOM, "allocation failed");
     int rc = RT_OK;
     if (copy_to_device(dev, cudaStreamPerThread, d, hdr, b) != cudaSuccess) {
         rc = fail(RT_ERR_CUDA, "copy failed");
@@ -2489,7 +2518,8 @@ int rt_tonemap(const float* hdr, int32_t width, int32_t height, float exposure_e
         if (cudaGetLastError() != cudaSuccess || copy_to_host(dev, cudaStreamPerThread, rgb, d + n * 3, b) != cudaSuccess)
             rc = fail(RT_ERR_CUDA, "tonemap failed");
     }
-    cudaFree(d);
+    if (rc != RT_OK) cudaStreamSynchronize(cudaStreamPerThread);   // nothing queued uses the buffer any more
+    if (!kept) cudaFree(d);
     return rc;
 }
 
