@@ -272,6 +272,19 @@ RT_D bool box_hit_te(float lx, float ly, float lz, float hx, float hy, float hz,
     return tx >= te;
 }
 
+// box_hit_te on a record's two corners (xyz and a word that takes no part),
+// the slab distances two an instruction.
+RT_D bool box_hit_te2(float4 lo, float4 hi, F2 nxy, F2 nz, F2 ixy, F2 iz, float tmin, float tmax, float& te) {
+    float t0x, t0y, t0z, t1x, t1y, t1z, w;
+    split2(mul2(add2(f2(lo.x, lo.y), nxy), ixy), t0x, t0y);
+    split2(mul2(add2(f2(lo.z, lo.w), nz), iz), t0z, w);
+    split2(mul2(add2(f2(hi.x, hi.y), nxy), ixy), t1x, t1y);
+    split2(mul2(add2(f2(hi.z, hi.w), nz), iz), t1z, w);
+    te = fmax3(tmin, fminf(t0x, t1x), fmaxf(fminf(t0y, t1y), fminf(t0z, t1z)));
+    float tx = fmin3(tmax, fmaxf(t0x, t1x), fminf(fmaxf(t0y, t1y), fmaxf(t0z, t1z)));
+    return tx >= te;
+}
+
 // Ordered depth-first traversal reproducing HittableList -> BvhNode -> Mesh ->
 // BvhNode -> Triangle (Geometry/HittableList.cs:19-37, Acceleration/BvhNode.cs:157-206).
 // The near child (sign of dir[split axis]) is visited first, fat leaves are
@@ -451,6 +464,7 @@ __device__ __forceinline__ bool traverse(const SceneView& s, V3 o, V3 d, float t
     best.kind = HIT_NONE;
     int code = kNone;
     const unsigned dpos = dir_signs(d);
+    const F2 nxy = f2(-o.x, -o.y), nz = f2(-o.z, 0.0f), ixy = f2(inv.x, inv.y), iz = f2(inv.z, 0.0f);
     if (has_root) {
         code = root;
         if (cnt && root >= 0) cnt->nodes++;   // the mesh root's own BvhNode.Hit
@@ -471,8 +485,8 @@ __device__ __forceinline__ bool traverse(const SceneView& s, V3 o, V3 d, float t
             float4 a = ldg_scene(np), b = ldg_scene(np + 1), c = ldg_scene(np + 2), e = ldg_scene(np + 3);
             if (cnt) cnt->nodes += 2;
             float tel, ter;
-            bool hl = box_hit_te(a.x, a.y, a.z, b.x, b.y, b.z, o, inv, tmin, closest, tel);
-            bool hr = box_hit_te(c.x, c.y, c.z, e.x, e.y, e.z, o, inv, tmin, closest, ter);
+            bool hl = box_hit_te2(a, b, nxy, nz, ixy, iz, tmin, closest, tel);
+            bool hr = box_hit_te2(c, e, nxy, nz, ixy, iz, tmin, closest, ter);
             int axis = __float_as_int(c.w);
             // An opaque any-hit answer does not depend on the visit order, so
             // that walk enters the child whose box the ray meets first (an
