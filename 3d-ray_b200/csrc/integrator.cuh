@@ -275,7 +275,10 @@ struct NoAdjoint {
 // Scatter draw (:1127-1225). The turns share their two Sobol draws, the light
 // samplers and the BSDF's evaluation, so each long stretch of code is compiled
 // once and the lanes of a warp run it together: shading is bound by
-// instruction supply. The NEE integrand and its MIS weight are evaluated
+// instruction supply (with a copy of the evaluation and the samplers at each of
+// their uses, shade took 8.9 against 7.2 ms on a Cornell box of 256x256x64
+// samples and 62.3 against 52.3 ms on four foggy views of 256x256x64). The NEE
+// integrand and its MIS weight are evaluated
 // before the shadow ray and the ray is dropped when they are zero (the
 // reference casts it first; only the cost differs: every draw happens in the
 // light sampler).

@@ -1474,7 +1474,6 @@ int rt_scene_create_ex(const RtWorldDesc* world, const RtSceneOptions* options, 
     int r = RT_OK;
     r = r ? r : upload(sc, h.cnodes, &v.cnodes);
     r = r ? r : upload(sc, h.cnodes4, &v.cnodes4);
-    r = r ? r : upload(sc, h.mesh_root4, &v.mesh_root4);
     r = r ? r : upload(sc, h.top_items, &v.top_items);
     r = r ? r : upload(sc, h.tris, &v.tris);
     r = r ? r : upload(sc, h.tri_entity, &v.tri_entity);
@@ -1500,7 +1499,6 @@ int rt_scene_create_ex(const RtWorldDesc* world, const RtSceneOptions* options, 
     v.num_lights = (int)h.lights.size();
     v.top_is_bvh = h.top_is_bvh;
     v.top_root = h.top_root_code;
-    v.top_root4 = h.top_root4;
     v.walk_root = h.walk_root;
     v.walk_root4 = h.walk_root4;
     v.num_top_items = (int)h.top_items.size();

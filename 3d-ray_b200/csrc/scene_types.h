@@ -155,7 +155,6 @@ struct Camera {
 struct SceneView {
     const float4* cnodes;       // 4 float4 per interior node (child-box layout)
     const float4* cnodes4;      // 8 float4 per four-wide record
-    const int* mesh_root4;      // per entity: a mesh's root code in cnodes4
     const int* top_items;
     const float4* tris;
     const int* tri_entity;
@@ -177,7 +176,6 @@ struct SceneView {
     int num_lights;
     int top_is_bvh;             // 0: the world is a flat list of top_items
     int top_root;               // child code of the top-level root (top_is_bvh only)
-    int top_root4;              // the same in the four-wide layout
     int num_top_items;          // flat list: entity count
     // Where the walks start (the counting build and Walker start at top_root or
     // the flat list). A copy of the top level in which a leaf's entities are
@@ -186,6 +184,8 @@ struct SceneView {
     // test; a quad, sphere or list mesh, which the reference tests without a box
     // of its own, stands there with an unbounded one. Order 3 (in place of an
     // axis) visits the children first to last, as the list is. May be a leaf code.
+    // (A full-HD icosphere frame of 64 samples: extend 37.7 to 28.8, occlude 44.2
+    // to 35.2 ms, the frame 137.0 to 116.7.)
     int walk_root, walk_root4;
     int has_medium;
     V3 sigma_a, sigma_s, sigma_t;

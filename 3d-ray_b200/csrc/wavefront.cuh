@@ -197,28 +197,6 @@ __constant__ WfOne c_wf_one;
 RT_D int fbits(float f) { return __float_as_int(f); }
 RT_D float ibits(int i) { return __int_as_float(i); }
 
-// Warp-aggregated atomic add of 1 per active lane; returns this lane's slot.
-RT_D unsigned long long wagg_next(unsigned long long* ctr) {
-    unsigned mask = __activemask();
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(mask) - 1;
-    int rank = __popc(mask & ((1u << lane) - 1u));
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(ctr, (unsigned long long)__popc(mask));
-    base = __shfl_sync(mask, base, leader);
-    return base + (unsigned long long)rank;
-}
-RT_D int wagg_next_int(int* ctr) {
-    unsigned mask = __activemask();
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(mask) - 1;
-    int rank = __popc(mask & ((1u << lane) - 1u));
-    int base = 0;
-    if (lane == leader) base = atomicAdd(ctr, __popc(mask));
-    base = __shfl_sync(mask, base, leader);
-    return base + rank;
-}
-
 // Stores a whole path state (the adjoint's replay).
 RT_D void wf_store(const WfArgs& a, int i, const PathState& ps, int flags) {
     int dead = (ps.mask.x == 0.0f ? PF_DEAD : 0) | (ps.mask.y == 0.0f ? 2 * PF_DEAD : 0) |
@@ -323,7 +301,11 @@ __device__ __noinline__ void wf_add(float4* dst, float x, float y, float z) {
 // The part of a path's state that a forward vertex works on. The radiance sums
 // and the primary clamp's terms stay in their slot and are written where they
 // change: a whole PathState held 15 more registers through the vertex and
-// moved 128 B more per slot.
+// moved 128 B more per slot. With both gone and a lone request's view and
+// constants in constant memory, shade went from 7.2 to 5.9 ms on a Cornell box
+// of 256x256x64 samples and from 42.2 to 34.8 ms on a full-HD icosphere frame of
+// 64 samples.
+
 // A batch with transmissive materials: the interior absorption and the depth of
 // the IOR stack. The stack's entries stay in the slot (a dielectric surface
 // alone reads them), and outside every dielectric (PF_INSIDE clear) there is
@@ -393,8 +375,10 @@ RT_D void film_add(const WfRequest& R, int lx, int ly, V3 L) {
     atomicAdd(R.accum + 2 * plane + k, (double)L.z);
 }
 
-// Threads of a regen block: one atomic per counter and block, on addresses that
-// every block shares.
+// Regen resolves finished paths and lists the free slots: bound by memory (64 B
+// read and three film atomics per finished path, 16 B of flags per slot).
+// Threads of a block: one atomic per counter and block, on addresses that every
+// block shares.
 constexpr int kRegenBlock = 512;
 template <int MODE>
 __global__ void __launch_bounds__(kRegenBlock) k_wf_regen(const __grid_constant__ WfArgs a) {
@@ -765,7 +749,11 @@ __global__ void __launch_bounds__(256) k_wf_extend_pt(const __grid_constant__ Wf
 // leaves a scene without a medium is a finished sample (the sky's radiance or
 // nothing) and never touches the path state. In an open scene those are most
 // camera rays: with a slot each, they cost the state's writes and reads in
-// regen, extend and shade, and left few bounce rays per iteration to sort.
+// regen, extend and shade, and left few bounce rays per iteration to sort. A
+// full-HD icosphere frame of 64 samples took 152.9 ms with a slot for each and
+// takes 141.5 (regen and the camera rays 13.7 to 22.7 ms, extend 51.3 to 37.8,
+// shade 34.8 to 29.3). The rays' walk bounds it: the warp's 8x4 block of pixels
+// is as coherent as the scene allows.
 // The paths that go on store only what their first vertex does not know: shade
 // sets the rest of a PF_FIRST path itself.
 //
@@ -1128,8 +1116,10 @@ RT_D void key_scan(int* hist, int* off, int* total) {
 }
 
 // Between shade and occlude, one launch: block 0 ends the iteration's
-// bookkeeping (whether the loop goes on, and the counters that the next
-// iteration accumulates; occlude reads none of them), the first cluster scans
+// bookkeeping (whether the loop goes on: a host that read the progress back
+// every few iterations cost a thumbnail of 12 K samples 0.83 against 0.44 ms and a
+// Cornell box of 4 M 11.4 against 10.0 ms; and the counters that the next
+// iteration accumulates, none of which occlude reads), the first cluster scans
 // the bounce rays' keys and the second the shadow records'. loop: the graph's
 // loop condition, 0 when the host runs the iterations itself.
 __global__ void __cluster_dims__(kPlanCluster, 1, 1) __launch_bounds__(1024)

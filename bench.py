@@ -284,7 +284,7 @@ def time_to_relmse(rt, lib, abi):
 
 def profile_frame(args):
     """One warm-up and one measured frame with fixed wavefront settings (4M
-    slots, block 256, material sort) or the megakernel: the workload the ncu
+    slots, material sort, --block for extend/occlude) or the megakernel: the workload the ncu
     summaries under profiles/ were captured on."""
     rt, world = build_world()
     abi = rt.abi
@@ -698,7 +698,7 @@ def main():
                     help="BVH records for --profile-frame: two-wide or four-wide")
     ap.add_argument("--split", action="store_true", help="--profile-frame: per-kernel event times")
     ap.add_argument("--block", type=int, default=256, choices=[64, 128, 256],
-                    help="--profile-frame: block size of extend/occlude (the others use 256)")
+                    help="--profile-frame: block size of extend/occlude")
     ap.add_argument("--ray-fetch", type=int, default=1, choices=[1, 2],
                     help="--profile-frame: one ray per thread (1) or persistent dynamic fetch (2)")
     ap.add_argument("--ray-groups", type=int, default=1, choices=[1, 2, 3, 4],

@@ -198,9 +198,12 @@ typedef struct RtRenderParams {
     int32_t mis_heuristic;          /* RT_MIS_* */
     int32_t light_strategy;         /* RT_LIGHTS_* (LightSamplingStrategy) */
     int32_t kernel;                 /* RT_KERNEL_* */
-    int32_t block_size;             /* wavefront: 64, 128 or 256; 0: autotuned / default */
-    int32_t wavefront_size;         /* wavefront: path slots; 0: autotuned / default */
-    int32_t sort_materials;         /* wavefront: 1 sort hits by material, 0 no, -1 autotuned / default */
+    int32_t block_size;             /* wavefront: block of extend/occlude unless trace_block_size gives
+                                       it: 64, 128 or 256; 0: autotuned / 128 */
+    int32_t wavefront_size;         /* wavefront: path slots; 0: autotuned / 4 M (8 M for renders of
+                                       32 M samples or more), never more than the samples */
+    int32_t sort_materials;         /* wavefront: 1 sort hits by material, 0 no, -1 autotuned / 1 unless
+                                       the wavefront has 64 K slots or fewer */
     int32_t pixel_x0, pixel_y0;     /* render window (0,0,0,0 = full frame) */
     int32_t window_w, window_h;
     int32_t count_work;             /* 1: counting build, fills the work fields of RtStats */
@@ -218,12 +221,13 @@ typedef struct RtRenderParams {
                                        walks the bounce rays sorted by origin cell and direction,
                                        then the camera rays in pixel order, 4 as 3 and occlude walks
                                        the shadow rays sorted the same way; 0 the autotuned choice
-                                       (else 4, or 1 when a scene has a participating medium) */
+                                       (else 4, or 1 when a scene has a participating medium or the
+                                       wavefront has 256 K slots or fewer) */
     /* Test-only limits of the wavefront, for exercising its failure paths.
-     * Both are 0 in production: the host then sizes the queue and bounds the
-     * iterations itself, and neither limit is ever reached. */
+     * Both are 0 in production: the host then sizes the queue and sets the
+     * bound on the iterations itself, and neither limit is ever reached. */
     int32_t iteration_limit;        /* > 0: the wavefront gives up after this many iterations and
-                                       returns RT_ERR_TIMEOUT (the host-side bound on its poll loop) */
+                                       returns RT_ERR_TIMEOUT (the bound on the device's loop) */
     int32_t shadow_queue_limit;     /* > 0: the shadow queue holds at most this many records; a fuller
                                        queue is refused by the kernel and the call returns RT_ERR_BOUNDS */
 } RtRenderParams;
@@ -241,8 +245,9 @@ typedef struct RtStats {
     uint64_t shadow_node_visits;    /* the same three for shadow rays (count_work only) */
     uint64_t shadow_prim_tests;
     uint64_t shadow_other_tests;
-    double   regen_ms, extend_ms, shade_ms, occlude_ms, sort_ms;   /* profile_kernels only; sort_ms holds
-                                       the material sort and the ray sorts' scans and scatter */
+    double   regen_ms, extend_ms, shade_ms, occlude_ms, sort_ms;   /* profile_kernels only; regen_ms holds
+                                       the camera rays too, sort_ms the material sort, the ray sorts'
+                                       scans and scatter and the end of the iteration */
     int32_t  iterations;            /* wavefront iterations */
     int32_t  kernel_launches;       /* kernels launched by the call */
     int32_t  rr_min_bounces;        /* the RR knobs the call used */
