@@ -625,9 +625,9 @@ RT_D void hit_store(const WfArgs& a, int i, int req, const SceneView& s, const H
 
 // A bounce ray's closest hit. One that leaves a scene with neither medium nor
 // sky ends its path here: shade would add nothing.
-RT_D void extend_store(const WfArgs& a, int i, int flags, int req, const SceneView& s, const Hit& h) {
+RT_D void extend_store(const WfArgs& a, int i, int req, const SceneView& s, const Hit& h) {
     if (h.kind == HIT_NONE && !s.has_medium && !s.sky_on) {
-        a.P.d[i].w = ibits((flags & ~PF_ALIVE) | PF_DONE);
+        a.P.d[i].w = ibits((fbits(a.P.d[i].w) & ~PF_ALIVE) | PF_DONE);
         return;
     }
     Sampler rng{0u, 0u, 0u};
@@ -645,7 +645,9 @@ RT_D void extend_store(const WfArgs& a, int i, int flags, int req, const SceneVi
 // one kind of ray and no longer waits on its slowest bounce ray.
 // The register budget of 5 blocks of 256 (48 registers) lets 10 blocks of the
 // autotuned 128 threads share an SM instead of 9: extend -2.5% per 64-spp
-// icosphere frame, for an 8-byte spill.
+// icosphere frame, for an 8-byte spill (6 blocks spill 100 bytes: -0.5% there,
+// +10% on a Cornell box; 4 blocks: +1%). For the same budget the flags are read
+// again where a miss changes them (mixed batch 20.0 to 19.7 ms).
 template <int STACK, bool L4, bool ONE>
 __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ WfArgs a) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -683,7 +685,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend(const __grid_constant__ Wf
     const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(a.reqs[req].scene, a.nviews)];
     Hit h;
     trace<false, STACK, L4>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps, kInf, h, nullptr, a.err);
-    extend_store(a, i, flags, req, s, h);
+    extend_store(a, i, req, s, h);
 }
 
 // Persistent form with dynamic ray fetch (Aila and Laine 2009): a grid sized
@@ -732,7 +734,7 @@ __global__ void __launch_bounds__(256) k_wf_extend_pt(const __grid_constant__ Wf
         if (slot >= 0) {
             const SceneView& s = a.views[RT_IX(a.reqs[req].scene, a.nviews)];
             if (w.step(s, nullptr, a.err)) {
-                extend_store(a, slot, flags, req, s, w.best);
+                extend_store(a, slot, req, s, w.best);
                 slot = -1;
             }
         }
@@ -988,6 +990,26 @@ RT_D void wf_rank_ray(const WfArgs& a, const SceneView& s, V3 o, V3 d, int i) {
     a.P.rrank[i] = base + __popc(grp & ((1u << lane) - 1u));
 }
 
+// Starts the loads of what a vertex reads of slot i first on their way into L2.
+// Shade does this for the slot that a thread of the block
+// kAheadBlocks later will work on, when the material order has scattered the
+// slots: their one block an SM runs in lockstep, so nothing else of the SM covers
+// the first loads, and the slots, over a gigabyte, come from DRAM. The distance
+// is the number of blocks in flight, one an SM. (Shade, with the first loads
+// issued together: four foggy views of 256x256x64 samples 17.6 to 15.9 ms, a
+// mixed batch 43.4 to 42.2, a full-HD icosphere frame of 64 samples 26.4 to 26.2.
+// The adjoint's vertex gained nothing from it.)
+constexpr int kAheadBlocks = 148;
+RT_D void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+RT_D void wf_prefetch(const WfArgs& a, int i) {
+    prefetch_l2(a.P.d + i);
+    prefetch_l2(a.P.id + i);
+    prefetch_l2(a.P.hit + i);
+    prefetch_l2(a.P.o + i);
+    prefetch_l2(a.P.beta + i);
+    prefetch_l2(a.P.w + i);
+}
+
 // Hit record of slot i as extend wrote it.
 RT_D Hit wf_hit(const WfArgs& a, int i) {
     float4 hh = a.P.hit[i];
@@ -1011,23 +1033,26 @@ constexpr int kShadeBlock = 512;
 template <bool MEDIUM, bool TRANSMIT, bool ONE>
 __global__ void __launch_bounds__(kShadeBlock, 1) k_wf_shade(const __grid_constant__ WfArgs a) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    int i;
+    int i, next = -1;
     if (a.sort) {
         // the scatter left the live slots in material order in order[0 .. live)
         if (t >= a.ctl->nlive) return;
         i = RT_IX(a.P.order[RT_IX(t, a.nslots)], a.nslots);
+        next = t + kAheadBlocks * blockDim.x;
+        next = next < a.ctl->nlive ? RT_IX(a.P.order[next], a.nslots) : -1;
     } else {
         if (t >= a.nslots) return;
         i = t;
     }
     float4 d = a.P.d[i];
+    int4 id = a.P.id[i];
+    Hit h = wf_hit(a, i);
+    if (next >= 0) wf_prefetch(a, next);
     int flags = fbits(d.w);
     if (!(flags & PF_ALIVE)) {
         a.S.cnt[t] = 0;
         return;
     }
-    int4 id = a.P.id[i];
-    Hit h = wf_hit(a, i);
     int req = ONE ? 0 : RT_IX(id.z, a.nreq);
     const RenderConst& rc = ONE ? c_wf_one.rc : a.reqs[req].rc;
     int scene = ONE ? 0 : RT_IX(a.reqs[req].scene, a.nviews);
@@ -1238,19 +1263,22 @@ __global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid
             return;
         }
     }
-    float4 o = a.S.o[j], d = a.S.d[j], c = a.S.c[j];
+    // The any-hit walk has no register to spare for what a visible ray adds: it
+    // is read after it, and added in one vector operation (full-HD icosphere frame
+    // of 64 samples 29.8 to 29.2 ms, smooth mesh 1.40 to 1.35, Cornell box 0.74 to
+    // 0.70). The transparent walk has, and takes it along: read late it lost 2%.
+    constexpr bool LATE = OPAQUE && ONE;
+    float4 o = a.S.o[j], d = a.S.d[j], c;
+    if (!LATE) c = a.S.c[j];
     const SceneView& s = ONE ? c_wf_one.view : a.views[RT_IX(fbits(c.w), a.nviews)];
     V3 tr = shadow_transmittance<STACK, L4>(s, OPAQUE ? 1 : a.opaque, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), kEps,
                                             o.w, nullptr, a.err);
     if (near_zero(tr)) return;
-    int packed = fbits(d.w);
+    if (LATE) c = a.S.c[j];
+    int packed = fbits(LATE ? a.S.d[j].w : d.w);
     int slot = RT_IX(packed >> 1, a.nslots);
     V3 v = v3(c.x, c.y, c.z) * tr;
-    float4* dst = (packed & 1) ? (a.P.la + slot) : (a.P.lp + slot);
-    float* f = reinterpret_cast<float*>(dst);
-    atomicAdd(f, v.x);
-    atomicAdd(f + 1, v.y);
-    atomicAdd(f + 2, v.z);
+    atomicAdd((packed & 1) ? (a.P.la + slot) : (a.P.lp + slot), make_float4(v.x, v.y, v.z, 0.0f));
 }
 
 // Mean of the accumulated sums into the films (Renderer.cs:711).
