@@ -1178,9 +1178,9 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     while (sblk > 64 && (int64_t)sblk * 148 > nslots) sblk /= 2;
     unsigned gs = (unsigned)((nslots + sblk - 1) / sblk);
     unsigned gst = (unsigned)((nslots + tblk - 1) / tblk);
-    dim3 gsh(gst, (unsigned)max_shadow);   // occlude and the shadow scatter: (shade's threads, records of each)
-    unsigned g256 = (unsigned)((nslots + 255) / 256);
-    dim3 gsh256(g256, (unsigned)max_shadow);
+    // occlude and the shadow scatter: (shade's threads, records of each)
+    const dim3 gsh(gst, (unsigned)max_shadow);
+    const dim3 gss((unsigned)std::min((nslots + 255) / 256, rt::kScatterBlocks), (unsigned)max_shadow);
     // the camera kernel: persistent warps, as many as are resident
     void (*camera)(const rt::WfArgs) =
         mode == rt::WF_RECORD ? rt::k_wf_camera<kStack, rt::WF_RECORD, true>
@@ -1232,7 +1232,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         }
         if (ev) cudaEventRecord(ev[4], stream);   // the ray sorts' scans and scatter count as sorting
         rt::k_wf_plan<<<gplan, 1024, 0, stream>>>(a, loop);
-        if (a.shadowsort) rt::k_wf_sscatter<<<gsh256, 256, 0, stream>>>(a);
+        if (a.shadowsort) rt::k_wf_sscatter<<<gss, 256, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[5], stream);
         if (mode != rt::WF_REPLAY) {
             if (pt && a.opaque) rt::k_wf_occlude_pt<kStack><<<gpt_o, tblk, 0, stream>>>(a);
@@ -1251,7 +1251,7 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
         // bytes key the cached ones.
         const unsigned shape[] = {(unsigned)blk, (unsigned)tblk, (unsigned)l4, (unsigned)l4_occ, (unsigned)pt,
                                   (unsigned)medium, (unsigned)transmit, (unsigned)one, (unsigned)one_scene, gpt_e, gpt_o, gs, gst,
-                                  (unsigned)max_shadow, g256, gcam, gplan, (unsigned)mode, gadj, (unsigned)adj_blk, (unsigned)adj_shmem};
+                                  (unsigned)max_shadow, gcam, gplan, (unsigned)mode, gadj, (unsigned)adj_blk, (unsigned)adj_shmem};
         std::vector<unsigned char> key(sizeof(a) + sizeof(shape));
         std::memcpy(key.data(), &a, sizeof(a));
         std::memcpy(key.data() + sizeof(a), shape, sizeof(shape));

@@ -86,6 +86,17 @@ def test_slot_counts_render_the_same_film(world, slots):
             same_film(s.render(160, 120, 16, 6, kernel=abi.KERNEL_WAVEFRONT, wavefront_size=slots, **kw), ref)
 
 
+# Slots around one and two turns of the shadow scatter's threads (1480 blocks of
+# 256) and a shade block on every SM (148 of 512), whose next wave is prefetched.
+@pytest.mark.parametrize("slots", [75776, 75776 + 256, 378880 - 256, 378880, 378880 + 256, 2 * 378880 + 256])
+@pytest.mark.parametrize("world", ["icospheres", "smooth"])
+def test_sorted_shadows_take_turns(world, slots):
+    with Scene(WORLDS[world]()) as s:
+        ref = s.render(320, 240, 16, 4, kernel=abi.KERNEL_MEGAKERNEL)
+        same_film(s.render(320, 240, 16, 4, kernel=abi.KERNEL_WAVEFRONT, wavefront_size=slots, ray_groups=4,
+                           sort_materials=1), ref)
+
+
 def test_no_bounce_and_no_depth():
     """max_depth 0 renders black, depth 1 only what camera rays see; twice, so
     that the second render replays a kept graph."""
