@@ -875,9 +875,11 @@ int default_groups(const std::vector<RtScene*>& scenes, int nslots) {
 // drain less weight, until the render is too short to fill them. 4 M against
 // 8 M: full-HD icospheres of 133 M samples 109.0 and 104.7 ms, the mixed batch
 // of 63 M 103.3 and 100.9; foggy views of 17 M 46.4 and 47.2, open sky of 11 M
-// 8.4 and 9.2. 16 M gained nothing anywhere.
+// 8.4 and 9.2. 16 M gained nothing anywhere. Where 8 M do not fit the device's
+// free memory, wf_render takes 4 M.
+constexpr int kDefaultSlots = 1 << 22;
 int default_slots(int64_t total, int max_shadow) {
-    return total >= (int64_t)1 << 25 && max_shadow <= 4 ? 1 << 23 : 1 << 22;
+    return total >= (int64_t)1 << 25 && max_shadow <= 4 ? 2 * kDefaultSlots : kDefaultSlots;
 }
 
 // Untuned material sort: on, except in a wavefront too small to fill the SMs
@@ -923,12 +925,10 @@ int wf_capture(cudaStream_t stream, F body, cudaGraphExec_t& exec) {
 // mode: rt::WF_RENDER renders the requests into their films; rt::WF_RECORD
 // and rt::WF_REPLAY are the two passes of the wavefront adjoint over the same
 // requests, with adj holding their buffers (rt_adjoint).
-int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st, int mode = rt::WF_RENDER,
-              const rt::WfAdjoint* adj = nullptr) {
+// Called with g_wf_mu held.
+int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st, int mode,
+                     const rt::WfAdjoint* adj) {
     auto t0 = std::chrono::steady_clock::now();
-    if (reqs.empty()) return RT_OK;
-    if (mode != rt::WF_RENDER && !adj) return fail(RT_ERR_INVALID_ARG, "adjoint pass without its buffers");
-    std::lock_guard<std::mutex> lk(g_wf_mu);
     RtScene* s0 = reqs[0].scene;
     int dev = s0->device;
     CUDA_TRY(cudaSetDevice(dev));
@@ -1378,6 +1378,21 @@ int wf_config(const RtScene* sc, const RtRenderParams* p, WfConfig& out) {
         return fail(RT_ERR_INVALID_ARG, "trace_block_size must be 64, 128 or 256");
     out = cfg;
     return RT_OK;
+}
+
+int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st, int mode = rt::WF_RENDER,
+              const rt::WfAdjoint* adj = nullptr) {
+    if (reqs.empty()) return RT_OK;
+    if (mode != rt::WF_RENDER && !adj) return fail(RT_ERR_INVALID_ARG, "adjoint pass without its buffers");
+    std::lock_guard<std::mutex> lk(g_wf_mu);
+    int rc = wf_render_locked(reqs, cfg, st, mode, adj);
+    if (rc == RT_ERR_OOM && cfg.slots <= 0) {   // the larger untuned size does not fit: the smaller may
+        cudaGetLastError();
+        WfConfig c = cfg;
+        c.slots = kDefaultSlots;
+        rc = wf_render_locked(reqs, c, st, mode, adj);
+    }
+    return rc;
 }
 
 int wf_render_one(RtScene* sc, const RtRenderParams* p, const RtCameraDesc& cam, float* d_film, RtStats* st) {
@@ -2519,7 +2534,10 @@ int rt_tonemap(const float* hdr, int32_t width, int32_t height, float exposure_e
     if (kept) d = static_cast<float*>(kept->mem);
     else if (cudaMalloc(&d, 2 * b) != cudaSuccess) return fail(RT_ERR_OOM, "allocation failed");
     int rc = RT_OK;
-    if (copy_to_device(dev, cudaStreamPerThread, d, hdr, b) != cudaSuccess) {
+    // a small image is not waited for twice: the copy back, which is, comes after it
+    const cudaError_t up = b < kStageChunk ? cudaMemcpyAsync(d, hdr, b, cudaMemcpyHostToDevice, cudaStreamPerThread)
+                                           : copy_to_device(dev, cudaStreamPerThread, d, hdr, b);
+    if (up != cudaSuccess) {
         rc = fail(RT_ERR_CUDA, "copy failed");
     } else {
         k_tonemap<<<(unsigned)((n + 255) / 256), 256, 0, cudaStreamPerThread>>>(d, (int)n, powf(2.0f, exposure_ev),
