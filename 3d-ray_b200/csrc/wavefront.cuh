@@ -900,6 +900,9 @@ __global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThre
     cg::cluster_group cluster = cg::this_cluster();
     const unsigned rank = cluster.block_rank();
     const int tid = threadIdx.x, first = blockIdx.x * (kSortThreads * kSortPer) + tid;
+    // A block's shared memory may be written by another once that block runs:
+    // all arrive here, and wait before the first remote store, behind the loads.
+    cluster.barrier_arrive();
     if (tid < 256) s_cnt[tid] = 0;
     __syncthreads();
     int key[kSortPer], pos[kSortPer];
@@ -917,6 +920,7 @@ __global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThre
         pos[k] = __shfl_sync(0xffffffffu, base, leader) + __popc(grp & ((1u << lane) - 1u));
     }
     __syncthreads();
+    cluster.barrier_wait();
     // every block gets every block's counts: a key's slots of the earlier blocks go first
     if (tid < 256)
         for (int q = 0; q < kSortCluster; q++) cluster.map_shared_rank(&s_all[0][0], q)[rank * 256 + tid] = s_cnt[tid];
@@ -1119,10 +1123,12 @@ RT_D void key_scan(int* hist, int* off, int* total) {
     cg::cluster_group cluster = cg::this_cluster();
     const unsigned rank = cluster.block_rank();
     const int at = (int)rank * 1024 + threadIdx.x;
+    cluster.barrier_arrive();   // every block of the cluster runs: see k_wf_scatter
     int4 v = reinterpret_cast<int4*>(hist)[at];
     reinterpret_cast<int4*>(hist)[at] = make_int4(0, 0, 0, 0);
     int sum;
     int base = block_scan(v.x + v.y + v.z + v.w, s_w, &sum);
+    cluster.barrier_wait();
     if (threadIdx.x < kPlanCluster) *cluster.map_shared_rank(&s_sum[rank], threadIdx.x) = sum;
     cluster.sync();
     int all = 0;
