@@ -182,3 +182,42 @@ def test_display_transform_at_the_copies_edges(w, h):
     c = x.astype(np.float64) * float(np.float32(2.0 ** 0.5))
     y = np.clip(c * (2.51 * c + 0.03) / (c * (2.43 * c + 0.59) + 0.14), 0.0, 1.0) ** (1.0 / 2.2)
     np.testing.assert_allclose(out, y.transpose(1, 2, 0), rtol=0, atol=1e-6)
+
+
+def test_renders_and_display_transforms_from_several_threads():
+    """Every caller gets its own film and its own display image, also where the
+    staging window and the display buffer are taken by another thread."""
+    import threading
+    rng = np.random.default_rng(8)
+    films = [np.exp(rng.normal(-1.0, 1.5, (3, 400, 700 + k))).astype(np.float32) for k in range(3)]
+    lib = abi.load()
+
+    def shown(x):
+        out = np.full(x.shape[1:] + (3,), -1.0, np.float32)
+        abi.check(lib.rt_tonemap(abi.ptr(x), x.shape[2], x.shape[1], 0.0, abi.ptr(out)), "rt_tonemap")
+        return out
+
+    worlds = [WORLDS["cornell"](), WORLDS["icospheres"]()]
+    size = dict(w=420, h=300, spp=2, depth=3, kernel=abi.KERNEL_WAVEFRONT)
+    alone = [shown(x) for x in films]
+    with Scene(worlds[0]) as a, Scene(worlds[1]) as b:
+        ref = [s.render(**size) for s in (a, b)]
+        wrong = []
+
+        def show(k):
+            for _ in range(12):
+                if not np.array_equal(shown(films[k]), alone[k]):
+                    wrong.append(("display", k))
+
+        def draw(s, want):
+            for _ in range(12):
+                if not np.allclose(s.render(**size), want, rtol=1e-5, atol=1e-6):
+                    wrong.append(("film", s))
+
+        threads = [threading.Thread(target=show, args=(k,)) for k in range(3)]
+        threads += [threading.Thread(target=draw, args=(s, r)) for s, r in ((a, ref[0]), (b, ref[1]))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not wrong
