@@ -46,13 +46,20 @@ inline cudaError_t stage_copy(int dev, cudaStream_t stream, char* host, char* de
     Stage& st = g_stage[dev];
     std::unique_lock<std::mutex> lk(st.mu, std::try_to_lock);
     if (!lk.owns_lock()) return plain();
-    if (!st.mem) {
-        if (cudaMallocHost(&st.mem, kStageChunk * kStageChunks) != cudaSuccess) {
+    if (!st.mem) {   // no window or no events: the driver's way
+        bool ok = cudaMallocHost(&st.mem, kStageChunk * kStageChunks) == cudaSuccess;
+        size_t made = 0;
+        while (ok && made < kStageChunks) {
+            ok = cudaEventCreateWithFlags(&st.landed[made], cudaEventDisableTiming) == cudaSuccess;
+            made += ok;
+        }
+        if (!ok) {
+            cudaGetLastError();
+            while (made) cudaEventDestroy(st.landed[--made]);
+            if (st.mem) cudaFreeHost(st.mem);
             st.mem = nullptr;
-            cudaGetLastError();   // no window: the driver's way
             return plain();
         }
-        for (cudaEvent_t& e : st.landed) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     }
     for (size_t w = 0; w < n; w += kStageChunk * kStageChunks) {   // one window at a time
         const size_t bytes = std::min(n - w, kStageChunk * kStageChunks);

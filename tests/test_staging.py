@@ -25,3 +25,9 @@ def binary(tmp_path_factory):
 def test_copies_are_done_when_they_return(binary):
     r = subprocess.run([binary], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.parametrize("events", [0, 1, 31])
+def test_without_events_copies_go_the_plain_way(binary, events):
+    r = subprocess.run([binary, str(events)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
