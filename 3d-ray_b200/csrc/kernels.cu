@@ -827,13 +827,20 @@ int wf_capture(cudaStream_t stream, F body, cudaGraphExec_t& exec) {
         cudaGraph_t inner = np.conditional.phGraph_out[0];
         e = cudaStreamBeginCaptureToGraph(stream, inner, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
+            cudaGetLastError();
             body(loop);
+            const cudaError_t launched = cudaGetLastError();   // a refused launch need not end the capture
             e = cudaStreamEndCapture(stream, &inner);
+            if (e == cudaSuccess) e = launched;
         }
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);   // the executable graph does not need it
+    // After a failed capture it is not documented whether the loop's body still
+    // stands: the graph is then left rather than destroyed over it. (A launch that
+    // the capture refused ended the process on these last lines; wf_render_locked
+    // refuses such sizes first.)
     if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    cudaGraphDestroy(graph);   // the executable graph does not need it
     return RT_OK;
 }
 
@@ -900,6 +907,8 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     int sort = (cfg.sort < 0 ? default_sort(nslots) : cfg.sort) && nkeys < 254;   // two keys beside the materials' (hit_store)
     int64_t cap = (int64_t)nslots * max_shadow;
     if (cap >= ((int64_t)1 << 31) || nslots >= (1 << 29)) return fail(RT_ERR_INVALID_ARG, "wavefront too large");
+    const int blk = cfg.block, tblk = cfg.tblock > 0 ? cfg.tblock : blk;
+    if (tblk > 256) return fail(RT_ERR_INVALID_ARG, "blocks of extend and occlude hold at most 256 threads");
     // Workspace layout: the call's tables first (one upload), then what one
     // memset clears, then the rest.
     auto align = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -1036,8 +1045,6 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     }
     CUDA_TRY(cudaMemsetAsync(static_cast<char*>(ws.mem) + clear_begin, 0, clear_end - clear_begin, stream));
     // One iteration: regen, camera, extend, [scatter], shade, plan, [sscatter], occlude.
-    int blk = cfg.block;
-    int tblk = cfg.tblock > 0 ? cfg.tblock : blk;
     bool l4 = cfg.layout == 4;
     for (const HostReq& q : reqs) l4 = l4 && q.scene->host.max_stack4 <= kStack;
     bool pt = !l4 && cfg.fetch == 2;
@@ -1200,9 +1207,11 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
             if (rc == RT_OK && cudaEventCreate(&e) != cudaSuccess) rc = fail(RT_ERR_CUDA, "event creation failed");
         while (rc == RT_OK) {
             launch_iter(pev, cudaGraphConditionalHandle{});
-            cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
-            if (cudaStreamSynchronize(stream) != cudaSuccess) {
-                rc = fail(RT_ERR_CUDA, std::string("wavefront iteration failed: ") + cudaGetErrorString(cudaGetLastError()));
+            cudaError_t e = cudaGetLastError();
+            if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) {
+                rc = fail(RT_ERR_CUDA, std::string("wavefront iteration failed: ") + cudaGetErrorString(e));
                 break;
             }
             float m[kEv - 1];

@@ -202,3 +202,28 @@ def test_batch_limits_apply_to_the_whole_batch(cornell_scene):
     common.iteration_limit = 0
     abi.check(s.lib.rt_render_batch(scenes, 1, reqs, 2, C.byref(common), optrs, C.byref(st)), "rt_render_batch")
     assert all(np.all(np.isfinite(o)) and o.mean() > 0 for o in outs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("profile", [0, 1])
+def test_a_block_the_kernels_do_not_take_is_refused_before_any_launch(cornell_scene, profile):
+    """A batch with blocks of 1024 threads is refused by the host (a launch that is
+    refused while the loop is captured ends the process in the driver); the error is
+    that call's alone, and both kernels render as before."""
+    s = cornell_scene
+    _, ref, _ = s.render(_wf())
+    mega = abi.render_params(48, 48, 64, 8, kernel=abi.KERNEL_MEGAKERNEL)
+    _, mega_ref, _ = s.render(mega)
+    req = (abi.RtRequest * 1)()
+    req[0].scene, req[0].width, req[0].height, req[0].spp, req[0].max_depth = 0, 32, 32, 32, 8
+    req[0].camera = abi.camera_desc(S.cornell().camera)
+    out = np.zeros((3, 32, 32), np.float32)
+    scenes, optrs, st = (C.c_void_p * 1)(s.h), (C.c_void_p * 1)(out.ctypes.data), abi.RtStats()
+    common = abi.render_params(1, 1, 1, 1, kernel=abi.KERNEL_WAVEFRONT, wavefront_size=1 << 12, block_size=1024,
+                               profile_kernels=profile)
+    assert s.lib.rt_render_batch(scenes, 1, req, 1, C.byref(common), optrs, C.byref(st)) == -1
+    assert not out.any()
+    for p, want in ((mega, mega_ref), (_wf(), ref)):
+        rc, img, _ = s.render(p)
+        assert rc == 0, s.lib.rt_last_error()
+        np.testing.assert_allclose(img, want, rtol=1e-4, atol=1e-6)
