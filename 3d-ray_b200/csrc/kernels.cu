@@ -844,6 +844,22 @@ int wf_capture(cudaStream_t stream, F body, cudaGraphExec_t& exec) {
     return RT_OK;
 }
 
+// Every way out of a call between its first work on the stream and its last wait
+// but the good one: what is queued uses the workspace, its pinned tables and the
+// constants, which the next call, of any scene and stream, writes again. No graph
+// of a failed call is replayed, and its error is not the next call's.
+struct WfExit {
+    cudaStream_t stream;
+    WfWorkspace& ws;
+    bool waited = false;
+    ~WfExit() {
+        if (waited) return;
+        cudaStreamSynchronize(stream);
+        cudaGetLastError();
+        ws.drop_graphs();
+    }
+};
+
 // mode: rt::WF_RENDER renders the requests into their films; rt::WF_RECORD
 // and rt::WF_REPLAY are the two passes of the wavefront adjoint over the same
 // requests, with adj holding their buffers (rt_adjoint).
@@ -1037,6 +1053,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     std::memcpy(ws.pinned + off_adj, &J, sizeof(J));
     std::memcpy(ws.pinned + off_films, films.data(), films.size() * sizeof(float*));
     std::memcpy(ws.pinned + off_fdims, fdims.data(), fdims.size() * sizeof(int));
+    WfExit way_out{stream, ws};
     CUDA_TRY(cudaMemcpyAsync(ws.mem, ws.pinned, table_bytes, cudaMemcpyHostToDevice, stream));
     if (one_scene) {
         rt::WfOne c{views[0], wreq[0].rc};
@@ -1221,7 +1238,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
             t_sort += m[2] + m[4];   // the material sort, then the ray sorts' scans and scatter
             t_shade += m[3];
             t_occlude += m[5];
-            if (back->done || back->overflow || back->iters >= back->limit) break;
+            if (back->done || back->overflow || back->err || back->iters >= back->limit) break;
         }
         for (auto e : pev)
             if (e) cudaEventDestroy(e);
@@ -1239,6 +1256,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) rc = fail(RT_ERR_CUDA, std::string("wavefront failed: ") + cudaGetErrorString(e));
+        else way_out.waited = true;
     }
     if (rc == RT_OK) {
         if (back->overflow) rc = fail(RT_ERR_BOUNDS, "shadow queue overflow");
@@ -1246,10 +1264,6 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         else if (back->err != 0) rc = fail(RT_ERR_BOUNDS, "device error " + std::to_string(back->err));
         else if (!back->done) rc = fail(RT_ERR_TIMEOUT, "wavefront did not drain within its iteration bound");
         else rc = checked_flag(stream);
-    }
-    if (rc == RT_ERR_CUDA) {   // a failed launch: finish what is queued, and replay no graph again
-        cudaStreamSynchronize(stream);
-        ws.drop_graphs();
     }
     if (rc != RT_OK) return rc;
     const int64_t iters = back->iters;

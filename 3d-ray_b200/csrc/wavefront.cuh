@@ -1159,7 +1159,7 @@ __global__ void __cluster_dims__(kPlanCluster, 1, 1) __launch_bounds__(1024)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         c->iters++;
         c->done = c->next >= c->total && c->live == 0;
-        if (loop && (c->done || c->overflow || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
+        if (loop && (c->done || c->overflow || c->err || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
         c->iter_first = c->next;
         c->live = 0;
         c->ext_next = 0;
