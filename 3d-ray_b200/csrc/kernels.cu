@@ -1249,10 +1249,6 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         if (mode == rt::WF_RENDER)
             rt::k_wf_finalize<<<g, 256, 0, stream>>>(d_reqs, (int)wreq.size(), d_films, d_fdims, d_fdims + reqs.size());
         cudaError_t e = cudaEventRecord(s0->ev1, stream);
-        for (size_t r = 0; r < reqs.size() && e == cudaSuccess; r++)
-            if (reqs[r].host_film)
-                e = copy_to_host(dev, stream, reqs[r].host_film, films[r],
-                                 (size_t)3 * reqs[r].W * reqs[r].H * sizeof(float));
         if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) rc = fail(RT_ERR_CUDA, std::string("wavefront failed: ") + cudaGetErrorString(e));
@@ -1264,6 +1260,15 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         else if (back->err != 0) rc = fail(RT_ERR_BOUNDS, "device error " + std::to_string(back->err));
         else if (!back->done) rc = fail(RT_ERR_TIMEOUT, "wavefront did not drain within its iteration bound");
         else rc = checked_flag(stream);
+    }
+    for (size_t r = 0; r < reqs.size() && rc == RT_OK; r++) {   // a failed call leaves its outputs as they were
+        if (!reqs[r].host_film) continue;
+        cudaError_t e = copy_to_host(dev, stream, reqs[r].host_film, films[r],
+                                     (size_t)3 * reqs[r].W * reqs[r].H * sizeof(float));
+        if (e != cudaSuccess) {
+            way_out.waited = false;
+            rc = fail(RT_ERR_CUDA, std::string("film copy failed: ") + cudaGetErrorString(e));
+        }
     }
     if (rc != RT_OK) return rc;
     const int64_t iters = back->iters;

@@ -227,3 +227,24 @@ def test_a_block_the_kernels_do_not_take_is_refused_before_any_launch(cornell_sc
         rc, img, _ = s.render(p)
         assert rc == 0, s.lib.rt_last_error()
         np.testing.assert_allclose(img, want, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit,code", [(dict(iteration_limit=1), -4), (dict(iteration_limit=3), -4),
+                                        (dict(shadow_queue_limit=64), -5)])
+def test_a_failed_batch_leaves_its_outputs_as_they_were(cornell_scene, limit, code):
+    s = cornell_scene
+    sizes = ((32, 24), (640, 480))   # copied plainly, and by the staging window
+    req = (abi.RtRequest * 2)()
+    outs = [np.full((3, h, w), 7.0, np.float32) for w, h in sizes]
+    for i, (w, h) in enumerate(sizes):
+        req[i].scene, req[i].width, req[i].height, req[i].spp, req[i].max_depth = 0, w, h, 2, 8
+        req[i].camera = abi.camera_desc(S.cornell().camera)
+    scenes, optrs = (C.c_void_p * 1)(s.h), (C.c_void_p * 2)(*[o.ctypes.data for o in outs])
+    st = abi.RtStats()
+    common = abi.render_params(1, 1, 1, 1, kernel=abi.KERNEL_WAVEFRONT, wavefront_size=1 << 14, **limit)
+    assert s.lib.rt_render_batch(scenes, 1, req, 2, C.byref(common), optrs, C.byref(st)) == code
+    assert all(np.all(o == 7.0) for o in outs)
+    common.iteration_limit = common.shadow_queue_limit = 0
+    abi.check(s.lib.rt_render_batch(scenes, 1, req, 2, C.byref(common), optrs, C.byref(st)), "rt_render_batch")
+    assert all(o.mean() > 0 and not np.any(o == 7.0) for o in outs)
