@@ -1117,9 +1117,10 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     while (sblk > 64 && (int64_t)sblk * 148 > nslots) sblk /= 2;
     unsigned gs = (unsigned)((nslots + sblk - 1) / sblk);
     unsigned gst = (unsigned)((nslots + tblk - 1) / tblk);
-    // occlude and the shadow scatter: (shade's threads, records of each)
-    const dim3 gsh(gst, (unsigned)max_shadow);
-    const dim3 gss((unsigned)std::min((nslots + 255) / 256, rt::kScatterBlocks), (unsigned)max_shadow);
+    // occlude and the shadow scatter: (shade's threads, records of each: shadow_row)
+    const unsigned rows = (unsigned)std::min(max_shadow, rt::kMaxRows), layers = (unsigned)((max_shadow + rt::kMaxRows - 1) / rt::kMaxRows);
+    const dim3 gsh(gst, rows, layers);
+    const dim3 gss((unsigned)std::min((nslots + 255) / 256, rt::kScatterBlocks), rows, layers);
     // the camera kernel: persistent warps, as many as are resident
     void (*camera)(const rt::WfArgs) =
         mode == rt::WF_RECORD ? rt::k_wf_camera<kStack, rt::WF_RECORD, true>

@@ -1182,6 +1182,12 @@ RT_D int shadow_record(const WfArgs& a, int t, int k) {
     return k * a.nslots + t;
 }
 
+// Occlude and the shadow scatter run a row of blocks per record that a vertex may
+// write (shade's threads along x). Rows lie along y and, past that axis's 65 535
+// (a light of 256 x 256 samples), along z.
+constexpr int kMaxRows = 65535;
+RT_D int shadow_row() { return (int)(blockIdx.z * gridDim.y + blockIdx.y); }
+
 // Shadow sort: each queued record goes to its key's offset plus its rank. Few
 // threads that take many turns: with a thread per possible record most blocks
 // had nothing to do, and starting them took longer than the records (8 M slots
@@ -1193,7 +1199,7 @@ constexpr int kScatterBlocks = 148 * 10;
 __global__ void k_wf_sscatter(const __grid_constant__ WfArgs a) {
     const int n = a.sort ? a.ctl->shaded : a.nslots;
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < (unsigned)n; t += gridDim.x * blockDim.x) {
-        int j = shadow_record(a, (int)t, blockIdx.y);
+        int j = shadow_record(a, (int)t, shadow_row());
         if (j < 0) continue;
         int pos = a.soff[RT_IX(a.S.key[j], kRayKeys)] + a.S.rank[j];
         if (pos < a.ctl->nshadow) a.S.order[pos] = j;
@@ -1259,12 +1265,12 @@ template <int STACK, bool L4, bool OPAQUE, bool ONE>
 __global__ void __launch_bounds__(256, OPAQUE ? 5 : 1) k_wf_occlude(const __grid_constant__ WfArgs a) {
     int j;
     if (a.shadowsort) {   // a flat grid over the sorted order
-        long long p = (long long)blockIdx.y * gridDim.x * blockDim.x + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        long long p = (long long)shadow_row() * gridDim.x * blockDim.x + (long long)blockIdx.x * blockDim.x + threadIdx.x;
         int n = a.ctl->nshadow;
         if (p >= n) return;
         j = RT_IX(a.S.order[p], a.nslots * a.S.per);
     } else {
-        j = shadow_record(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+        j = shadow_record(a, blockIdx.x * blockDim.x + threadIdx.x, shadow_row());
         if (a.regroup) {   // shadow rays by direction octant
             __shared__ int s_idx[256], s_cnt[8][8], s_tot;
             int cls = -1;

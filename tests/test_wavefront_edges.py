@@ -97,6 +97,19 @@ def test_sorted_shadows_take_turns(world, slots):
                            sort_materials=1), ref)
 
 
+# Shadow samples whose records a vertex fill one axis of a grid, and one more row.
+# Film values are sums of that many positive terms in another order: each addition
+# rounds by 2^-24 of the sum at most, 65 536 x 2^-24 on either side.
+@pytest.mark.parametrize("side", [255, 256])
+@pytest.mark.parametrize("kw", [dict(ray_groups=1), dict(ray_groups=2), dict(ray_groups=4, sort_materials=1)])
+def test_a_light_of_many_shadow_samples(side, kw):
+    with Scene(S.cornell(shadow_samples=side * side)) as s:
+        ref = s.render(6, 5, 1, 2, kernel=abi.KERNEL_MEGAKERNEL)
+        got = s.render(6, 5, 1, 2, kernel=abi.KERNEL_WAVEFRONT, **kw)
+    assert ref.any()
+    np.testing.assert_allclose(got, ref, rtol=2 * 65536 * 2.0 ** -24, atol=1e-6)
+
+
 def test_no_bounce_and_no_depth():
     """max_depth 0 renders black, depth 1 only what camera rays see; twice, so
     that the second render replays a kept graph."""
