@@ -790,9 +790,10 @@ int default_groups(const std::vector<RtScene*>& scenes, int nslots) {
 // drain less weight, until the render is too short to fill them. 4 M against
 // 8 M: full-HD icospheres of 133 M samples 109.0 and 104.7 ms, the mixed batch
 // of 63 M 103.3 and 100.9; foggy views of 17 M 46.4 and 47.2, open sky of 11 M
-// 8.4 and 9.2. 16 M gained nothing anywhere. Where 8 M do not fit the device's
-// free memory, wf_render takes 4 M.
+// 8.4 and 9.2. 16 M gained nothing anywhere. Where the device has no room for 8 M,
+// the render takes 4 M (wf_render).
 constexpr int kDefaultSlots = 1 << 22;
+constexpr size_t kMemorySpare = size_t(64) << 20;   // what the larger size must leave free
 int default_slots(int64_t total, int max_shadow) {
     return total >= (int64_t)1 << 25 && max_shadow <= 4 ? 2 * kDefaultSlots : kDefaultSlots;
 }
@@ -863,9 +864,11 @@ struct WfExit {
 // mode: rt::WF_RENDER renders the requests into their films; rt::WF_RECORD
 // and rt::WF_REPLAY are the two passes of the wavefront adjoint over the same
 // requests, with adj holding their buffers (rt_adjoint).
-// Called with g_wf_mu held.
+// Called with g_wf_mu held. no_room: set when the larger untuned wavefront does
+// not fit the device's memory. The free memory is asked first, so that a device
+// too small for it keeps the smaller workspace and its graphs from call to call.
 int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st, int mode,
-                     const rt::WfAdjoint* adj) {
+                     const rt::WfAdjoint* adj, bool& no_room) {
     auto t0 = std::chrono::steady_clock::now();
     RtScene* s0 = reqs[0].scene;
     int dev = s0->device;
@@ -1000,11 +1003,23 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     WfWorkspace& ws = g_wf_ws[dev];
     size_t need = layout(nullptr) + 1024;
     if (ws.bytes < need) {
+        const bool larger = cfg.slots <= 0 && nslots > kDefaultSlots;
+        size_t free_bytes = 0, all_bytes = 0;
+        if (larger && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess &&
+            free_bytes + ws.bytes < need + kMemorySpare) {
+            no_room = true;
+            return RT_ERR_OOM;
+        }
         ws.drop_graphs();   // captured with pointers into the old workspace
         if (ws.mem) cudaFree(ws.mem);
         ws.mem = nullptr;
         ws.bytes = 0;
-        if (cudaMalloc(&ws.mem, need) != cudaSuccess) return fail(RT_ERR_OOM, "wavefront workspace allocation failed");
+        if (cudaMalloc(&ws.mem, need) != cudaSuccess) {
+            cudaGetLastError();
+            ws.mem = nullptr;
+            no_room = larger;
+            return fail(RT_ERR_OOM, "wavefront workspace allocation failed");
+        }
         ws.bytes = need;
     }
     layout(static_cast<char*>(ws.mem));
@@ -1329,12 +1344,12 @@ int wf_render(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtStats* st
     if (reqs.empty()) return RT_OK;
     if (mode != rt::WF_RENDER && !adj) return fail(RT_ERR_INVALID_ARG, "adjoint pass without its buffers");
     std::lock_guard<std::mutex> lk(g_wf_mu);
-    int rc = wf_render_locked(reqs, cfg, st, mode, adj);
-    if (rc == RT_ERR_OOM && cfg.slots <= 0) {   // the larger untuned size does not fit: the smaller may
-        cudaGetLastError();
+    bool no_room = false;
+    int rc = wf_render_locked(reqs, cfg, st, mode, adj, no_room);
+    if (no_room) {
         WfConfig c = cfg;
         c.slots = kDefaultSlots;
-        rc = wf_render_locked(reqs, c, st, mode, adj);
+        rc = wf_render_locked(reqs, c, st, mode, adj, no_room);
     }
     return rc;
 }

@@ -110,6 +110,44 @@ def test_a_light_of_many_shadow_samples(side, kw):
     np.testing.assert_allclose(got, ref, rtol=2 * 65536 * 2.0 ** -24, atol=1e-6)
 
 
+def large_render_in_a_full_device():
+    """Run by the test below in a process of its own (its workspace starts empty)."""
+    import torch
+    spare = 256 << 20
+    size = dict(w=1024, h=1024, spp=33, depth=2, kernel=abi.KERNEL_WAVEFRONT)   # 34.6 M samples, past the 8 M line
+    with Scene(S.cornell()) as s:
+        stats = abi.RtStats()
+
+        def render(**kw):
+            p = abi.render_params(size["w"], size["h"], size["spp"], size["depth"], kernel=size["kernel"], **kw)
+            out = np.zeros((3, size["h"], size["w"]), np.float32)
+            abi.check(s.lib.rt_render(s.h, C.byref(p), abi.ptr(out), C.byref(stats)), "rt_render")
+            return out, stats.iterations
+
+        ref, small = render(wavefront_size=1 << 22)
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - spare, dtype=torch.uint8, device="cuda")
+        before = torch.cuda.mem_get_info()[0]
+        for _ in range(2):   # no room for 8 M beside the filling: 4 M, in the workspace at hand
+            img, n = render()
+            same_film(img, ref)
+            assert abs(n - small) <= 2, (n, small)
+            assert abs(torch.cuda.mem_get_info()[0] - before) < 64 << 20
+        del fill
+        torch.cuda.empty_cache()
+        img, n = render()
+        same_film(img, ref)
+        assert n < small - 2, (n, small)   # 8 M: about half the iterations
+
+
+def test_untuned_large_render_where_its_wavefront_fits_and_where_not():
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = "import sys; sys.path.insert(0, 'tests'); import test_wavefront_edges as t; t.large_render_in_a_full_device()"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_no_bounce_and_no_depth():
     """max_depth 0 renders black, depth 1 only what camera rays see; twice, so
     that the second render replays a kept graph."""
