@@ -923,7 +923,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     }
     int nslots = (int)std::max<int64_t>(1024, std::min<int64_t>(cfg.slots > 0 ? cfg.slots : default_slots(total, max_shadow), total));
     nslots = (nslots + 255) / 256 * 256;
-    int sort = (cfg.sort < 0 ? default_sort(nslots) : cfg.sort) && nkeys < 254;   // two keys beside the materials' (hit_store)
+    int sort = (cfg.sort < 0 ? default_sort(nslots) : cfg.sort) && nkeys + 2 <= rt::kSortKeys;   // two keys beside the materials' (hit_store)
     int64_t cap = (int64_t)nslots * max_shadow;
     if (cap >= ((int64_t)1 << 31) || nslots >= (1 << 29)) return fail(RT_ERR_INVALID_ARG, "wavefront too large");
     const int blk = cfg.block, tblk = cfg.tblock > 0 ? cfg.tblock : blk;

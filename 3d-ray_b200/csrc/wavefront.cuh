@@ -893,9 +893,10 @@ RT_D int block_scan(int v, int* s_w, int* total) {
 // 27.1 to 30.4 ms on the full-HD icosphere frame with its 65 materials.)
 constexpr int kSortThreads = 1024, kSortPer = 8, kSortCluster = 8;
 constexpr int kSortChunk = kSortThreads * kSortPer * kSortCluster;
+constexpr int kSortKeys = 256;   // keys of a chunk's counts
 __global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThreads)
     k_wf_scatter(const __grid_constant__ WfArgs a) {
-    __shared__ int s_w[32], s_cnt[256], s_all[kSortCluster][256], s_base;
+    __shared__ int s_w[32], s_cnt[kSortKeys], s_all[kSortCluster][kSortKeys], s_base;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const unsigned rank = cluster.block_rank();
@@ -903,7 +904,7 @@ __global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThre
     // A block's shared memory may be written by another once that block runs:
     // all arrive here, and wait before the first remote store, behind the loads.
     cluster.barrier_arrive();
-    if (tid < 256) s_cnt[tid] = 0;
+    if (tid < kSortKeys) s_cnt[tid] = 0;
     __syncthreads();
     int key[kSortPer], pos[kSortPer];
 #pragma unroll
@@ -922,18 +923,18 @@ __global__ void __cluster_dims__(kSortCluster, 1, 1) __launch_bounds__(kSortThre
     __syncthreads();
     cluster.barrier_wait();
     // every block gets every block's counts: a key's slots of the earlier blocks go first
-    if (tid < 256)
-        for (int q = 0; q < kSortCluster; q++) cluster.map_shared_rank(&s_all[0][0], q)[rank * 256 + tid] = s_cnt[tid];
+    if (tid < kSortKeys)
+        for (int q = 0; q < kSortCluster; q++) cluster.map_shared_rank(&s_all[0][0], q)[rank * kSortKeys + tid] = s_cnt[tid];
     cluster.sync();
     int sum = 0, before = 0, live;
-    if (tid < 256)
+    if (tid < kSortKeys)
         for (int q = 0; q < kSortCluster; q++) {
             int c = s_all[q][tid];
             if (q < (int)rank) before += c;
             sum += c;
         }
     int off = block_scan(sum, s_w, &live);
-    if (tid < 256) s_cnt[tid] = off + before;
+    if (tid < kSortKeys) s_cnt[tid] = off + before;
     if (rank == 0 && tid == 0) {
         int b = live ? atomicAdd(&a.ctl->nlive, live) : 0;
         for (int q = 0; q < kSortCluster; q++) *cluster.map_shared_rank(&s_base, q) = b;

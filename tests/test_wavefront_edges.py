@@ -97,6 +97,27 @@ def test_sorted_shadows_take_turns(world, slots):
                            sort_materials=1), ref)
 
 
+# Materials around the number of keys the material sort holds (256, two of them for
+# what is no material): the most that sort, and one more.
+@pytest.mark.parametrize("n", [253, 254, 255])
+def test_material_sort_up_to_its_keys(n):
+    w = S.cornell()
+    while len(w.materials) < n:
+        k = len(w.materials)
+        m = w.add_material(f"m{k}", S.disney((0.2 + 0.7 * (k % 7) / 7, 0.5, 0.9 - 0.6 * (k % 5) / 5)))
+        w.add_sphere((30.0 + 500 * (k % 16) / 16, 30.0 + 500 * (k // 16) / 16, 300.0), 14.0, m)
+    with Scene(w) as s:
+        ref = s.render(120, 90, 8, 4, kernel=abi.KERNEL_MEGAKERNEL)
+        launches = []
+        for sort in (0, 1):
+            p = abi.render_params(120, 90, 8, 4, kernel=abi.KERNEL_WAVEFRONT, sort_materials=sort, ray_groups=1)
+            out, st = np.zeros((3, 90, 120), np.float32), abi.RtStats()
+            abi.check(s.lib.rt_render(s.h, C.byref(p), abi.ptr(out), C.byref(st)), "rt_render")
+            same_film(out, ref)
+            launches.append((st.kernel_launches - 1) // st.iterations)
+    assert launches[1] - launches[0] == (1 if n <= 254 else 0)
+
+
 # Shadow samples whose records a vertex fill one axis of a grid, and one more row.
 # Film values are sums of that many positive terms in another order: each addition
 # rounds by 2^-24 of the sum at most, 65 536 x 2^-24 on either side.
