@@ -798,6 +798,13 @@ int default_slots(int64_t total, int max_shadow) {
     return total >= (int64_t)1 << 25 && max_shadow <= 4 ? 2 * kDefaultSlots : kDefaultSlots;
 }
 
+// The shadow records a vertex of the scene can write.
+int shadow_records(const RtScene* sc) {
+    int n = 0;
+    for (const rt::Light& l : sc->host.lights) n += l.shadow_samples;
+    return std::max(1, n);
+}
+
 // Untuned material sort: on, except in a wavefront too small to fill the SMs
 // with whole warps of one material (slot order, off against on: 12 K samples
 // 0.53 and 0.60 ms on a Cornell box, 0.53 and 0.64 on icospheres; 49 K 0.57 and
@@ -896,9 +903,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         views.push_back(sc->view);
         key_base.push_back(nkeys);
         nkeys += (int)sc->host.materials.size();
-        int sh = 0;
-        for (const rt::Light& l : sc->host.lights) sh += l.shadow_samples;
-        max_shadow = std::max(max_shadow, sh);
+        max_shadow = std::max(max_shadow, shadow_records(sc));
         opaque &= sc->opaque;
         dielectrics |= sc->dielectrics;
     }
@@ -1983,10 +1988,39 @@ int rt_autotune(RtScene* sc, const RtRenderParams* params, RtRenderParams* best)
             pick.fetch = 2;
         }
     }
+    // A render that takes 8 M slots untuned: the slice above is too short to fill
+    // them, so the winner is timed at both sizes over up to 64 M samples, in turn
+    // (full-HD icospheres of 133 M samples: 120.7 ms at 4 M, 115.8 at 8 M; a Cornell
+    // box of 42 M 83.7 and 84.9). Where 8 M have no room, 4 M stay.
+    bool by_size = false;
+    if (rc == RT_OK && pick.slots == kDefaultSlots && default_slots(npix * params->spp, shadow_records(sc)) > kDefaultSlots) {
+        double ms[2] = {1e30, 1e30};
+        for (int turn = 0; turn < 4 && rc == RT_OK; turn++) {
+            RtRenderParams p = *params;
+            p.kernel = RT_KERNEL_WAVEFRONT;
+            p.spp = (int)std::max<int64_t>(1, std::min<int64_t>(params->spp, ((int64_t)1 << 26) / npix + 1));
+            p.count_work = 0;
+            p.wavefront_size = (turn & 1) ? 2 * kDefaultSlots : kDefaultSlots;
+            p.block_size = pick.block;
+            p.sort_materials = pick.sort;
+            p.node_layout = pick.layout;
+            p.ray_fetch = pick.fetch;
+            p.trace_block_size = pick.tblock;
+            p.ray_groups = pick.groups;
+            RtStats s1{};
+            rc = render_to_device(sc, &p, sc->host.camera, d_film, &s1);
+            if (rc == RT_ERR_OOM && (turn & 1)) {
+                rc = RT_OK;
+                break;
+            }
+            if (rc == RT_OK) ms[turn & 1] = std::min(ms[turn & 1], s1.kernel_ms);
+        }
+        by_size = ms[1] < ms[0];
+    }
     cudaFree(d_film);
     if (rc != RT_OK) return rc;
     sc->tuned = 1;
-    sc->tuned_slots = pick.slots;
+    sc->tuned_slots = by_size ? 0 : pick.slots;   // 8 M for the renders that take them untuned, 4 M for the others
     sc->tuned_block = pick.block;
     sc->tuned_sort = pick.sort;
     sc->tuned_layout = pick.layout;
@@ -1996,7 +2030,7 @@ int rt_autotune(RtScene* sc, const RtRenderParams* params, RtRenderParams* best)
     if (best) {
         *best = *params;
         best->kernel = RT_KERNEL_WAVEFRONT;
-        best->wavefront_size = pick.slots;
+        best->wavefront_size = by_size ? default_slots(npix * params->spp, shadow_records(sc)) : pick.slots;
         best->block_size = pick.block;
         best->sort_materials = pick.sort;
         best->node_layout = pick.layout;

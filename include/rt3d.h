@@ -402,7 +402,9 @@ int rt_render_capture(RtScene* scene, const RtRenderParams* params, float* hdr_r
  * and shadow rays} and the persistent dynamic-fetch kernels, on a bounded
  * slice of `params` (the full window at the spp giving ~16 M samples), keeps
  * the fastest for this scene (used when those params fields are 0 / -1) and
- * returns it. */
+ * returns it. Where 4 M slots win and the full render would take 8 M untuned,
+ * both are timed on up to 64 M samples; if 8 M win, renders of that size take
+ * them and smaller ones 4 M. */
 int rt_autotune(RtScene* scene, const RtRenderParams* params, RtRenderParams* best);
 
 /* ---- differentiation ----------------------------------------------------- */
