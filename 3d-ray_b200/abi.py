@@ -320,6 +320,7 @@ def load(path: str | None = None):
         "rt_energy_lut": (C.c_int, [P, P]),
         "rt_probe_l2_bandwidth": (C.c_int, [C.c_int32, C.c_int64, C.c_int32, C.POINTER(C.c_double)]),
         "rt_tonemap": (C.c_int, [P, C.c_int32, C.c_int32, C.c_float, P]),
+        "rt_release_memory": (C.c_int, [C.c_int32]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)

@@ -2543,6 +2543,42 @@ int rt_tonemap(const float* hdr, int32_t width, int32_t height, float exposure_e
     return rc;
 }
 
+int rt_release_memory(int32_t device) {
+    int ndev = 0, before = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(RT_ERR_NO_DEVICE, "no CUDA device");
+    if (device < -1 || device >= ndev) return fail(RT_ERR_INVALID_ARG, "bad device");
+    CUDA_TRY(cudaGetDevice(&before));
+    for (int dev = std::max(device, 0); dev < std::min(device < 0 ? ndev : device + 1, 16); dev++) {
+        // A call holds its lock until its last copy has landed, so what a lock
+        // guards is idle once it is taken.
+        auto enter = [&](bool held) { return held && cudaSetDevice(dev) == cudaSuccess; };
+        {
+            std::lock_guard<std::mutex> lk(g_wf_mu);
+            WfWorkspace& ws = g_wf_ws[dev];
+            if (enter(ws.mem || ws.pinned || !ws.graphs.empty())) {
+                ws.drop_graphs();
+                cudaFree(ws.mem);
+                cudaFreeHost(ws.pinned);
+                ws.mem = nullptr;
+                ws.pinned = nullptr;
+                ws.bytes = ws.pinned_bytes = 0;
+            }
+        }
+        {
+            std::lock_guard<std::mutex> lk(g_tone[dev].mu);
+            if (enter(g_tone[dev].mem)) {
+                cudaFree(g_tone[dev].mem);
+                g_tone[dev].mem = nullptr;
+                g_tone[dev].bytes = 0;
+            }
+        }
+        std::lock_guard<std::mutex> lk(rt::g_stage[dev].mu);
+        if (enter(rt::g_stage[dev].mem)) rt::g_stage[dev].release();
+    }
+    CUDA_TRY(cudaSetDevice(before));
+    return RT_OK;
+}
+
 }  // extern "C"
 
 namespace {

@@ -30,6 +30,15 @@ struct Stage {
     std::mutex mu;
     char* mem = nullptr;
     cudaEvent_t landed[kStageChunks] = {};
+    // With mu held, which a copy holds until it is done.
+    void release() {
+        for (cudaEvent_t& e : landed) {
+            if (e) cudaEventDestroy(e);
+            e = {};
+        }
+        if (mem) cudaFreeHost(mem);
+        mem = nullptr;
+    }
 };
 inline Stage g_stage[16];
 
@@ -48,16 +57,14 @@ inline cudaError_t stage_copy(int dev, cudaStream_t stream, char* host, char* de
     if (!lk.owns_lock()) return plain();
     if (!st.mem) {   // no window or no events: the driver's way
         bool ok = cudaMallocHost(&st.mem, kStageChunk * kStageChunks) == cudaSuccess;
-        size_t made = 0;
-        while (ok && made < kStageChunks) {
-            ok = cudaEventCreateWithFlags(&st.landed[made], cudaEventDisableTiming) == cudaSuccess;
-            made += ok;
+        if (!ok) st.mem = nullptr;
+        for (size_t c = 0; ok && c < kStageChunks; c++) {
+            ok = cudaEventCreateWithFlags(&st.landed[c], cudaEventDisableTiming) == cudaSuccess;
+            if (!ok) st.landed[c] = {};
         }
         if (!ok) {
             cudaGetLastError();
-            while (made) cudaEventDestroy(st.landed[--made]);
-            if (st.mem) cudaFreeHost(st.mem);
-            st.mem = nullptr;
+            st.release();
             return plain();
         }
     }

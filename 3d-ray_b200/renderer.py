@@ -197,6 +197,12 @@ class Renderer:
         return out
 
 
+def release_memory(device: int = -1) -> None:
+    """Gives back the memory that calls keep on a device (-1: all) beside the
+    scenes' own (rt_release_memory); later calls allocate it again."""
+    abi.check(abi.load().rt_release_memory(device), "rt_release_memory")
+
+
 def render_batch(requests, worlds, common_kernel: str = "wavefront", **kw):
     """Renders many (scene, camera, size, spp, depth) requests in one
     persistent wavefront launch (rt_render_batch). `worlds` is a list of

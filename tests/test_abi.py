@@ -51,6 +51,7 @@ def test_no_device_fails_cleanly(lib):
     rc = lib.rt_scene_create(abi.PackedWorld(rt.scenes.cornell()).ref(), C.byref(h))
     assert rc == -8 and h.value is None
     assert b"device" in lib.rt_last_error()
+    assert lib.rt_release_memory(-1) == -8
 
 
 def test_renderer_params_mirror_reference_defaults():

@@ -317,3 +317,40 @@ def test_renders_and_display_transforms_from_several_threads():
         for t in threads:
             t.join()
     assert not wrong
+
+
+def test_kept_memory_is_given_back():
+    """After large calls rt_release_memory frees what they left, also from a second
+    thread while renders run; films and display images stay what they were."""
+    import threading
+    import torch
+    lib = abi.load()
+    x = np.exp(np.random.default_rng(2).normal(-1.0, 1.5, (3, 1080, 1920))).astype(np.float32)
+    shown = [np.empty((1080, 1920, 3), np.float32) for _ in range(2)]
+    size = dict(w=512, h=384, spp=24, depth=6, kernel=abi.KERNEL_WAVEFRONT)
+    with Scene(WORLDS["sky"]()) as s:
+        ref = s.render(**size)   # 4.7 M samples: 4 M slots, over 1 GB
+        abi.check(lib.rt_tonemap(abi.ptr(x), 1920, 1080, 0.0, abi.ptr(shown[0])), "rt_tonemap")
+        before = torch.cuda.mem_get_info()[0]
+        abi.check(lib.rt_release_memory(-1), "rt_release_memory")
+        assert torch.cuda.mem_get_info()[0] - before > 1 << 30
+        assert lib.rt_release_memory(99) == -1 and lib.rt_release_memory(-2) == -1
+        same_film(s.render(**size), ref)
+        abi.check(lib.rt_tonemap(abi.ptr(x), 1920, 1080, 0.0, abi.ptr(shown[1])), "rt_tonemap")
+        assert np.array_equal(*shown)
+        stop = threading.Event()
+
+        def release():
+            while not stop.is_set():
+                abi.check(lib.rt_release_memory(0), "rt_release_memory")
+
+        t = threading.Thread(target=release)
+        t.start()
+        try:
+            for _ in range(10):
+                same_film(s.render(**size), ref)
+                abi.check(lib.rt_tonemap(abi.ptr(x), 1920, 1080, 0.0, abi.ptr(shown[1])), "rt_tonemap")
+                assert np.array_equal(*shown)
+        finally:
+            stop.set()
+            t.join()
