@@ -870,12 +870,6 @@ RT_D void tangent_frame(V3 n, V3& t, V3& b) {   // Microfacet.cs:22-37
         b = v3(bb, 1.0f - n.y * n.y * a, -n.y);
     }
 }
-RT_D float d_ggx(V3 h, float ax, float ay) {   // :43-49
-    float hx = h.x / ax;
-    float hy = h.y / ay;
-    float d = hx * hx + hy * hy + h.z * h.z;
-    return 1.0f / fmaxf(kPi * ax * ay * d * d, 1e-20f);
-}
 RT_D float g1_ggx(V3 w, float ax, float ay) {   // :55-69
     float c2 = w.z * w.z;
     float lam;
@@ -1046,7 +1040,7 @@ RT_D void bsdf_eval_pdf(const Material& m, const Surface& rec, const BsdfView& b
     float ndh = dot(N, H);
     float vdh = fmaxf(dot(V, H), 0.0f);
     V3 hl = b.fr.to_local(H);
-    float hx = hl.x / m.alpha_x, hy = hl.y / m.alpha_y;   // d_ggx with pi ax ay from the material
+    float hx = hl.x / m.alpha_x, hy = hl.y / m.alpha_y;   // the GGX density (:43-49), pi ax ay from the material
     float hd = hx * hx + hy * hy + hl.z * hl.z;
     float D = 1.0f / fmaxf(m.pi_axy * hd * hd, 1e-20f);
     bool spec_ok = m.alpha > kDeltaAlpha;
@@ -1470,7 +1464,7 @@ __device__ __noinline__ void light_sample_sphere_env(const SceneView& s, const L
         if (cl <= 0.0f) return;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-            r.ray_tmax = length(sp - so) - kEps;
+        r.ray_tmax = length(sp - so) - kEps;
         float atten = 1.0f / (pdf * (float)l.shadow_samples);
         r.color = l.emission * atten;
         return;
@@ -1515,7 +1509,7 @@ __device__ __noinline__ void light_sample_sphere_env(const SceneView& s, const L
         if (cl <= 0.0f) return;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-            r.ray_tmax = length(sp - so) - kEps;
+        r.ray_tmax = length(sp - so) - kEps;
         float sa = 2.0f * kPi * (1.0f - cmax);
         float atten = l.intensity * sa / (float)l.shadow_samples;
         r.color = l.color * atten;
@@ -1614,7 +1608,7 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         }
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-            r.ray_tmax = length(sp - so) - kEps;
+        r.ray_tmax = length(sp - so) - kEps;
         float atten = area * cl / (d2 * (float)l.shadow_samples);
         r.color = l.emission * atten;
         return r;
@@ -1652,7 +1646,7 @@ RT_D LightSample light_sample(const SceneView& s, const Light& l, V3 p, V3 sn, i
         if (cl <= 0.0f) return r;   // not in shadow, zero colour
         V3 so = offset_origin(p, sn);
         r.has_ray = 1;
-            r.ray_tmax = length(sp - so) - kEps;
+        r.ray_tmax = length(sp - so) - kEps;
         float ad2 = d2;
         if (l.soft_radius > 0.0f) ad2 = fmaxf(ad2, l.soft_radius * l.soft_radius);
         float atten = l.intensity * l.area * cl / (ad2 * (float)l.shadow_samples);

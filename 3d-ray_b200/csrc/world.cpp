@@ -386,7 +386,7 @@ struct WalkBuilder {
     HostScene& sc;
     struct Kid {
         Box box;
-        int code = INT_MIN, code4 = INT_MIN;
+        int code = INT_MIN;   // in the layout at hand
     };
     static Box unbounded() {
         const float inf = std::numeric_limits<float>::infinity();
@@ -397,14 +397,11 @@ struct WalkBuilder {
         std::memcpy(&f, &i, 4);
         return f;
     }
-    // One entity of a list. `tested`: its own box was tested where its leaf's was.
-    Kid entity(int e) const {
+    // One entity of a list, in the two- or four-wide layout.
+    Kid entity(int e, bool four) const {
         const Entity& en = sc.entities[e];
-        if (en.kind != ENT_MESH) {
-            int c = leaf_code(e, LEAF_ENT1, 1);
-            return {unbounded(), c, c};
-        }
-        Kid k{unbounded(), en.index, sc.mesh_root4[(size_t)e]};
+        if (en.kind != ENT_MESH) return {unbounded(), leaf_code(e, LEAF_ENT1, 1)};
+        Kid k{unbounded(), four ? sc.mesh_root4[(size_t)e] : en.index};
         if (en.index >= 0) {
             const float4 &lo = sc.ent_box[2 * (size_t)e], &hi = sc.ent_box[2 * (size_t)e + 1];
             k.box = {v3(lo.x, lo.y, lo.z), v3(hi.x, hi.y, hi.z)};
@@ -424,12 +421,12 @@ struct WalkBuilder {
         const float inf = std::numeric_limits<float>::infinity();
         float lo[3][4], hi[3][4], cf[4];
         for (int j = 0; j < 4; j++) {
-            bool used = k[j].code4 != INT_MIN;
+            bool used = k[j].code != INT_MIN;
             for (int a = 0; a < 3; a++) {
                 lo[a][j] = used ? axis_of(k[j].box.mn, a) : inf;
                 hi[a][j] = used ? axis_of(k[j].box.mx, a) : inf;
             }
-            cf[j] = bits(k[j].code4);
+            cf[j] = bits(k[j].code);
         }
         for (int a = 0; a < 3; a++) sc.cnodes4.push_back(float4{lo[a][0], lo[a][1], lo[a][2], lo[a][3]});
         for (int a = 0; a < 3; a++) sc.cnodes4.push_back(float4{hi[a][0], hi[a][1], hi[a][2], hi[a][3]});
@@ -437,73 +434,75 @@ struct WalkBuilder {
         sc.cnodes4.push_back(float4{bits(axes[0]), bits(axes[1]), bits(axes[2]), 0.0f});
         return i;
     }
-    // A list of entities in order (a top-level leaf, at most 4, or the flat list).
-    Kid list(const int* items, int n) const {
-        if (n == 1) return entity(items[0]);
-        Kid out{unbounded(), 0, 0};
-        out.code = record2(entity(items[0]), list2(items + 1, n - 1), 3);
+    // A list of entities in order (a top-level leaf or the flat list, at most 4).
+    Kid list2(const int* items, int n) const {
+        if (n == 1) return entity(items[0], false);
+        return {unbounded(), record2(entity(items[0], false), list2(items + 1, n - 1), 3)};
+    }
+    Kid list4(const int* items, int n) const {
+        if (n == 1) return entity(items[0], true);
         Kid k[4];
-        for (int j = 0; j < n; j++) k[j] = entity(items[j]);
+        for (int j = 0; j < n; j++) k[j] = entity(items[j], true);
         const int order[3] = {3, 3, 3};
-        out.code4 = record4(k, order);
-        return out;
+        return {unbounded(), record4(k, order)};
     }
-    Kid list2(const int* items, int n) const {   // the rest of a list, in the two-wide layout alone
-        if (n == 1) return entity(items[0]);
-        Kid out{unbounded(), 0, INT_MIN};
-        out.code = record2(entity(items[0]), list2(items + 1, n - 1), 3);
-        return out;
+    // Node n of the binary top-level tree: its own box guards a leaf's list too.
+    bool inner(int n, int& l, int& r, int& axis) const {
+        int b;
+        std::memcpy(&l, &sc.nodes[n].lo[3], 4);
+        std::memcpy(&b, &sc.nodes[n].hi[3], 4);
+        r = b & 0x3FFFFFFF;
+        axis = (int)((unsigned)b >> 30);
+        return l >= 0;
     }
-    // The binary top-level tree, its leaves as lists; kids4 of a record are the
-    // node's grandchildren where a child is an interior node itself.
-    struct Node {
-        Kid self;
-        bool inner = false;
-        int axis = 0;
-        Kid l, r;
-    };
-    Node node(int n) const {
-        const NodeF& f = sc.nodes[n];
+    const int* leaf(int n, int& count) const {
         int a, b;
-        std::memcpy(&a, &f.lo[3], 4);
-        std::memcpy(&b, &f.hi[3], 4);
-        Node out;
-        Box box{v3(f.lo[0], f.lo[1], f.lo[2]), v3(f.hi[0], f.hi[1], f.hi[2])};
-        if (a < 0) {
-            out.self = list(&sc.top_items[~a], b & 0xFFFF);
-            out.self.box = box;   // the leaf's own box guards the list
-            return out;
+        std::memcpy(&a, &sc.nodes[n].lo[3], 4);
+        std::memcpy(&b, &sc.nodes[n].hi[3], 4);
+        count = b & 0xFFFF;
+        return &sc.top_items[~a];
+    }
+    Box box(int n) const {
+        const NodeF& f = sc.nodes[n];
+        return {v3(f.lo[0], f.lo[1], f.lo[2]), v3(f.hi[0], f.hi[1], f.hi[2])};
+    }
+    Kid node2(int n) const {
+        int l, r, axis, count;
+        if (inner(n, l, r, axis)) {
+            Kid kl = node2(l), kr = node2(r);
+            return {box(n), record2(kl, kr, axis)};
         }
-        Node L = node(a), R = node(b & 0x3FFFFFFF);
-        out.inner = true;
-        out.axis = (int)((unsigned)b >> 30);
-        out.l = L.self;
-        out.r = R.self;
-        out.self.box = box;
-        out.self.code = record2(L.self, R.self, out.axis);
+        const int* items = leaf(n, count);
+        return {box(n), list2(items, count).code};
+    }
+    // One record spans two levels: it holds a node's grandchildren where a child
+    // is an interior node itself.
+    Kid node4(int n) const {
+        int c[2], axes[3] = {0, 0, 0}, count;
+        if (!inner(n, c[0], c[1], axes[0])) {
+            const int* items = leaf(n, count);
+            return {box(n), list4(items, count).code};
+        }
         Kid k[4];
-        int axes[3] = {out.axis, 0, 0};
         for (int side = 0; side < 2; side++) {
-            const Node& c = side == 0 ? L : R;
-            if (c.inner) {
-                k[2 * side] = c.l;
-                k[2 * side + 1] = c.r;
-                axes[1 + side] = c.axis;
+            int l, r, axis;
+            if (inner(c[side], l, r, axis)) {
+                k[2 * side] = node4(l);
+                k[2 * side + 1] = node4(r);
+                axes[1 + side] = axis;
             } else {
-                k[2 * side] = c.self;
+                k[2 * side] = node4(c[side]);
             }
         }
-        out.self.code4 = record4(k, axes);
-        return out;
+        return {box(n), record4(k, axes)};
     }
 };
 
 void build_walk(HostScene& sc) {
     WalkBuilder b{sc};
-    WalkBuilder::Kid root = sc.top_is_bvh ? b.node(sc.top_root).self
-                                          : b.list(sc.top_items.data(), (int)sc.top_items.size());
-    sc.walk_root = root.code;
-    sc.walk_root4 = root.code4;
+    const int n = (int)sc.top_items.size();
+    sc.walk_root = (sc.top_is_bvh ? b.node2(sc.top_root) : b.list2(sc.top_items.data(), n)).code;
+    sc.walk_root4 = (sc.top_is_bvh ? b.node4(sc.top_root) : b.list4(sc.top_items.data(), n)).code;
 }
 
 }  // namespace
@@ -763,7 +762,8 @@ int build_world(const RtWorldDesc* w, HostScene& sc, std::string& err, const Bui
         }
         if (sc.top_is_bvh) sc.top_root_code = code_of(sc.top_root);
         // --- four-wide layout: one record per interior node at even depth of
-        // each tree, holding its grandchildren (see SceneView).
+        // each mesh's tree, holding its grandchildren (see SceneView; the top
+        // level's records are build_walk's).
         {
             auto kids = [&](int node, int& l, int& r, int& axis) {
                 int a, b;
@@ -777,7 +777,6 @@ int build_world(const RtWorldDesc* w, HostScene& sc, std::string& err, const Bui
             };
             std::vector<int> ridx(sc.nodes.size(), -1), rnode;
             std::vector<int> work;
-            if (sc.top_is_bvh) work.push_back(sc.top_root);
             for (int e : mesh_ids) work.push_back(sc.entities[e].index);
             while (!work.empty()) {
                 int n = work.back();
@@ -839,7 +838,6 @@ int build_world(const RtWorldDesc* w, HostScene& sc, std::string& err, const Bui
             }
             sc.mesh_root4.assign((size_t)ne, 0);
             for (int e : mesh_ids) sc.mesh_root4[(size_t)e] = code4(sc.entities[e].index);
-            if (sc.top_is_bvh) sc.top_root4 = code4(sc.top_root);
             // a record pushes at most three slots; it spans two binary levels
             sc.max_stack4 = 3 * ((top_depth + 1) / 2) + 4 + 3 * ((max_blas_depth + 1) / 2) + 1;
         }
