@@ -775,7 +775,9 @@ void apply_test_limits(WfConfig& cfg, const RtRenderParams* p) {
 //     2.74 / 2.00 and 2.19 / 1.55 and 1.60; 3.1 M 6.2 and 5.4 / 3.4 and 3.5 /
 //     3.06 and 3.05. The Cornell box has the line at 300 K, icospheres past 3 M
 //     (a full-HD frame of 133 M samples gains 10%): it lies where the first of
-//     them starts to gain.
+//     them starts to gain, and icospheres between it and 3 M lose 3 to 15%. What
+//     tells the two apart is the share of slots with bounce rays, which the host
+//     does not know.
 constexpr int kSortRaysSlots = 1 << 18;
 int default_groups(const std::vector<RtScene*>& scenes, int nslots) {
     if (nslots <= kSortRaysSlots) return 1;
@@ -784,8 +786,8 @@ int default_groups(const std::vector<RtScene*>& scenes, int nslots) {
     return 4;
 }
 
-// Untuned wavefront size: 4 M path slots, 8 M (about 330 bytes each with two
-// shadow records) for a render of 32 M samples or more whose vertices queue at
+// Untuned wavefront size: 4 M path slots, 8 M (300 bytes each with two shadow
+// records, 348 in batches with dielectrics) for a render of 32 M samples or more whose vertices queue at
 // most four records. More slots give the ray sorts more rays a key and the
 // drain less weight, until the render is too short to fill them. 4 M against
 // 8 M: full-HD icospheres of 133 M samples 109.0 and 104.7 ms, the mixed batch

@@ -1,19 +1,23 @@
 // Persistent, request-batched wavefront form of the bounce loop.
 //
 // A fixed pool of path slots (the wavefront) is advanced one vertex per
-// iteration by five small kernels instead of one large one:
+// iteration by small kernels instead of one large one:
 //   regen   : resolve finished samples into their request's film and list the
 //             free slots.
 //   camera  : take the next (request, sample, pixel) work items, trace their
 //             camera rays and start the paths that hit something in free slots.
 //   extend  : closest hit of every other live path's current ray.
+//   scatter : optionally, the live slots by material (a counting sort in chunks),
+//             so that shade's warps hold one material.
 //   shade   : one TraceRay vertex (medium, emission, NEE, BSDF sample, RR).
 //             Shadow rays go to a queue instead of being traced inline.
+//   plan    : the iteration's bookkeeping: whether the loop goes on, and the ray
+//             sorts' key scans.
+//   sscatter: optionally, the shadow records in key order.
 //   occlude : any-hit (or the transparent walk) of the queued shadow rays;
 //             visible contributions are added to their path's accumulator.
-// The iteration is captured once in a CUDA graph and replayed until every
-// request's samples are done. Optional material sorting (a counting sort of
-// live slots by material id) feeds shade coherent warps.
+// The iteration is the body of a loop in a CUDA graph, which plan ends on the
+// device when every request's samples are done.
 //
 // Many requests of uneven resolution, spp and depth share the pool: a work id
 // maps to (request, sample, pixel) with a binary search over the requests'
@@ -218,7 +222,7 @@ RT_D int wf_flags(const PS& ps, int alive) {
 }
 
 // The window's pixels in 8-pixel-wide column strips, rows inside a strip:
-// regen hands out work ids in this order, so the 32 camera rays of a warp
+// work ids run in this order, so the 32 camera rays of a warp of the camera kernel
 // cover an 8x4 block rather than a 32x1 run, and the accumulation buffer is
 // laid out the same way, so that the film atomics of consecutive slots stay
 // contiguous. The last strip is narrower when ww % 8 != 0.

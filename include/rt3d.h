@@ -542,9 +542,9 @@ int rt_sobol_batch(const uint32_t* sample_index, const uint32_t* dim, const uint
 int rt_tonemap(const float* hdr_rgb_planar, int32_t width, int32_t height, float exposure_ev, float* rgb_out);
 
 /* Gives back what the library keeps on a device between calls, beside its
- * scenes: the wavefront's workspace (up to 2.7 GB after an untuned render of 32 M
- * samples or more; it grows with a batch's films) and graphs, the display
- * transform's buffer (up to 256 MiB) and the pinned windows of host copies.
+ * scenes: the wavefront's workspace (2.5 GB after an untuned render of 32 M samples
+ * or more with two shadow samples a vertex; it grows with those and with a batch's
+ * films) and graphs, the display transform's buffer (up to 256 MiB) and the pinned windows of host copies.
  * device -1: every device. Waits for calls that use them; any call may follow,
  * and allocates again what it needs. For a process that shares the GPU with other
  * work; no counterpart in the reference. */

@@ -7,8 +7,8 @@ faults, traps or waits forever:
 - RT_ERR_STACK: a world whose traversal needs more stack entries than the
   kernels hold (the host computes the bound at build time) is refused before
   any launch, by every entry point that traces;
-- RT_ERR_TIMEOUT: the wavefront's host-side iteration bound (the loop that
-  polls the device) expires, forced with the test-only `iteration_limit`;
+- RT_ERR_TIMEOUT: the bound on the wavefront's iterations, at which the device
+  ends its loop, is reached, forced with the test-only `iteration_limit`;
 - RT_ERR_BOUNDS: the shadow queue fills up, forced with the test-only
   `shadow_queue_limit`; the kernel refuses the extra records and sets a flag
   the host reads.
