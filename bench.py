@@ -325,7 +325,7 @@ def profile_adjoint(args):
     slots += [ds.slot("fit_sphere", n) for n in ("roughness", "metallic", "specular", "sheen")]
     res, spp = 256, 32
     wimg = np.random.default_rng(2).uniform(0, 1, (3, res, res)).astype(np.float32)
-    rp = abi.render_params(res, res, spp, 8, kernel=adjoint_kernel(args))
+    rp = abi.render_params(res, res, spp, 8, kernel=adjoint_kernel(args), profile_kernels=int(args.split))
     for i in range(2):
         g = ds.adjoint(rp, wimg, slots)
         st = ds.last_stats
@@ -696,7 +696,8 @@ def main():
     ap.add_argument("--spp", type=int, default=SPP)
     ap.add_argument("--node-layout", type=int, default=2, choices=[2, 4],
                     help="BVH records for --profile-frame: two-wide or four-wide")
-    ap.add_argument("--split", action="store_true", help="--profile-frame: per-kernel event times")
+    ap.add_argument("--split", action="store_true", help="--profile-frame, --profile-adjoint: the host runs "
+                    "the iterations, kernel by kernel with event times")
     ap.add_argument("--block", type=int, default=256, choices=[64, 128, 256],
                     help="--profile-frame: block size of extend/occlude")
     ap.add_argument("--ray-fetch", type=int, default=1, choices=[1, 2],
