@@ -283,8 +283,8 @@ def time_to_relmse(rt, lib, abi):
 
 
 def profile_frame(args):
-    """One warm-up and one measured frame with fixed wavefront settings (4M
-    slots, material sort, --block for extend/occlude) or the megakernel: the workload the ncu
+    """One warm-up and one measured frame with fixed wavefront settings (--slots
+    path slots, material sort, --block for extend/occlude) or the megakernel: the workload the ncu
     summaries under profiles/ were captured on."""
     rt, world = build_world()
     abi = rt.abi
@@ -293,7 +293,7 @@ def profile_frame(args):
     scene = C.c_void_p()
     abi.check(lib.rt_scene_create(pw.ref(), C.byref(scene)), "rt_scene_create")
     kern = abi.KERNEL_WAVEFRONT if args.kernel == "wavefront" else abi.KERNEL_MEGAKERNEL
-    p = abi.render_params(W, H, args.spp, DEPTH, kernel=kern, wavefront_size=1 << 22, block_size=256,
+    p = abi.render_params(W, H, args.spp, DEPTH, kernel=kern, wavefront_size=args.slots, block_size=256,
                           trace_block_size=args.block,
                           sort_materials=1, node_layout=args.node_layout, ray_fetch=args.ray_fetch,
                           ray_groups=args.ray_groups, profile_kernels=int(args.split))
@@ -698,6 +698,7 @@ def main():
                     help="BVH records for --profile-frame: two-wide or four-wide")
     ap.add_argument("--split", action="store_true", help="--profile-frame, --profile-adjoint: the host runs "
                     "the iterations, kernel by kernel with event times")
+    ap.add_argument("--slots", type=int, default=1 << 22, help="--profile-frame: path slots of the wavefront")
     ap.add_argument("--block", type=int, default=256, choices=[64, 128, 256],
                     help="--profile-frame: block size of extend/occlude")
     ap.add_argument("--ray-fetch", type=int, default=1, choices=[1, 2],
@@ -877,7 +878,7 @@ def main():
                 l2_bytes = float(line.split(":")[1])
     roof["traffic"] = traffic
     roof["traffic_source"] = (f"profiles/{roof['kernel']}_icospheres.md: ncu DRAM read + write of a steady-state "
-                              "launch (all 4 M slots busy), measured on the same kernels") if traffic else None
+                              "launch at 8 M slots, measured on the same kernels") if traffic else None
     # L2 roofline beside the HBM one: the scene is largely L2-resident, so the
     # traversal kernels are compared against L2 bandwidth too. The peak is a
     # project micro-benchmark (L2-only float4 streams over a 32 MiB buffer).
