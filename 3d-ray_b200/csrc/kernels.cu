@@ -1174,7 +1174,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
     const unsigned grg = (unsigned)((nslots + rt::kRegenBlock - 1) / rt::kRegenBlock);
     const unsigned gsort = (unsigned)((nslots + rt::kSortChunk - 1) / rt::kSortChunk) * rt::kSortCluster;
     // ev (profiling only): boundaries between the kernel groups of one iteration.
-    auto launch_iter = [&](cudaEvent_t* ev, cudaGraphConditionalHandle loop) {
+    auto launch_iter = [&](cudaEvent_t* ev, const cudaGraphConditionalHandle* loop) {
         if (ev) cudaEventRecord(ev[0], stream);
         regen<<<grg, rt::kRegenBlock, 0, stream>>>(a);
         if (mode != rt::WF_REPLAY) camera<<<gcam, 128, 0, stream>>>(a);
@@ -1193,7 +1193,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
             shade<<<gs, sblk, 0, stream>>>(a);
         }
         if (ev) cudaEventRecord(ev[4], stream);   // the ray sorts' scans and scatter count as sorting
-        rt::k_wf_plan<<<gplan, 1024, 0, stream>>>(a, loop);
+        rt::k_wf_plan<<<gplan, 1024, 0, stream>>>(a, loop ? *loop : cudaGraphConditionalHandle{}, loop != nullptr);
         if (a.shadowsort) rt::k_wf_sscatter<<<gss, 256, 0, stream>>>(a);
         if (ev) cudaEventRecord(ev[5], stream);
         if (mode != rt::WF_REPLAY) {
@@ -1224,7 +1224,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         } else {
             WfGraph g;
             g.key = std::move(key);
-            rc = wf_capture(stream, [&](cudaGraphConditionalHandle h) { launch_iter(nullptr, h); }, g.exec);
+            rc = wf_capture(stream, [&](const cudaGraphConditionalHandle& h) { launch_iter(nullptr, &h); }, g.exec);
             if (rc != RT_OK) return rc;
             if (ws.graphs.size() >= kMaxGraphs) {
                 cudaGraphExecDestroy(ws.graphs.back().exec);
@@ -1246,7 +1246,7 @@ int wf_render_locked(const std::vector<HostReq>& reqs, const WfConfig& cfg, RtSt
         for (auto& e : pev)
             if (rc == RT_OK && cudaEventCreate(&e) != cudaSuccess) rc = fail(RT_ERR_CUDA, "event creation failed");
         while (rc == RT_OK) {
-            launch_iter(pev, cudaGraphConditionalHandle{});
+            launch_iter(pev, nullptr);
             cudaError_t e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_ctl, sizeof(rt::WfCtl), cudaMemcpyDeviceToHost, stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);

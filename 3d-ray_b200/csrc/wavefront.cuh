@@ -1157,14 +1157,15 @@ RT_D void key_scan(int* hist, int* off, int* total) {
 // Cornell box of 4 M 11.4 against 10.0 ms; and the counters that the next
 // iteration accumulates, none of which occlude reads), the first cluster scans
 // the bounce rays' keys and the second the shadow records'. loop: the graph's
-// loop condition, 0 when the host runs the iterations itself.
+// loop condition, in_loop: whether there is one (a handle has no value that means
+// none, and a loop that nobody ends does not end).
 __global__ void __cluster_dims__(kPlanCluster, 1, 1) __launch_bounds__(1024)
-    k_wf_plan(const __grid_constant__ WfArgs a, cudaGraphConditionalHandle loop) {
+    k_wf_plan(const __grid_constant__ WfArgs a, cudaGraphConditionalHandle loop, bool in_loop) {
     WfCtl* c = a.ctl;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         c->iters++;
         c->done = c->next >= c->total && c->live == 0;
-        if (loop && (c->done || c->overflow || c->err || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
+        if (in_loop && (c->done || c->overflow || c->err || c->iters >= c->limit)) cudaGraphSetConditional(loop, 0);
         c->iter_first = c->next;
         c->live = 0;
         c->ext_next = 0;
